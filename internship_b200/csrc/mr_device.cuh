@@ -141,6 +141,56 @@ struct Rng {
     --left;
     return u01(x);
   }
+  // RngRing's interface
+  __device__ __forceinline__ void prime() {}
+  __device__ __forceinline__ float take() { return next(); }
+};
+
+// The same stream with eight draws buffered per thread in shared memory, for
+// the trackers' loops. With four draws in registers the lanes of a warp run
+// dry at different draws, and nearly every draw of the warp executes Philox
+// for a few lanes. Here prime() tops a lane up once per four draws, at the
+// same loop iteration in all lanes: one Philox call per four draws of the
+// warp. Slot j of a lane is at base[32 j] (one bank per lane).
+constexpr int kRingWords = 8;
+struct RngRing {
+  uint32_t a, b, tag, key;
+  uint32_t head, end;  // draws taken and draws generated
+  uint32_t* base;
+  // ring: kRingWords * blockDim.x words of shared memory
+  __device__ __forceinline__ void attach(uint32_t* ring) {
+    base = ring + (threadIdx.x >> 5) * (32 * kRingWords) + (threadIdx.x & 31);
+  }
+  __device__ __forceinline__ void init(uint32_t seed, uint32_t a_, uint32_t b_, uint32_t tag_) {
+    a = a_; b = b_; tag = tag_; key = seed; head = end = 0;
+  }
+  __device__ __forceinline__ void refill() {
+    uint32_t o[4];
+    philox4x32_10(a, b, end >> 2, tag, key, 0u, o);
+    uint32_t* p = base + 32 * (end & (kRingWords - 1));  // end is a multiple of 4
+    p[0] = o[0]; p[32] = o[1]; p[64] = o[2]; p[96] = o[3];
+    end += 4;
+  }
+  // at least four draws available afterwards
+  __device__ __forceinline__ void prime() {
+    if (end - head <= 4u) refill();
+  }
+  // a draw known to be available
+  __device__ __forceinline__ float take() {
+    const uint32_t x = base[32 * (head & (kRingWords - 1))];
+    ++head;
+    return u01(x);
+  }
+  // the next draw, consumed only if `c`
+  __device__ __forceinline__ float take_if(bool c) {
+    const uint32_t x = base[32 * (head & (kRingWords - 1))];
+    head += c ? 1u : 0u;
+    return u01(x);
+  }
+  __device__ __forceinline__ float next() {
+    if (head == end) refill();
+    return take();
+  }
 };
 
 // ---- samplers over raw grids (index (x*res+y)*res+z) --------------------------

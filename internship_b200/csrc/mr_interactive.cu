@@ -88,12 +88,9 @@ __device__ __forceinline__ uint32_t pack_bgra(F3 res, float exposure, int tone) 
 // ---- per-frame delta tracking with histograms -------------------------------------
 
 struct InterArgs {
-  Medium m;
-  PathScene sc;
-  CameraModel cam;
-  uint32_t seed;
-  int frame, fnum, checker, flip;
-  float* accum;
+  int W, H;
+  int fnum, checker, flip;
+  float* accum;  // in: this frame's radiance at the rendered pixels; out: the running mean
   mr_histogram* hist;
   double* mom;  // 5 x npx FP64 sums: r, g, b, l, l^2
   size_t npx;
@@ -112,8 +109,10 @@ __global__ void k_seed_moments(const float* __restrict__ accum, const mr_histogr
   mom[4 * npx + p] = (double)hist[p].x2 * n;
 }
 
+// Blends the frame's paths (launch_path_frame wrote their radiance to accum)
+// into the histograms, the FP64 sums and the running means.
 __global__ void __launch_bounds__(128) k_interactive_pt(InterArgs a) {
-  const int W = a.cam.width, H = a.cam.height;
+  const int W = a.W, H = a.H;
   const int per_row = a.checker ? (W + 1) / 2 : W;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= per_row * H) return;
@@ -121,13 +120,8 @@ __global__ void __launch_bounds__(128) k_interactive_pt(InterArgs a) {
   const int col = a.checker ? 2 * c + ((row + a.flip) & 1) : c;
   if (col >= W) return;
   const int pix = row * W + col;
-  TrackStats st{0, 0};
-  Rng rng;
-  rng.init(a.seed, (uint32_t)pix, (uint32_t)a.frame, TAG_PT);
-  const float jx = rng.next(), jy = rng.next();
-  float tt;
-  F3 L = path_radiance(a.m, a.sc, rng, a.cam.ori, camera_dir(a.cam, row, col, jx, jy), &tt, st);
-  L = vmax(L, f3(0, 0, 0));
+  float* acc = a.accum + 3 * (size_t)pix;
+  const F3 L = f3(acc[0], acc[1], acc[2]);
   mr_histogram& h = a.hist[pix];
   double* m = a.mom + pix;
   const size_t N = a.npx;
@@ -154,7 +148,6 @@ __global__ void __launch_bounds__(128) k_interactive_pt(InterArgs a) {
   m[3 * N] = s3;
   m[4 * N] = s4;
   const double inv = 1.0 / (double)(1 + a.fnum);
-  float* acc = a.accum + 3 * (size_t)pix;
   acc[0] = (float)(s0 * inv);
   acc[1] = (float)(s1 * inv);
   acc[2] = (float)(s2 * inv);
@@ -423,6 +416,8 @@ __global__ void k_reproject_pack(const float* accum, mr_histogram* hist, uint32_
 extern int check_params(const mr_render_params* p);
 extern CameraModel make_camera(const mr_render_params* p);
 extern PathScene make_path_scene(const mr_render_params* p);
+int launch_path_frame(Volume* v, const mr_render_params* p, uint32_t sample, int checker, int flip, float* dev_rgb,
+                      cudaStream_t s);
 int render_neural_dist(Volume* v, const Network* net, const mr_render_params* p, float* dev_rgb, float* dev_dist,
                        cudaStream_t s);
 
@@ -480,14 +475,8 @@ extern "C" int mr_render_interactive(mr_volume* h, const mr_network* net, const 
   const int fnum = it->checkerboard ? it->frame_index / 2 : it->frame_index;
   if (p->render_type == MR_RT_PT) {
     InterArgs a;
-    a.m = Medium{v->density, v->res, v->max_density, p->tr_scale, 0};
-    rc = density_gather_texture(v, s, &a.m.tex);
-    if (rc) return rc;
-    a.sc = make_path_scene(p);
-    attach_env(a.sc, v);
-    a.cam = make_camera(p);
-    a.seed = p->seed;
-    a.frame = it->frame_index;
+    a.W = W;
+    a.H = H;
     a.fnum = fnum;
     a.checker = it->checkerboard ? 1 : 0;
     a.flip = it->frame_index & 1;
@@ -515,6 +504,8 @@ extern "C" int mr_render_interactive(mr_volume* h, const mr_network* net, const 
     }
     a.mom = v->mom;
     a.npx = npx;
+    rc = launch_path_frame(v, p, (uint32_t)it->frame_index, a.checker, a.flip, dev_accum, s);
+    if (rc) return rc;
     const int per_row = a.checker ? (W + 1) / 2 : W;
     const long long n = (long long)per_row * H;
     k_interactive_pt<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(a);

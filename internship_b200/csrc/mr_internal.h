@@ -18,6 +18,9 @@ namespace mr {
 // Counters kept per volume on the device ([0] density fetches, [1] paths,
 // [2] loop-cap hits, [3] active neural pixels, [4..7] scratch).
 constexpr int kCounters = 8;
+// One more word behind them: the work queue of launch_path_frame, which the
+// counters' resets leave alone.
+constexpr int kCounterWords = kCounters + 1;
 
 // Optional per-stage CUDA-event timing (mr_volume_set_timing).
 enum Stage {

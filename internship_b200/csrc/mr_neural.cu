@@ -99,9 +99,11 @@ __device__ __forceinline__ unsigned claim_slot(unsigned* counter) {
 // active record (job = its batch job, -1 for a single render).
 __device__ __forceinline__ unsigned trace_pixel(const Medium& m, const PathScene& sc, const CameraModel& cam,
                                                 uint32_t seed, uint32_t frame_index, int pix, float* out,
-                                                float* dist, const Records& rec, int job, TrackStats& st) {
+                                                float* dist, const Records& rec, int job, uint32_t* ring,
+                                                TrackStats& st) {
   int row = pix / cam.width, col = pix - row * cam.width;
-  Rng rng;
+  RngRing rng;
+  rng.attach(ring);
   rng.init(seed, (uint32_t)pix, frame_index, TAG_NN);
   float jx = rng.next(), jy = rng.next();
   F3 dir = camera_dir(cam, row, col, jx, jy);
@@ -116,10 +118,6 @@ __device__ __forceinline__ unsigned trace_pixel(const Medium& m, const PathScene
     active = next_vertex(m, rng, sc.alpha, 0.0f, sp, dir, maxd, p0, p1, st);
     if (active) pos = p0;
   }
-  Frame f;
-  F3 ly, lz;
-  frame_from(rng, dir, f.X, f.Y, f.Z);
-  frame_from(rng, sc.L, f.LX, ly, lz);
   if (dist) dist[pix] = active ? length(cam.ori - pos) : -1.0f;
   if (!active) {
     const F3 e = sky(sc, dir);  // SkyBox(dir) for pixels that see no medium
@@ -128,6 +126,10 @@ __device__ __forceinline__ unsigned trace_pixel(const Medium& m, const PathScene
     out[3 * (size_t)pix + 2] = fmaxf(e.z, 0.0f);
     return 0;
   }
+  Frame f;
+  F3 ly, lz;
+  frame_from(rng, dir, f.X, f.Y, f.Z);
+  frame_from(rng, sc.L, f.LX, ly, lz);
   float d2 = ray_box_distance(pos, f.LX);
   float ph = hg_phase(dot(f.X, f.LX), sc.g);
   float tr = transmittance(m, rng, pos, f.LX, d2, sc.alpha, st) * ph;
@@ -160,14 +162,18 @@ __device__ __forceinline__ void trace_counters(unsigned long long* counters, con
   }
 }
 
-// Bound by the latency of dependent density fetches: registers capped for
-// twelve 128-thread blocks per SM.
-__global__ void __launch_bounds__(128, 12) k_nn_trace(NNTraceArgs a) {
+// Bound by the latency of dependent density fetches (long_scoreboard 60 % of
+// the stalls, issue active 62 %): ten 128-thread blocks per SM. At 1080p over
+// a 512^3 cloud: 0.420 ms with draws in registers and twelve blocks; with the
+// draws in shared memory 0.422 ms at twelve blocks (spills), 0.359 at ten,
+// 0.375 at eight.
+__global__ void __launch_bounds__(128, 10) k_nn_trace(NNTraceArgs a) {
   int pix = blockIdx.x * blockDim.x + threadIdx.x;
   int npx = a.cam.width * a.cam.height;
+  __shared__ uint32_t ring[kRingWords * 128];
   TrackStats st{0, 0};
   unsigned act = 0;
-  if (pix < npx) act = trace_pixel(a.m, a.sc, a.cam, a.seed, a.frame_index, pix, a.out, a.dist, a.rec, -1, st);
+  if (pix < npx) act = trace_pixel(a.m, a.sc, a.cam, a.seed, a.frame_index, pix, a.out, a.dist, a.rec, -1, ring, st);
   trace_counters(a.counters, st, act);
 }
 
@@ -1125,6 +1131,7 @@ struct BatchJob {
 __global__ void __launch_bounds__(256) k_trace_batch(const BatchJob* __restrict__ jobs, int njobs, long long w0,
                                                      long long w1, const BatchOut* __restrict__ bout, Records rec,
                                                      unsigned long long* counters) {
+  extern __shared__ uint32_t ring[];  // kRingWords * blockDim.x
   const long long p = w0 + (long long)blockIdx.x * blockDim.x + threadIdx.x;
   TrackStats st{0, 0};
   unsigned act = 0;
@@ -1146,7 +1153,7 @@ __global__ void __launch_bounds__(256) k_trace_batch(const BatchJob* __restrict_
     const bool mine = p < w1 && lo == jj;
     if (mine) {
       const BatchJob& j = jobs[jj];
-      act = trace_pixel(j.m, j.sc, j.cam, j.seed, j.frame, (int)(p - j.pix0), bout[jj].out, nullptr, rec, jj, st);
+      act = trace_pixel(j.m, j.sc, j.cam, j.seed, j.frame, (int)(p - j.pix0), bout[jj].out, nullptr, rec, jj, ring, st);
     }
     todo &= ~__ballot_sync(0xffffffffu, mine);
   }
@@ -1308,7 +1315,7 @@ static int batch_launches(Batch& b, const Network* net, cudaStream_t s) {
     const long long w1 = std::min(b.total, w0 + b.wave);
     MR_CUDA(cudaMemsetAsync(rec.count, 0, sizeof(unsigned), s));
     const unsigned tgrid = (unsigned)((w1 - w0 + b.trace_block - 1) / b.trace_block);
-    k_trace_batch<<<tgrid, b.trace_block, 0, s>>>(b.d_jobs, nj, w0, w1, b.d_out, rec, b.counters);
+    k_trace_batch<<<tgrid, b.trace_block, kRingWords * sizeof(uint32_t) * b.trace_block, s>>>(b.d_jobs, nj, w0, w1, b.d_out, rec, b.counters);
     MR_CUDA(cudaGetLastError());
     const unsigned ggrid = (unsigned)((w1 - w0 + b.gather_block - 1) / b.gather_block);
     if (hw)

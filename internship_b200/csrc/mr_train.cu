@@ -115,48 +115,71 @@ struct LabelArgs {
 };
 
 // Work item = (label k, chunk of `chunk` samples), claimed from a global queue
-// so that long and short paths balance across the grid. Sample s of label k
-// uses the stream (seed; k, s, ., TAG_LABEL).
-__global__ void __launch_bounds__(128) k_train_labels(LabelArgs a) {
-  const unsigned long long per = (unsigned long long)((a.spp + a.chunk - 1) / a.chunk);
-  const unsigned long long total = per * (unsigned long long)a.n;
-  TrackStats st{0, 0};
-  for (;;) {
-    const unsigned long long w = claim_work(a.queue);
-    if (w >= total) break;
-    const int k = (int)(w / per);
-    const int s0 = (int)(w % per) * a.chunk;
-    const int s1 = min(a.spp, s0 + a.chunk);
-    const F3 p0 = f3(a.pos[3 * k], a.pos[3 * k + 1], a.pos[3 * k + 2]);
-    const F3 d0 = f3(a.dir[3 * k], a.dir[3 * k + 1], a.dir[3 * k + 2]);
-    double acc = 0.0;
-    for (int s = s0; s < s1; ++s) {
-      Rng rng;
-      rng.init(a.seed, (uint32_t)k, (uint32_t)s, TAG_LABEL);
-      const float e0 = rng.next(), e1 = rng.next();
-      F3 rd = hg_sample_dir(e0, e1, d0, a.g);
-      F3 sp = p0;
-      float rate = 1.0f, res = 0.0f;
-      for (int b = 0; b < a.max_bounces; ++b) {
-        F3 np, nd;
-        float dis = ray_box_distance(sp, rd);
-        if (!next_vertex(a.m, rng, a.alpha, a.g, sp, rd, dis, np, nd, st)) {
-          // escaped: SkyBox(dir) * rate (core/render.cuh:294-296), channel 0
-          if (a.env.env_map) res = res + rate * sky(a.env, rd).x;
-          break;
-        }
-        sp = np;
-        rate = rate * 1.001f * a.albedo;
-        dis = ray_box_distance(sp, a.L);
-        const float ph = hg_phase(dot(rd, a.L), a.g);
-        res = res + rate * (transmittance(a.m, rng, sp, a.L, dis, a.alpha, st) * ph);
-        rd = nd;
-      }
-      acc += (double)res;
+// so that long and short paths balance across the grid; a lane runs the
+// samples of its item one after the other as paths of run_paths. Sample s of
+// label k uses the stream (seed; k, s, ., TAG_LABEL).
+// 4096 labels x 256 spp on a 256^3 cloud: 22.0 ms with a chunk of 64 samples a
+// lane (16 k lanes at work on a GPU that holds 114 k) and whole paths in
+// lockstep; 7.4 ms with run_paths; 1.03 ms with the chunk sized to the grid.
+// Density through texture gathers instead of texel loads: within 2 %, so no
+// layered copy of the grid is made for labels.
+struct LabelPaths {
+  const LabelArgs& a;
+  unsigned long long per, total;
+  RngRing rng;
+  F3 p0, d0;
+  double acc;
+  float rate, res;
+  int k, s, s1;  // label, next sample and end of the item (s == s1: no item)
+
+  __device__ __forceinline__ bool begin(F3& pos, F3& rd) {
+    if (s == s1) {
+      if (k >= 0) atomicAdd(a.sum + k, acc);
+      const unsigned long long w = claim_work(a.queue);
+      if (w >= total) return false;
+      k = (int)(w / per);
+      s = (int)(w % per) * a.chunk;
+      s1 = min(a.spp, s + a.chunk);
+      p0 = f3(a.pos[3 * k], a.pos[3 * k + 1], a.pos[3 * k + 2]);
+      d0 = f3(a.dir[3 * k], a.dir[3 * k + 1], a.dir[3 * k + 2]);
+      acc = 0.0;
     }
-    atomicAdd(a.sum + k, acc);
+    rng.init(a.seed, (uint32_t)k, (uint32_t)s, TAG_LABEL);
+    ++s;
+    const float e0 = rng.next(), e1 = rng.next();
+    rd = hg_sample_dir(e0, e1, d0, a.g);
+    pos = p0;
+    rate = 1.0f;
+    res = 0.0f;
+    return true;
   }
+  // SkyBox(dir) * rate (core/render.cuh:294-296), channel 0
+  __device__ __forceinline__ void escape(F3 rd) {
+    if (a.env.env_map) res = res + rate * sky(a.env, rd).x;
+  }
+  __device__ __forceinline__ void scatter() { rate = rate * 1.001f * a.albedo; }
+  __device__ __forceinline__ void light(float x) { res = res + rate * x; }
+  __device__ __forceinline__ void finish() { acc += (double)res; }
+};
+
+__global__ void __launch_bounds__(128) k_train_labels(const __grid_constant__ LabelArgs a) {
+  __shared__ uint32_t ring[kRingWords * 128];
+  const unsigned long long per = (unsigned long long)((a.spp + a.chunk - 1) / a.chunk);
+  TrackStats st{0, 0};
+  LabelPaths lp{a, per, per * (unsigned long long)a.n, {}, {}, {}, 0.0, 0.0f, 0.0f, -1, 0, 0};
+  lp.rng.attach(ring);
+  run_paths(lp, a.m, a.alpha, a.g, a.L, a.max_bounces, st);
   if (st.caps) atomicAdd(a.caps, st.caps);
+}
+
+// Resident grid of the label kernel on the current device.
+static int label_grid() {
+  static DeviceCache cache;
+  return cache.get([] {
+    int per_sm = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_train_labels, 128, 0);
+    return std::max(per_sm, 1) * sm_count();
+  });
 }
 
 // Frames of NNPredict for view direction dir[k] and light L: stream
@@ -469,13 +492,19 @@ extern "C" int mr_train_labels(mr_volume* h, const float* dev_pos, const float* 
   Volume* v = &h->v;
   cudaStream_t s = (cudaStream_t)stream;
   MR_CUDA(cudaMemsetAsync(v->d_counters, 0, kCounters * sizeof(unsigned long long), s));
+  if (max_bounces == 0) return MR_OK;  // no vertex: every sum stays as it is
   LabelArgs a;
-  a.m = Medium{v->density, v->res, v->max_density, 1.0f};
+  a.m = Medium{v->density, v->res, v->max_density, 1.0f, 0};
   a.pos = dev_pos;
   a.dir = dev_dir;
   a.n = n;
   a.spp = spp;
-  a.chunk = std::min(spp, 64);
+  // Samples a lane runs per claimed item: enough items for eight per resident
+  // lane, so that labels in small numbers still fill the GPU, and at most 64
+  // samples per FP64 atomic.
+  const int grid = label_grid();
+  a.chunk = (int)std::min<long long>(64, std::max<long long>(1, (long long)n * spp / (8ll * 128 * grid)));
+  a.chunk = std::min(a.chunk, spp);
   a.max_bounces = max_bounces;
   a.L = normalize(to_f3(light_dir));
   a.alpha = alpha;
@@ -488,7 +517,7 @@ extern "C" int mr_train_labels(mr_volume* h, const float* dev_pos, const float* 
   a.env = PathScene{};
   a.env.env = f3(1.0f, 1.0f, 1.0f);  // the map at unit scale; black without one
   attach_env(a.env, v);
-  k_train_labels<<<sm_count() * 16, 128, 0, s>>>(a);
+  k_train_labels<<<grid, 128, 0, s>>>(a);
   MR_CUDA(cudaGetLastError());
   return MR_OK;
 }

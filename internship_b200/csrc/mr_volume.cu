@@ -434,8 +434,8 @@ int mr_volume_create(int32_t resolution, mr_volume** out) {
   if (e == cudaSuccess) e = cudaMalloc(&v->tr, kTrTotal * sizeof(float));
   if (e == cudaSuccess) e = cudaMalloc(&v->lut, kLut * kLut * sizeof(float));
   if (e == cudaSuccess) e = cudaMalloc(&v->d_max, sizeof(float));
-  if (e == cudaSuccess) e = cudaMalloc(&v->d_counters, kCounters * sizeof(unsigned long long));
-  if (e == cudaSuccess) e = cudaMemset(v->d_counters, 0, kCounters * sizeof(unsigned long long));
+  if (e == cudaSuccess) e = cudaMalloc(&v->d_counters, kCounterWords * sizeof(unsigned long long));
+  if (e == cudaSuccess) e = cudaMemset(v->d_counters, 0, kCounterWords * sizeof(unsigned long long));
   if (e == cudaSuccess) e = cudaMemset(v->density, 0, n * sizeof(float));
   if (e != cudaSuccess) {
     mr_volume_destroy(h);
