@@ -12,12 +12,10 @@
 //    its view direction, FP64 accumulation over the samples of a label.
 //  * k_train_frames: the two random frames NNPredict draws
 //    (core/render.cuh:355-369,469-523) for the view and light directions.
-//  * k_train_fwd_bwd: one thread per training row: the network of
-//    core/radiancePredict.cu:370-485 (first albedo channel) forward in fp32
-//    with every pre-activation kept in local memory, the loss
-//    (X - log(1 + label/srp))^2 on the head output X, and the backward pass;
-//    weight gradients are summed over the warp with shuffles and added to a
-//    global fp32 gradient with one atomic per warp and weight.
+//  * the step: the network of core/radiancePredict.cu:370-485 (first albedo
+//    channel) forward, the loss (X - log(1 + label/srp))^2 on the head output
+//    X, and the backward pass, in fp32 over tiles of rows (mr_train_tile.cu)
+//    or with the head's products on the tensor cores (mr_train_tc.cu).
 //  * k_adam: Adam with bias correction on the fp32 master weights.
 #include <algorithm>
 #include <cmath>
@@ -197,213 +195,7 @@ __global__ void k_train_frames(const float* dir, int n, F3 L, uint32_t seed, flo
   f[6] = Z.x; f[7] = Z.y; f[8] = Z.z; f[9] = LX.x; f[10] = LX.y; f[11] = LX.z;
 }
 
-// ---- network forward / backward ----------------------------------------------------
-
-// Trunk blocks in evaluation order: main trunk (radiancePredict.cu:396-421),
-// then the light-direction trunk (:424-437). Per block: width S, mode (0 SE +
-// ADD3, 1 SERES + ADD3, 2 SERES + REP3), descriptor offset, pool index, SE
-// weights and the three branch layers (density, transmittance, phase).
-struct TrainArgs {
-  const float* w;       // fp32 master weights (blob layout)
-  float* grad;          // fp32 gradient accumulator (blob layout)
-  const float* desc;    // n x 576, row-major
-  const float* aux;     // n x 5 (g, gamma, srp.xyz)
-  const float* label;   // n radiance labels
-  int n;
-  float inv_batch;      // loss weight 1/n
-  float* loss;          // summed (X - T)^2 / n
-  float* h0;            // TR_TRUNK_FWD: the head input per row (n x 128), written
-  const float* dh0;     // TR_TRUNK_BWD: its gradient per row (n x 128), read
-};
-
-// Parts of the training step the kernel runs: the whole network (fp32), or
-// the two halves around the tensor-core head of the BF16 step (the trunks'
-// forward up to the head input, and the trunks' backward from its gradient,
-// the forward recomputed).
-enum { TR_FULL = 0, TR_TRUNK_FWD = 1, TR_TRUNK_BWD = 2 };
-
-template <int MODE>
-__global__ void __launch_bounds__(128) k_train_fwd_bwd(TrainArgs a) {
-  const int k0 = blockIdx.x * blockDim.x + threadIdx.x;
-  const bool valid = k0 < a.n;
-  const int k = valid ? k0 : a.n - 1;
-  const float* __restrict__ W = a.w;
-  float* G = a.grad;
-  const float* d = a.desc + (size_t)k * 576;
-  const float g = a.aux[5 * (size_t)k], gamma = a.aux[5 * (size_t)k + 1], srp = a.aux[5 * (size_t)k + 2];
-  const TrainTables& T = c_tt;
-
-  // ---- forward, keeping what the backward pass needs
-  float X[12][3][32], YP[12][3][32], Gt[12][3], HP[12][8], TM[12][8];
-  float y[3][32];
-  float pool[75];
-  float YM[3][32], YL[3][8], CMP[3][32], CLP[3][8];
-#pragma unroll 1
-  for (int b = 0; b < 12; ++b) {
-    const int S = T.S[b], mode = T.mode[b], from = T.from[b];
-    float mean[3], mx[3];
-    for (int br = 0; br < 3; ++br) {
-      float s = 0.0f, m = -10000.0f;
-      for (int i = 0; i < S; ++i) {
-        const float v = d[br * 192 + from + i];
-        s += v;
-        m = fmaxf(m, v);
-      }
-      mean[br] = s / (float)S;
-      mx[br] = m;
-      pool[T.pid[b] + br] = mean[br];
-      pool[36 + T.pid[b] + br] = mx[br];
-    }
-    const float tmp[8] = {mean[0], mean[1], mean[2], mx[0], mx[1], mx[2], g, gamma};
-    float h[8];
-    for (int i = 0; i < 8; ++i) {
-      float s = 0.0f;
-      for (int j = 0; j < 8; ++j) s += tmp[j] * __ldg(W + T.se0[b] + j + i * 8);
-      TM[b][i] = tmp[i];
-      HP[b][i] = s;
-      h[i] = relu(s);
-    }
-    for (int i = 0; i < 3; ++i) {
-      float s = 0.0f;
-      for (int j = 0; j < 8; ++j) s += h[j] * __ldg(W + T.se1[b] + j + i * 8);
-      Gt[b][i] = sigmoid(s);
-    }
-    for (int br = 0; br < 3; ++br) {
-      for (int i = 0; i < S; ++i) {
-        const float v = d[br * 192 + from + i] * Gt[b][br];
-        X[b][br][i] = mode == 0 ? v : v + y[br][i];
-      }
-      dense_fwd(W + T.w[b][br], W + T.b[b][br], X[b][br], S, S, YP[b][br]);
-      for (int i = 0; i < S; ++i) {
-        const float s = d[br * 192 + from + i];
-        if (mode == 2) {
-          y[br][i] = relu(YP[b][br][i]);
-          y[br][S + i] = s;
-        } else {
-          y[br][i] = relu(YP[b][br][i]) + s;
-        }
-      }
-    }
-    if (b == 7) {
-      for (int br = 0; br < 3; ++br) {
-        for (int i = 0; i < 32; ++i) YM[br][i] = y[br][i];
-        dense_fwd(W + T.l81w[br], W + T.l81b[br], YM[br], 32, 32, CMP[br]);
-      }
-    }
-    if (b == 11) {
-      for (int br = 0; br < 3; ++br) {
-        for (int i = 0; i < 8; ++i) YL[br][i] = y[br][i];
-        dense_fwd(W + T.ld41w[br], W + T.ld41b[br], YL[br], 8, 8, CLP[br]);
-      }
-    }
-  }
-  pool[72] = g; pool[73] = gamma; pool[74] = srp;
-  float FP[16], SW[16], SPP[6], SP[6], X8P[8];
-  dense_fwd(W + T.f1, nullptr, pool, 75, 16, FP);
-  for (int j = 0; j < 16; ++j) SW[j] = relu(FP[j]);
-  dense_fwd(W + T.f2, nullptr, SW, 16, 6, SPP);
-  for (int i = 0; i < 6; ++i) SP[i] = sigmoid(SPP[i]);
-  const float gg3[3] = {g, gamma, srp};
-  dense_fwd(W + T.ggw, W + T.ggb, gg3, 3, 8, X8P);
-  float H0[128];
-  for (int br = 0; br < 3; ++br)
-    for (int i = 0; i < 32; ++i) H0[32 * br + i] = relu(CMP[br][i]) * SP[br];
-  for (int br = 0; br < 3; ++br)
-    for (int i = 0; i < 8; ++i) H0[96 + 8 * br + i] = relu(CLP[br][i]) * SP[3 + br];
-  for (int i = 0; i < 8; ++i) H0[120 + i] = relu(X8P[i]);
-  if constexpr (MODE == TR_TRUNK_FWD) {
-    if (valid) {
-      float4* o = reinterpret_cast<float4*>(a.h0 + (size_t)k * 128);
-      for (int i = 0; i < 32; ++i) o[i] = make_float4(H0[4 * i], H0[4 * i + 1], H0[4 * i + 2], H0[4 * i + 3]);
-    }
-    return;
-  }
-  float dH0[128];
-  if constexpr (MODE == TR_TRUNK_BWD) {
-    const float4* gi = reinterpret_cast<const float4*>(a.dh0 + (size_t)k * 128);
-    for (int i = 0; i < 32; ++i) {
-      const float4 q = valid ? gi[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-      dH0[4 * i] = q.x; dH0[4 * i + 1] = q.y; dH0[4 * i + 2] = q.z; dH0[4 * i + 3] = q.w;
-    }
-  } else {
-    float A1P[128], A1[128], A2P[64], A2[64], A3P[32], A3[32];
-    dense_fwd(W + T.lc0w, W + T.lc0b, H0, 128, 128, A1P);
-    for (int i = 0; i < 128; ++i) A1[i] = relu(A1P[i]);
-    dense_fwd(W + T.lc1w, W + T.lc1b, A1, 128, 64, A2P);
-    for (int i = 0; i < 64; ++i) A2[i] = relu(A2P[i]);
-    dense_fwd(W + T.lc2w, W + T.lc2b, A2, 64, 32, A3P);
-    for (int i = 0; i < 32; ++i) A3[i] = relu(A3P[i]);
-    float d3[32], dA3[32], d2[64], dA2[64], d1[128], dA1[128];
-    tail_fwd_bwd(W, G, T, A3, a.label[k], srp, valid, a.inv_batch, a.loss, d3);
-    for (int i = 0; i < 32; ++i) dA3[i] = A3P[i] > 0.0f ? d3[i] : 0.0f;
-    for (int i = 0; i < 64; ++i) d2[i] = 0.0f;
-    dense_bwd(W + T.lc2w, G + T.lc2w, G + T.lc2b, A2, dA3, d2, 64, 32);
-    for (int i = 0; i < 64; ++i) dA2[i] = A2P[i] > 0.0f ? d2[i] : 0.0f;
-    for (int i = 0; i < 128; ++i) d1[i] = 0.0f;
-    dense_bwd(W + T.lc1w, G + T.lc1w, G + T.lc1b, A1, dA2, d1, 128, 64);
-    for (int i = 0; i < 128; ++i) { dA1[i] = A1P[i] > 0.0f ? d1[i] : 0.0f; dH0[i] = 0.0f; }
-    dense_bwd(W + T.lc0w, G + T.lc0w, G + T.lc0b, H0, dA1, dH0, 128, 128);
-  }
-  // head input: gated combs and LGGS
-  float dSP[6] = {0, 0, 0, 0, 0, 0};
-  float dCM[3][32], dCL[3][8];
-  for (int br = 0; br < 3; ++br)
-    for (int i = 0; i < 32; ++i) {
-      const float dh = dH0[32 * br + i];
-      dSP[br] += dh * relu(CMP[br][i]);
-      dCM[br][i] = CMP[br][i] > 0.0f ? dh * SP[br] : 0.0f;
-    }
-  for (int br = 0; br < 3; ++br)
-    for (int i = 0; i < 8; ++i) {
-      const float dh = dH0[96 + 8 * br + i];
-      dSP[3 + br] += dh * relu(CLP[br][i]);
-      dCL[br][i] = CLP[br][i] > 0.0f ? dh * SP[3 + br] : 0.0f;
-    }
-  {
-    float dX8[8];
-    for (int i = 0; i < 8; ++i) dX8[i] = X8P[i] > 0.0f ? dH0[120 + i] : 0.0f;
-    dense_bwd(W + T.ggw, G + T.ggw, G + T.ggb, gg3, dX8, nullptr, 3, 8);
-    float dSPP[6], dSW[16], dFP[16];
-    for (int i = 0; i < 6; ++i) dSPP[i] = dSP[i] * SP[i] * (1.0f - SP[i]);
-    for (int j = 0; j < 16; ++j) dSW[j] = 0.0f;
-    dense_bwd(W + T.f2, G + T.f2, nullptr, SW, dSPP, dSW, 16, 6);
-    for (int j = 0; j < 16; ++j) dFP[j] = FP[j] > 0.0f ? dSW[j] : 0.0f;
-    dense_bwd(W + T.f1, G + T.f1, nullptr, pool, dFP, nullptr, 75, 16);
-  }
-  // trunks, last block first; dy holds the gradient of the running y
-  float dy[3][32];
-#pragma unroll 1
-  for (int trunk = 0; trunk < 2; ++trunk) {
-    const int last = trunk == 0 ? 11 : 7, first = trunk == 0 ? 8 : 0;
-    for (int br = 0; br < 3; ++br)
-      for (int i = 0; i < 32; ++i) dy[br][i] = 0.0f;
-    if (trunk == 0) {
-      for (int br = 0; br < 3; ++br) dense_bwd(W + T.ld41w[br], G + T.ld41w[br], G + T.ld41b[br], YL[br], dCL[br], dy[br], 8, 8);
-    } else {
-      for (int br = 0; br < 3; ++br) dense_bwd(W + T.l81w[br], G + T.l81w[br], G + T.l81b[br], YM[br], dCM[br], dy[br], 32, 32);
-    }
-#pragma unroll 1
-    for (int b = last; b >= first; --b) {
-      const int S = T.S[b], mode = T.mode[b], from = T.from[b];
-      float dgate[3];
-      for (int br = 0; br < 3; ++br) {
-        float dp[32], dx[32];
-        for (int o = 0; o < S; ++o) { dp[o] = YP[b][br][o] > 0.0f ? dy[br][o] : 0.0f; dx[o] = 0.0f; }
-        dense_bwd(W + T.w[b][br], G + T.w[b][br], G + T.b[b][br], X[b][br], dp, dx, S, S);
-        float s = 0.0f;
-        for (int i = 0; i < S; ++i) s += dx[i] * d[br * 192 + from + i];
-        dgate[br] = s;
-        for (int i = 0; i < 32; ++i) dy[br][i] = (mode != 0 && i < S) ? dx[i] : 0.0f;
-      }
-      float dgp[3], h[8], dh[8];
-      for (int i = 0; i < 3; ++i) dgp[i] = dgate[i] * Gt[b][i] * (1.0f - Gt[b][i]);
-      for (int j = 0; j < 8; ++j) { h[j] = relu(HP[b][j]); dh[j] = 0.0f; }
-      dense_bwd(W + T.se1[b], G + T.se1[b], nullptr, h, dgp, dh, 8, 3);
-      for (int j = 0; j < 8; ++j) dh[j] = HP[b][j] > 0.0f ? dh[j] : 0.0f;
-      dense_bwd(W + T.se0[b], G + T.se0[b], nullptr, TM[b], dh, nullptr, 8, 8);
-    }
-  }
-}
+// ---- the training step -------------------------------------------------------------
 
 __global__ void k_adam(float* w, float* m, float* v, float* grad, int n, float lr, float b1, float b2, float eps,
                        float c1, float c2) {
@@ -426,19 +218,20 @@ struct Trainer {
   float* loss = nullptr;
   int step = 0;
   float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
-  // MR_PREC_BF16: the head on the tensor cores (mr_train_tc.cu) between the
-  // trunks' forward and backward halves, which exchange the head input and
-  // its gradient per row through h0 / dh0 (cap rows each).
   int precision = MR_PREC_FP32;
-  float* h0 = nullptr;
-  float* dh0 = nullptr;
+  // The step's buffers (TrainWork) for up to `cap` rows, grown on demand to
+  // at most kStepRows: larger batches run in pieces.
+  float* work = nullptr;
   size_t cap = 0;
   uint8_t* img = nullptr;  // BF16 head weights, rebuilt from w every step
   int* err = nullptr;      // set when a bounded wait of the head kernel gives up
 };
 
-int launch_head_tc(const float* w, float* grad, uint8_t* img, const float* h0, float* dh0, const float* aux,
-                   const float* label, int n, float inv_batch, float* loss, int* err, cudaStream_t s);
+// Rows of one pass of a step: 65,536 rows take 136 MB of buffers.
+constexpr int kStepRows = 65536;
+
+int launch_head_pack(const float* w, uint8_t* img, cudaStream_t s);
+int launch_head_tc(const TrainArgs& a, const uint8_t* img, int* err, cudaStream_t s);
 size_t head_image_bytes();
 
 }  // namespace mr
@@ -566,8 +359,7 @@ extern "C" int mr_trainer_destroy(mr_trainer* h) {
   cudaFree(h->t.v);
   cudaFree(h->t.grad);
   cudaFree(h->t.loss);
-  cudaFree(h->t.h0);
-  cudaFree(h->t.dh0);
+  cudaFree(h->t.work);
   cudaFree(h->t.img);
   cudaFree(h->t.err);
   delete h;
@@ -601,41 +393,55 @@ static int head_error(Trainer& t) {
 
 static int fwd_bwd(Trainer& t, const float* desc, const float* aux, const float* label, int n, cudaStream_t s) {
   MR_CUDA(cudaMemsetAsync(t.loss, 0, sizeof(float), s));
+  const size_t need = (size_t)(std::min(n, kStepRows) + kTrainRows - 1) / kTrainRows * kTrainRows;
+  // Under a capture that comes before any call of this size, the buffers are
+  // nodes of the graph instead.
+  float* temp = nullptr;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (need > t.cap && s && cudaStreamIsCapturing(s, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusActive) {
+    MR_CUDA(cudaMallocAsync(&temp, need * kTrainWorkFloats * sizeof(float), s));
+  } else if (need > t.cap) {
+    cudaFree(t.work);
+    t.work = nullptr;
+    t.cap = 0;
+    cudaError_t e = cudaMalloc(&t.work, need * kTrainWorkFloats * sizeof(float));
+    if (e != cudaSuccess) return set_error(MR_ERR_NOMEM, "training buffers for %zu rows: %s", need, cudaGetErrorString(e));
+    t.cap = need;
+  }
   TrainArgs a;
   a.w = t.w;
   a.grad = t.grad;
-  a.desc = desc;
-  a.aux = aux;
-  a.label = label;
-  a.n = n;
   a.inv_batch = 1.0f / (float)n;
   a.loss = t.loss;
-  a.h0 = nullptr;
-  a.dh0 = nullptr;
-  const unsigned grid = (unsigned)((n + 127) / 128);
-  if (t.precision != MR_PREC_BF16) {
-    k_train_fwd_bwd<TR_FULL><<<grid, 128, 0, s>>>(a);
-    MR_CUDA(cudaGetLastError());
-    return MR_OK;
+  float* p = temp ? temp : t.work;
+  a.wk.rows = temp ? need : t.cap;
+  auto take = [&](size_t floats) {
+    float* q = p;
+    p += floats * a.wk.rows;
+    return q;
+  };
+  a.wk.h0 = take(128);
+  a.wk.dh0 = take(128);
+  a.wk.pool = take(72);
+  a.wk.gate = take(36);
+  a.wk.sp = take(6);
+  a.wk.dgate = take(72);
+  a.wk.dsp = take(12);
+  a.wk.a3 = take(32);
+  a.wk.da3 = take(32);
+  const bool tc = t.precision == MR_PREC_BF16;
+  int rc = tc ? launch_head_pack(t.w, t.img, s) : (int)MR_OK;
+  for (int r0 = 0; r0 < n && !rc; r0 += kStepRows) {
+    a.n = std::min(kStepRows, n - r0);
+    a.desc = desc + (size_t)r0 * 576;
+    a.aux = aux + (size_t)r0 * 5;
+    a.label = label + r0;
+    rc = launch_train_trunk_fwd(a, s);
+    if (!rc) rc = tc ? launch_head_tc(a, t.img, t.err, s) : launch_train_head(a, s);
+    if (!rc) rc = launch_train_trunk_bwd(a, s);
   }
-  if ((size_t)n > t.cap) {
-    cudaFree(t.h0);
-    cudaFree(t.dh0);
-    t.h0 = t.dh0 = nullptr;
-    t.cap = 0;
-    MR_CUDA(cudaMalloc(&t.h0, (size_t)n * 128 * sizeof(float)));
-    MR_CUDA(cudaMalloc(&t.dh0, (size_t)n * 128 * sizeof(float)));
-    t.cap = (size_t)n;
-  }
-  a.h0 = t.h0;
-  a.dh0 = t.dh0;
-  k_train_fwd_bwd<TR_TRUNK_FWD><<<grid, 128, 0, s>>>(a);
-  MR_CUDA(cudaGetLastError());
-  int rc = launch_head_tc(t.w, t.grad, t.img, t.h0, t.dh0, aux, label, n, a.inv_batch, t.loss, t.err, s);
-  if (rc) return rc;
-  k_train_fwd_bwd<TR_TRUNK_BWD><<<grid, 128, 0, s>>>(a);
-  MR_CUDA(cudaGetLastError());
-  return MR_OK;
+  if (temp) MR_CUDA(cudaFreeAsync(temp, s));
+  return rc;
 }
 
 extern "C" int mr_trainer_gradient(mr_trainer* h, const float* dev_desc, const float* dev_aux, const float* dev_label,

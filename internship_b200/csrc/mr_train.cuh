@@ -1,7 +1,7 @@
-// Training pieces shared by the fp32 training kernel (mr_train.cu) and the
-// BF16 tensor-core head (mr_train_tc.cu): the offsets of the network's weight
-// arrays per block, per-row dense layers with their backward passes, and the
-// head's tail (core/radiancePredict.cu:370-485).
+// Training pieces shared by the trainer (mr_train.cu), the fp32 tile kernels
+// (mr_train_tile.cu) and the BF16 tensor-core head (mr_train_tc.cu): the
+// offsets of the network's weight arrays per block
+// (core/radiancePredict.cu:370-485), the step's arguments and buffers.
 #pragma once
 #include "mr_internal.h"
 #include "mr_net_layout.cuh"
@@ -64,95 +64,40 @@ static __constant__ TrainTables c_tt = make_train_tables();
 __device__ __forceinline__ float relu(float x) { return x > 0.0f ? x : 0.0f; }
 __device__ __forceinline__ float sigmoid(float x) { return 1.0f / (1.0f + expf(-x)); }
 
-// Warp sum of v, added to G[idx] by lane 0. Every lane of the warp calls it
-// with the same idx.
-__device__ __forceinline__ void gacc(float* G, int idx, float v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  if ((threadIdx.x & 31) == 0 && v != 0.0f) atomicAdd(G + idx, v);
-}
+// Rows of a tile of the training kernels (mr_train_tile.cu).
+constexpr int kTrainRows = 64;
 
-// ypre[o] = b[o] + sum_i W[o*K + i] x[i]
-__device__ __forceinline__ void dense_fwd(const float* __restrict__ W, const float* __restrict__ B, const float* x,
-                                          int K, int N, float* ypre) {
-#pragma unroll 1
-  for (int o = 0; o < N; ++o) {
-    float a = 0.0f;
-#pragma unroll 4
-    for (int i = 0; i < K; ++i) a += x[i] * __ldg(W + o * K + i);
-    ypre[o] = a + (B ? __ldg(B + o) : 0.0f);
-  }
-}
-// Given dpre (N), input x (K): gradients of W (GW) and B (GB), and dx += W^T dpre
-// (dx may be null).
-__device__ __forceinline__ void dense_bwd(const float* __restrict__ W, float* GW, float* GB, const float* x,
-                                          const float* dpre, float* dx, int K, int N) {
-#pragma unroll 1
-  for (int o = 0; o < N; ++o) {
-    const float d = dpre[o];
-    if (!__any_sync(0xffffffffu, d != 0.0f)) continue;  // dead unit for the whole warp
-    if (GB) gacc(GB, o, d);
-#pragma unroll 4
-    for (int i = 0; i < K; ++i) gacc(GW, o * K + i, d * x[i]);
-  }
-  if (dx) {
-#pragma unroll 1
-    for (int i = 0; i < K; ++i) {
-      float a = 0.0f;
-#pragma unroll 4
-      for (int o = 0; o < N; ++o) a += __ldg(W + o * K + i) * dpre[o];
-      dx[i] += a;
-    }
-  }
-}
+// Buffers of a training step, `rows` rows each (a multiple of kTrainRows).
+// Feature-major ones hold feature f of row r at [f * rows + r].
+struct TrainWork {
+  size_t rows;
+  float* h0;     // head input, rows x 128
+  float* dh0;    // its gradient, rows x 128
+  float* pool;   // 72 features: segment means, then maxima
+  float* gate;   // 36: squeeze-excitation gates
+  float* sp;     // 6: gates of the trunk outputs
+  float* dgate;  // 2 x 36: gradients of the gates, two partial sums
+  float* dsp;    // 2 x 6: gradients of the output gates, two partial sums
+  float* a3;     // BF16 step: LC2 output after ReLU, rows x 32
+  float* da3;    // BF16 step: its gradient, 0 where a3 is 0
+};
+constexpr size_t kTrainWorkFloats = 128 + 128 + 72 + 36 + 6 + 72 + 12 + 32 + 32;  // per row
 
-// The head's tail (LX, the six residual pairs, LX12; radiancePredict.cu:454-473)
-// for one row: forward from A3 (LC2's 32 outputs after ReLU), the loss
-// (X - log(1 + label/srp))^2 / n summed over the warp into *loss, and the
-// backward to d3 = dL/dA3; weight gradients go to G. Rows with valid false
-// contribute nothing.
-__device__ __forceinline__ void tail_fwd_bwd(const float* __restrict__ W, float* G, const TrainTables& T,
-                                             const float* A3, float label, float srp, bool valid, float inv_batch,
-                                             float* loss, float* d3) {
-  float AXP[16];
-  dense_fwd(W + T.lxw, W + T.lxb, A3, 32, 16, AXP);
-  float AR[7][16], TP[6][16], TT[6][16], UP[6][16];
-  for (int i = 0; i < 16; ++i) AR[0][i] = relu(AXP[i]);
-#pragma unroll 1
-  for (int r = 0; r < 6; ++r) {
-    dense_fwd(W + T.lxrw[2 * r], W + T.lxrb[2 * r], AR[r], 16, 16, TP[r]);
-    for (int i = 0; i < 16; ++i) TT[r][i] = relu(TP[r][i]);
-    dense_fwd(W + T.lxrw[2 * r + 1], W + T.lxrb[2 * r + 1], TT[r], 16, 16, UP[r]);
-    for (int i = 0; i < 16; ++i) AR[r + 1][i] = AR[r][i] + relu(UP[r][i]);
-  }
-  float OP;
-  dense_fwd(W + T.lx12w, W + T.lx12b, AR[6], 16, 1, &OP);
-  const float Xo = relu(OP);
-  const float target = log1pf(fmaxf(label, 0.0f) / srp);
-  const float err = valid ? Xo - target : 0.0f;
-  {
-    float l = err * err * inv_batch;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-    if ((threadIdx.x & 31) == 0) atomicAdd(loss, l);
-  }
-  float dOP = 2.0f * err * inv_batch * (OP > 0.0f ? 1.0f : 0.0f);
-  float da[16];
-  for (int i = 0; i < 16; ++i) da[i] = 0.0f;
-  dense_bwd(W + T.lx12w, G + T.lx12w, G + T.lx12b, AR[6], &dOP, da, 16, 1);
-#pragma unroll 1
-  for (int r = 5; r >= 0; --r) {
-    float du[16], dt[16], dtp[16];
-    for (int i = 0; i < 16; ++i) { du[i] = UP[r][i] > 0.0f ? da[i] : 0.0f; dt[i] = 0.0f; }
-    dense_bwd(W + T.lxrw[2 * r + 1], G + T.lxrw[2 * r + 1], G + T.lxrb[2 * r + 1], TT[r], du, dt, 16, 16);
-    for (int i = 0; i < 16; ++i) dtp[i] = TP[r][i] > 0.0f ? dt[i] : 0.0f;
-    dense_bwd(W + T.lxrw[2 * r], G + T.lxrw[2 * r], G + T.lxrb[2 * r], AR[r], dtp, da, 16, 16);  // da += W^T dtp
-  }
-  float dAX[16];
-  for (int i = 0; i < 16; ++i) dAX[i] = AXP[i] > 0.0f ? da[i] : 0.0f;
-  for (int i = 0; i < 32; ++i) d3[i] = 0.0f;
-  dense_bwd(W + T.lxw, G + T.lxw, G + T.lxb, A3, dAX, d3, 32, 16);
-}
+struct TrainArgs {
+  const float* w;       // fp32 master weights (blob layout)
+  float* grad;          // fp32 gradient accumulator (blob layout)
+  const float* desc;    // n x 576, row-major
+  const float* aux;     // n x 5 (g, gamma, srp.xyz)
+  const float* label;   // n radiance labels
+  int n;
+  float inv_batch;      // loss weight: 1 / rows of the whole batch
+  float* loss;          // sum of (X - T)^2 / batch, added to
+  TrainWork wk;
+};
 
+int launch_train_trunk_fwd(const TrainArgs& a, cudaStream_t s);
+int launch_train_head(const TrainArgs& a, cudaStream_t s);
+int launch_train_tail(const TrainArgs& a, cudaStream_t s);
+int launch_train_trunk_bwd(const TrainArgs& a, cudaStream_t s);
 
 }  // namespace mr

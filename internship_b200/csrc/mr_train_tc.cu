@@ -139,20 +139,6 @@ __global__ void k_pack_head(const float* __restrict__ w, uint8_t* __restrict__ i
   *reinterpret_cast<__nv_bfloat16*>(img + base + canon_off(o, k, K)) = b;
 }
 
-struct HeadTrainArgs {
-  const uint8_t* img;   // kHeadImgBytes BF16 image (k_pack_head)
-  const float* w;       // fp32 master weights (biases, the tail)
-  float* grad;          // fp32 gradient (blob layout)
-  const float* h0;      // head input per row, n x 128
-  float* dh0;           // its gradient per row, n x 128
-  const float* aux;     // n x 5 (g, gamma, srp.xyz)
-  const float* label;   // n
-  int n;
-  float inv_batch;
-  float* loss;
-  int* err;             // set when a bounded wait gives up
-};
-
 // 16 consecutive values of a row -> BF16 at columns c0..c0+15 of a K-major tile.
 __device__ __forceinline__ void put16(uint8_t* tile, int row, int c0, int kp, const float* v) {
   uint32_t p[8];
@@ -165,13 +151,44 @@ __device__ __forceinline__ void put16(uint8_t* tile, int row, int c0, int kp, co
   *reinterpret_cast<uint4*>(tile + canon_off(row, c0 + 8, kp)) = make_uint4(p[4], p[5], p[6], p[7]);
 }
 
-// The head of the training step for tiles of 128 rows, one thread per row
-// (TMEM lane): LC0 -> LC1 -> LC2 forward as MMAs, the tail and the loss on
-// the CUDA cores (tail_fwd_bwd), then per layer one MMA round with the input
-// gradient (dY W, W read MN-major) and the weight gradient (dY^T X, both
-// tiles read MN-major) accumulated in tensor memory; the head-input gradient
-// goes to dh0 for the trunks' backward.
-__global__ void __launch_bounds__(128, 1) k_train_head_tc(const __grid_constant__ HeadTrainArgs a) {
+// Column sums over the rows of a warp: v[16] per lane (lane = row) into one
+// sum per lane, that of column col16(lane), by halving the columns and the
+// lanes together (16 shuffles, where a full reduction per column takes 80).
+__device__ __forceinline__ float col_sums16(float (&v)[16]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int h = 8; h >= 1; h >>= 1) {
+    const bool up = (lane & h) != 0;
+#pragma unroll
+    for (int i = 0; i < h; ++i) {
+      const float give = up ? v[i] : v[i + h];
+      const float keep = up ? v[i + h] : v[i];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, give, h);
+    }
+  }
+  return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 16);
+}
+// Adds the warp's column sums of v (a gradient chunk of 16 columns) to g[0..15].
+__device__ __forceinline__ void add_col_sums16(float* g, const float (&v)[16]) {
+  float x[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) x[i] = v[i];
+  const float s = col_sums16(x);
+  const int lane = threadIdx.x & 31;
+  if (lane < 16 && s != 0.0f) atomicAdd(g + lane, s);
+}
+
+// The head's tensor-core halves for tiles of 128 rows, one thread per row
+// (TMEM lane). BWD false: LC0 -> LC1 -> LC2 forward as MMAs, A3 (after ReLU)
+// to wk.a3 for the tail kernel (k_train_tail). BWD true: the forward of LC0
+// and LC1 again, then from wk.da3 per layer one MMA round with the input
+// gradient (dY W, W read MN-major) and the weight gradient (dY^T X, both tiles
+// read MN-major) accumulated in tensor memory; the head-input gradient goes to
+// wk.dh0 for the trunks' backward. One kernel with the tail in between, its
+// rows' products on the same 128 threads, took 2.44 ms for 65,536 rows.
+template <bool BWD>
+__global__ void __launch_bounds__(128, 1) k_train_head_tc(const __grid_constant__ TrainArgs a,
+                                                          const uint8_t* __restrict__ image, int* err) {
   extern __shared__ __align__(1024) uint8_t sm[];
   uint8_t* img = sm;
   uint8_t* tH0 = sm + kOffH0;
@@ -182,7 +199,7 @@ __global__ void __launch_bounds__(128, 1) k_train_head_tc(const __grid_constant_
   uint32_t* holder = reinterpret_cast<uint32_t*>(sm + kOffWk + kWkSlot + 8);
   const int t = threadIdx.x, warp = t >> 5;
   for (int i = t; i < kHeadImgBytes / 16; i += 128)
-    reinterpret_cast<uint4*>(img)[i] = __ldg(reinterpret_cast<const uint4*>(a.img) + i);
+    reinterpret_cast<uint4*>(img)[i] = __ldg(reinterpret_cast<const uint4*>(image) + i);
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(holder)),
                  "r"(512));
@@ -223,8 +240,8 @@ __global__ void __launch_bounds__(128, 1) k_train_head_tc(const __grid_constant_
     const int k = valid ? row : a.n - 1;
     // H0 -> BF16 tile
     {
-      const float4* src = reinterpret_cast<const float4*>(a.h0 + (size_t)k * 128);
-#pragma unroll 1
+      const float4* src = reinterpret_cast<const float4*>(a.wk.h0 + (size_t)k * 128);
+#pragma unroll 2
       for (int c = 0; c < 128; c += 16) {
         float v[16];
 #pragma unroll
@@ -241,7 +258,7 @@ __global__ void __launch_bounds__(128, 1) k_train_head_tc(const __grid_constant_
     });
     // A1 = ReLU(LC0 H0 + b)
     uint32_t m1[4] = {0u, 0u, 0u, 0u};
-#pragma unroll 1
+#pragma unroll
     for (int h = 0; h < 8; ++h) {
       float v[16];
       tmem_ld16(tm + lane + kColWork + 16 * h, v);
@@ -259,7 +276,7 @@ __global__ void __launch_bounds__(128, 1) k_train_head_tc(const __grid_constant_
     });
     // A2 = ReLU(LC1 A1 + b)
     uint32_t m2[2] = {0u, 0u};
-#pragma unroll 1
+#pragma unroll
     for (int h = 0; h < 4; ++h) {
       float v[16];
       tmem_ld16(tm + lane + kColWork + 16 * h, v);
@@ -271,94 +288,96 @@ __global__ void __launch_bounds__(128, 1) k_train_head_tc(const __grid_constant_
       }
       put16(tA2, t, 16 * h, 64, v);
     }
-    round([&] {
-      const uint32_t id = idesc_bf16_mn(128, 32, 0, 0);
-      for (int s = 0; s < 4; ++s) umma_bf16(tm + kColWork, kdesc(sA2, 64, s), kdesc(sW2, 64, s), id, s > 0);
-    });
-    // A3 = ReLU(LC2 A2 + b), the tail, the loss and the tail's backward
-    float A3[32], d3[32];
-    uint32_t m3 = 0u;
+    if constexpr (!BWD) {
+      round([&] {
+        const uint32_t id = idesc_bf16_mn(128, 32, 0, 0);
+        for (int s = 0; s < 4; ++s) umma_bf16(tm + kColWork, kdesc(sA2, 64, s), kdesc(sW2, 64, s), id, s > 0);
+      });
+      // A3 = ReLU(LC2 A2 + b)
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      float v[16];
-      tmem_ld16(tm + lane + kColWork + 16 * h, v);
+      for (int h = 0; h < 2; ++h) {
+        float v[16];
+        tmem_ld16(tm + lane + kColWork + 16 * h, v);
 #pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        const float x = v[i] + __ldg(W + T.lc2b + 16 * h + i);
-        if (x > 0.0f) m3 |= 1u << (16 * h + i);
-        A3[16 * h + i] = x > 0.0f ? x : 0.0f;
+        for (int i = 0; i < 16; ++i) v[i] = relu(v[i] + __ldg(W + T.lc2b + 16 * h + i));
+        if (valid) {
+          float4* o = reinterpret_cast<float4*>(a.wk.a3 + (size_t)row * 32 + 16 * h);
+#pragma unroll
+          for (int q = 0; q < 4; ++q) o[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+        }
       }
-    }
-    const float srp = a.aux[5 * (size_t)k + 2];
-    tail_fwd_bwd(W, G, T, A3, a.label[k], srp, valid, a.inv_batch, a.loss, d3);
-    // dA3 -> working tile; LC2's input and weight gradients
+    } else {
+      // dA3 -> working tile; LC2's input and weight gradients
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      float v[16];
+      for (int h = 0; h < 2; ++h) {
+        float v[16];
+        const float4* src = reinterpret_cast<const float4*>(a.wk.da3 + (size_t)k * 32 + 16 * h);
 #pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        v[i] = (m3 >> (16 * h + i)) & 1u ? d3[16 * h + i] : 0.0f;
-        gacc(G, T.lc2b + 16 * h + i, v[i]);
+        for (int q = 0; q < 4; ++q) {
+          const float4 x = valid ? src[q] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+          v[4 * q] = x.x; v[4 * q + 1] = x.y; v[4 * q + 2] = x.z; v[4 * q + 3] = x.w;
+        }
+        add_col_sums16(G + T.lc2b + 16 * h, v);
+        put16(tWk, t, 16 * h, 32, v);
       }
-      put16(tWk, t, 16 * h, 32, v);
-    }
-    const uint32_t acc0 = first ? 0u : 1u;
-    round([&] {
-      const uint32_t dx = idesc_bf16_mn(128, 64, 0, 1), dw = idesc_bf16_mn(128, 64, 1, 1);
-      for (int s = 0; s < 2; ++s) umma_bf16(tm + kColWork, kdesc(sWk, 32, s), mndesc(sW2, 64, s), dx, s > 0);
-      for (int s = 0; s < 8; ++s) umma_bf16(tm + kColG2, mndesc(sWk, 32, s), mndesc(sA2, 64, s), dw, s > 0 || acc0);
-    });
-    // dA2 = (dA3 LC2) * [A2 > 0]
-#pragma unroll 1
-    for (int h = 0; h < 4; ++h) {
-      float v[16];
-      tmem_ld16(tm + lane + kColWork + 16 * h, v);
+      const uint32_t acc0 = first ? 0u : 1u;
+      round([&] {
+        const uint32_t dx = idesc_bf16_mn(128, 64, 0, 1), dw = idesc_bf16_mn(128, 64, 1, 1);
+        for (int s = 0; s < 2; ++s) umma_bf16(tm + kColWork, kdesc(sWk, 32, s), mndesc(sW2, 64, s), dx, s > 0);
+        for (int s = 0; s < 8; ++s) umma_bf16(tm + kColG2, mndesc(sWk, 32, s), mndesc(sA2, 64, s), dw, s > 0 || acc0);
+      });
+      // dA2 = (dA3 LC2) * [A2 > 0]
 #pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        const int j = 16 * h + i;
-        v[i] = (m2[j >> 5] >> (j & 31)) & 1u ? v[i] : 0.0f;
-        gacc(G, T.lc1b + j, v[i]);
+      for (int h = 0; h < 4; ++h) {
+        float v[16];
+        tmem_ld16(tm + lane + kColWork + 16 * h, v);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          const int j = 16 * h + i;
+          v[i] = (m2[j >> 5] >> (j & 31)) & 1u ? v[i] : 0.0f;
+        }
+        add_col_sums16(G + T.lc1b + 16 * h, v);
+        put16(tWk, t, 16 * h, 64, v);
       }
-      put16(tWk, t, 16 * h, 64, v);
-    }
-    round([&] {
-      const uint32_t dx = idesc_bf16_mn(128, 128, 0, 1), dw = idesc_bf16_mn(128, 128, 1, 1);
-      for (int s = 0; s < 4; ++s) umma_bf16(tm + kColWork, kdesc(sWk, 64, s), mndesc(sW1, 128, s), dx, s > 0);
-      for (int s = 0; s < 8; ++s) umma_bf16(tm + kColG1, mndesc(sWk, 64, s), mndesc(sA1, 128, s), dw, s > 0 || acc0);
-    });
-    // dA1 = (dA2 LC1) * [A1 > 0]
-#pragma unroll 1
-    for (int h = 0; h < 8; ++h) {
-      float v[16];
-      tmem_ld16(tm + lane + kColWork + 16 * h, v);
+      round([&] {
+        const uint32_t dx = idesc_bf16_mn(128, 128, 0, 1), dw = idesc_bf16_mn(128, 128, 1, 1);
+        for (int s = 0; s < 4; ++s) umma_bf16(tm + kColWork, kdesc(sWk, 64, s), mndesc(sW1, 128, s), dx, s > 0);
+        for (int s = 0; s < 8; ++s) umma_bf16(tm + kColG1, mndesc(sWk, 64, s), mndesc(sA1, 128, s), dw, s > 0 || acc0);
+      });
+      // dA1 = (dA2 LC1) * [A1 > 0]
 #pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        const int j = 16 * h + i;
-        v[i] = (m1[j >> 5] >> (j & 31)) & 1u ? v[i] : 0.0f;
-        gacc(G, T.lc0b + j, v[i]);
+      for (int h = 0; h < 8; ++h) {
+        float v[16];
+        tmem_ld16(tm + lane + kColWork + 16 * h, v);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          const int j = 16 * h + i;
+          v[i] = (m1[j >> 5] >> (j & 31)) & 1u ? v[i] : 0.0f;
+        }
+        add_col_sums16(G + T.lc0b + 16 * h, v);
+        put16(tWk, t, 16 * h, 128, v);
       }
-      put16(tWk, t, 16 * h, 128, v);
-    }
-    round([&] {
-      const uint32_t dx = idesc_bf16_mn(128, 128, 0, 1), dw = idesc_bf16_mn(128, 128, 1, 1);
-      for (int s = 0; s < 8; ++s) umma_bf16(tm + kColWork, kdesc(sWk, 128, s), mndesc(sW0, 128, s), dx, s > 0);
-      for (int s = 0; s < 8; ++s) umma_bf16(tm + kColG0, mndesc(sWk, 128, s), mndesc(sH0, 128, s), dw, s > 0 || acc0);
-    });
-    // dH0 = dA1 LC0
-#pragma unroll 1
-    for (int h = 0; h < 8; ++h) {
-      float v[16];
-      tmem_ld16(tm + lane + kColWork + 16 * h, v);
-      if (valid) {
-        float4* o = reinterpret_cast<float4*>(a.dh0 + (size_t)row * 128 + 16 * h);
+      round([&] {
+        const uint32_t dx = idesc_bf16_mn(128, 128, 0, 1), dw = idesc_bf16_mn(128, 128, 1, 1);
+        for (int s = 0; s < 8; ++s) umma_bf16(tm + kColWork, kdesc(sWk, 128, s), mndesc(sW0, 128, s), dx, s > 0);
+        for (int s = 0; s < 8; ++s) umma_bf16(tm + kColG0, mndesc(sWk, 128, s), mndesc(sH0, 128, s), dw, s > 0 || acc0);
+      });
+      // dH0 = dA1 LC0
+#pragma unroll 2
+      for (int h = 0; h < 8; ++h) {
+        float v[16];
+        tmem_ld16(tm + lane + kColWork + 16 * h, v);
+        if (valid) {
+          float4* o = reinterpret_cast<float4*>(a.wk.dh0 + (size_t)row * 128 + 16 * h);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) o[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+          for (int q = 0; q < 4; ++q) o[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+        }
       }
     }
     first = false;
   }
   // the CTA's weight gradients: TMEM lane = output unit
-  if (!first && ok) {
+  if (BWD && !first && ok) {
 #pragma unroll 1
     for (int h = 0; h < 8; ++h) {
       float v[16];
@@ -385,7 +404,7 @@ __global__ void __launch_bounds__(128, 1) k_train_head_tc(const __grid_constant_
       }
     }
   }
-  if (!ok && t == 0) atomicExch(a.err, 1);
+  if (!ok && t == 0) atomicExch(err, 1);
   tc_fence_before();
   __syncthreads();
   if (warp == 0) {
@@ -394,32 +413,28 @@ __global__ void __launch_bounds__(128, 1) k_train_head_tc(const __grid_constant_
   }
 }
 
-// The BF16 training step's three launches after the weight image: the trunks'
-// forward (head input per row), the tensor-core head, the trunks' backward.
-int launch_head_tc(const float* w, float* grad, uint8_t* img, const float* h0, float* dh0, const float* aux,
-                   const float* label, int n, float inv_batch, float* loss, int* err, cudaStream_t s) {
+// The BF16 weight image of the head.
+int launch_head_pack(const float* w, uint8_t* img, cudaStream_t s) {
+  k_pack_head<<<(kHeadImgBytes / 2 + 255) / 256, 256, 0, s>>>(w, img);
+  MR_CUDA(cudaGetLastError());
+  return MR_OK;
+}
+
+// The head of the BF16 step: wk.h0 -> loss, gradients, wk.dh0.
+int launch_head_tc(const TrainArgs& a, const uint8_t* img, int* err, cudaStream_t s) {
   static DeviceCache attr;
   int rc = attr.once([] {
-    MR_CUDA(cudaFuncSetAttribute(k_train_head_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, kHeadTrainSmem));
+    MR_CUDA(cudaFuncSetAttribute(k_train_head_tc<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kHeadTrainSmem));
+    MR_CUDA(cudaFuncSetAttribute(k_train_head_tc<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kHeadTrainSmem));
     return (int)MR_OK;
   });
   if (rc) return rc;
-  k_pack_head<<<(kHeadImgBytes / 2 + 255) / 256, 256, 0, s>>>(w, img);
+  const int grid = std::min((a.n + 127) / 128, sm_count());
+  k_train_head_tc<false><<<grid, 128, kHeadTrainSmem, s>>>(a, img, err);
   MR_CUDA(cudaGetLastError());
-  HeadTrainArgs a;
-  a.img = img;
-  a.w = w;
-  a.grad = grad;
-  a.h0 = h0;
-  a.dh0 = dh0;
-  a.aux = aux;
-  a.label = label;
-  a.n = n;
-  a.inv_batch = inv_batch;
-  a.loss = loss;
-  a.err = err;
-  const int tiles = (n + 127) / 128;
-  k_train_head_tc<<<std::min(tiles, sm_count()), 128, kHeadTrainSmem, s>>>(a);
+  rc = launch_train_tail(a, s);
+  if (rc) return rc;
+  k_train_head_tc<true><<<grid, 128, kHeadTrainSmem, s>>>(a, img, err);
   MR_CUDA(cudaGetLastError());
   return MR_OK;
 }
