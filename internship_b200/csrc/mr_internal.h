@@ -47,6 +47,7 @@ struct Volume {
   float* mips = nullptr;     // kMipTotal
   float* var = nullptr;      // kMipTotal
   float* tr = nullptr;       // kTrTotal
+  float2* tr_pairs = nullptr;  // mips 1..8 as padded z pairs, read by the TR build (20 MB)
   float* lut = nullptr;      // 512 x 512
   float* d_max = nullptr;    // device majorant (one float)
   unsigned long long* d_counters = nullptr;

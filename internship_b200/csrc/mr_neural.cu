@@ -503,9 +503,35 @@ __device__ __forceinline__ void point_table_seg(const Tables& t, const float* __
   }
 }
 
-template <int MIP, bool SPHERE, int SAMP, int I0, int I1, class Sink>
+// ray_box_offset with its fused steps spelled out: which of an axis' two
+// products is rounded first is otherwise the compiler's choice, differs with
+// the code around it, and moves a shadow sample outside the box by an ulp.
+// Bit k of AX: on axis k the position's product is the rounded one, else the
+// face's. kBoxSingle / box_batch keep the values each kernel has had.
+constexpr int kBoxSingle = 0;
+constexpr int box_batch(int samp) { return samp == kSampGather ? 7 : 6; }
+template <int AX>
+__device__ __forceinline__ float box_entry(F3 p, F3 dir) {
+  const F3 d = inv3(dir);
+  auto axis = [](bool pos, float p, float d, float& lo, float& hi) {
+    const float r = pos ? __fmul_rn(-p, d) : __fmul_rn(0.4999f, d);
+    const float a = pos ? __fmaf_rn(0.4999f, d, r) : __fmaf_rn(-p, d, r);
+    const float b = pos ? __fmaf_rn(-0.4999f, d, r) : __fmaf_rn(-p, d, -r);
+    lo = fminf(a, b);
+    hi = fmaxf(a, b);
+  };
+  F3 lo, hi;
+  axis((AX & 1) != 0, p.x, d.x, lo.x, hi.x);
+  axis((AX & 2) != 0, p.y, d.y, lo.y, hi.y);
+  axis((AX & 4) != 0, p.z, d.z, lo.z, hi.z);
+  const float tmi = fmaxf(lo.x, fmaxf(lo.y, lo.z)), tma = fminf(hi.x, fminf(hi.y, hi.z));
+  return tma >= tmi ? fmaxf(tmi, 0.0f) : -1.0f;
+}
+
+// Points [b, e) of the segment (whole chunks of 4).
+template <int MIP, bool SPHERE, int SAMP, int I0, int I1, int AX, class Sink>
 __device__ __forceinline__ void gather_seg(const Tables& t, const float* __restrict__ stencil, const PixelGather& q,
-                                           float off, const float* h0s, Sink& sink) {
+                                           float off, const float* h0s, Sink& sink, int b, int e) {
   constexpr int R = 256 >> MIP;
   constexpr int TL = MIP > 0 ? MIP - 1 : 0;
   constexpr int RT = 128 >> TL;
@@ -516,7 +542,7 @@ __device__ __forceinline__ void gather_seg(const Tables& t, const float* __restr
   float vrow = h0s ? h0s[192 + I0] : atanf(0.5f * radius / off) / kAng;
   static_assert(I0 % 4 == 0 && I1 % 4 == 0, "segments are whole 4-feature chunks");
 #pragma unroll 1
-  for (int i0 = I0; i0 < I1; i0 += 4)
+  for (int i0 = b; i0 < e; i0 += 4)
 #pragma unroll
   for (int u = 0; u < 4; ++u) {
     const int i = i0 + u;
@@ -556,7 +582,7 @@ __device__ __forceinline__ void gather_seg(const Tables& t, const float* __restr
     float xs = 1.0f;
     bool fetch = true;
     if (p.x < -0.5f || p.y < -0.5f || p.z < -0.5f || p.x > 0.5f || p.y > 0.5f || p.z > 0.5f) {
-      const float o2 = ray_box_offset(p, q.LX);  // ShadowTerm_TRTex (core/renderResources.cu:121-139)
+      const float o2 = box_entry<AX>(p, q.LX);  // ShadowTerm_TRTex (core/renderResources.cu:121-139)
       fetch = o2 >= 0;
       pt = p + q.LX * o2;
     }
@@ -569,7 +595,7 @@ __device__ __forceinline__ void gather_seg(const Tables& t, const float* __restr
 }
 
 // The per-point table (see point_table_seg), with the segment offsets of
-// gather_fast.
+// gather_points.
 template <int SAMP>
 __device__ __forceinline__ void point_table(const Tables& t, const float* __restrict__ stencil, float* tab) {
   const float ms = 0.6f;
@@ -593,11 +619,7 @@ __global__ void k_sphere_h0(Tables t, const float* __restrict__ stencil, float* 
   point_table<SAMP>(t, stencil, h0s);
 }
 
-// h0s: the per-point table (k_sphere_h0), or null to compute its entries per
-// point.
-template <int SAMP, class Sink>
-__device__ __forceinline__ void gather_fast(const Tables& t, const float* __restrict__ stencil, F3 pos, F3 L,
-                                            const Frame& f, float alpha, float g, const float* h0s, Sink sink) {
+__device__ __forceinline__ PixelGather pixel_gather(F3 pos, F3 L, const Frame& f, float alpha, float g) {
   PixelGather q;
   q.pos = pos; q.L = L; q.X = f.X; q.Y = f.Y; q.Z = f.Z; q.LX = f.LX;
   q.lx = dot(f.LX, f.X); q.ly = dot(f.LX, f.Y); q.lz = dot(f.LX, f.Z);
@@ -605,39 +627,95 @@ __device__ __forceinline__ void gather_fast(const Tables& t, const float* __rest
   q.cLXL = dot(f.LX, L);
   q.alpha = alpha;
   q.hg0 = __logf(hg_phase(dot(f.X, L), g) + 1.0f);
-  const float ms = 0.6f;
-  gather_seg<0, true, SAMP, 0, 8>(t, stencil, q, 1.0f / 256.0f * lerpf(ms, 1.0f, 1.0f), h0s, sink);
-  gather_seg<1, true, SAMP, 8, 16>(t, stencil, q, 2.5f / 256.0f * lerpf(ms, 1.0f, 0.8f), h0s, sink);
-  gather_seg<2, true, SAMP, 16, 32>(t, stencil, q, 5.5f / 256.0f * lerpf(ms, 1.0f, 0.6f), h0s, sink);
-  gather_seg<3, true, SAMP, 32, 48>(t, stencil, q, 11.5f / 256.0f * lerpf(ms, 1.0f, 0.4f), h0s, sink);
-  gather_seg<4, true, SAMP, 48, 64>(t, stencil, q, 23.5f / 256.0f * lerpf(ms, 1.0f, 0.2f), h0s, sink);
-  gather_seg<5, true, SAMP, 64, 96>(t, stencil, q, 47.5f / 256.0f * ms, h0s, sink);
-  gather_seg<6, true, SAMP, 96, 128>(t, stencil, q, 95.5f / 256.0f * ms, h0s, sink);
-  gather_seg<7, true, SAMP, 128, 160>(t, stencil, q, 191.5f / 256.0f * ms, h0s, sink);
-  gather_seg<0, false, SAMP, 160, 168>(t, stencil, q, 1.0f, h0s, sink);
-  gather_seg<1, false, SAMP, 168, 176>(t, stencil, q, 1.0f, h0s, sink);
-  gather_seg<2, false, SAMP, 176, 184>(t, stencil, q, 1.0f, h0s, sink);
-  gather_seg<3, false, SAMP, 184, 192>(t, stencil, q, 1.0f, h0s, sink);
+  return q;
 }
 
-// Gather only, for explicit points and frames (test / training entry).
-__global__ void k_gather(Tables t, const float* __restrict__ stencil, const float* __restrict__ pos,
+// Points [b, e) of a record (multiples of 8: every segment is a whole number
+// of such eighths). h0s: the per-point table (k_sphere_h0), or null to compute
+// its entries per point.
+constexpr int kPoints = 192;
+template <int SAMP, int AX, class Sink>
+__device__ __forceinline__ void gather_points(const Tables& t, const float* __restrict__ stencil, const PixelGather& q,
+                                              const float* h0s, int b, int e, Sink sink) {
+  const float ms = 0.6f;
+#define MR_SEG(MIP, SPHERE, I0, I1, OFF) \
+  if (b < I1 && e > I0) gather_seg<MIP, SPHERE, SAMP, I0, I1, AX>(t, stencil, q, OFF, h0s, sink, max(b, I0), min(e, I1));
+  MR_SEG(0, true, 0, 8, 1.0f / 256.0f * lerpf(ms, 1.0f, 1.0f))
+  MR_SEG(1, true, 8, 16, 2.5f / 256.0f * lerpf(ms, 1.0f, 0.8f))
+  MR_SEG(2, true, 16, 32, 5.5f / 256.0f * lerpf(ms, 1.0f, 0.6f))
+  MR_SEG(3, true, 32, 48, 11.5f / 256.0f * lerpf(ms, 1.0f, 0.4f))
+  MR_SEG(4, true, 48, 64, 23.5f / 256.0f * lerpf(ms, 1.0f, 0.2f))
+  MR_SEG(5, true, 64, 96, 47.5f / 256.0f * ms)
+  MR_SEG(6, true, 96, 128, 95.5f / 256.0f * ms)
+  MR_SEG(7, true, 128, 160, 191.5f / 256.0f * ms)
+  MR_SEG(0, false, 160, 168, 1.0f)
+  MR_SEG(1, false, 168, 176, 1.0f)
+  MR_SEG(2, false, 176, 184, 1.0f)
+  MR_SEG(3, false, 184, 192, 1.0f)
+#undef MR_SEG
+}
+
+// How many groups of points a record's gather is split into, each group a
+// work item of its own, `threads` items at a time: fewer points per item fill
+// the GPU when there are few records and shorten a nearly empty last wave.
+// Group by group over all records, neighbouring warps read the same mip
+// levels: the texture filter gains from that, the exact sampler's footprints
+// lose a little (their cost per point, `pen`, measured on 322 k records).
+// Gather at 1, 3 and 6 groups: exact, 322 k records 751 / 792 / 810 us, 144 k
+// (1.3 waves) 446 / 343 / 345; texture filter, 322 k records 596 / 550 / 570,
+// 144 k 341 / 270 / 269. 2.2 k records: 138 us at one group, 19 at 24.
+__host__ __device__ __forceinline__ int gather_groups(unsigned n, unsigned threads, bool tex) {
+  int best = 1;
+  float least = 3.0e38f;
+  for (int i = 0; i < 5; ++i) {
+    const int g = i == 0 ? 1 : 3 << (i - 1);  // 1, 3, 6, 12, 24
+    const float pen = tex ? (i == 0 ? 1.08f : i == 1 ? 1.0f : i == 2 ? 1.03f : i == 3 ? 1.06f : 1.15f)
+                          : (i == 0 ? 1.0f : i == 1 ? 1.07f : i == 2 ? 1.08f : i == 3 ? 1.1f : 1.2f);
+    const float waves = ceilf((float)n * (float)g / (float)threads);
+    const float cost = pen * waves / (float)g;
+    if (cost < least) {
+      least = cost;
+      best = g;
+    }
+  }
+  return best;
+}
+
+// Gather only, for explicit points and frames (test / training entry): one
+// row of 576 features per point.
+__global__ void __launch_bounds__(128) k_gather(Tables t, const float* __restrict__ stencil, const float* __restrict__ pos,
                          const float* __restrict__ frame, int n, F3 L, float alpha, float g, F3 srp,
-                         float* __restrict__ desc, float* __restrict__ aux) {
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
+                         float* __restrict__ desc, float* __restrict__ aux, int groups, bool wide) {
+  const int per = kPoints / groups, tiles = (n + 127) / 128;
+  const int grp = blockIdx.x / tiles, k = (blockIdx.x - grp * tiles) * 128 + threadIdx.x;
   if (k >= n) return;
-  Frame f = load_frame(frame + 12 * (size_t)k);
+  const Frame f = load_frame(frame + 12 * (size_t)k);
   float* d = desc + 576 * (size_t)k;
-  auto sink = [&](int i, int, float xv, float xs, float xh) {
-    d[i] = xv;
-    d[192 + i] = xs;
-    d[384 + i] = xh;
+  float4 bv, bs, bh;
+  auto sink = [&](int i, int u, float xv, float xs, float xh) {
+    if (wide) {
+      (&bv.x)[u] = xv;
+      (&bs.x)[u] = xs;
+      (&bh.x)[u] = xh;
+      if (u == 3) {
+        *reinterpret_cast<float4*>(d + i - 3) = bv;
+        *reinterpret_cast<float4*>(d + 192 + i - 3) = bs;
+        *reinterpret_cast<float4*>(d + 384 + i - 3) = bh;
+      }
+    } else {
+      d[i] = xv;
+      d[192 + i] = xs;
+      d[384 + i] = xh;
+    }
   };
-  gather_fast<kSampLoad>(t, stencil, f3(pos[3 * k], pos[3 * k + 1], pos[3 * k + 2]), L, f, alpha, g, nullptr, sink);
-  float* ax = aux + 5 * (size_t)k;
-  ax[0] = g;
-  ax[1] = acosf(dot(f.X, f.LX));
-  ax[2] = srp.x; ax[3] = srp.y; ax[4] = srp.z;
+  const PixelGather q = pixel_gather(f3(pos[3 * (size_t)k], pos[3 * (size_t)k + 1], pos[3 * (size_t)k + 2]), L, f, alpha, g);
+  gather_points<kSampLoad, kBoxSingle>(t, stencil, q, nullptr, grp * per, grp * per + per, sink);
+  if (grp == 0) {
+    float* ax = aux + 5 * (size_t)k;
+    ax[0] = g;
+    ax[1] = acosf(dot(f.X, f.LX));
+    ax[2] = srp.x; ax[3] = srp.y; ax[4] = srp.z;
+  }
 }
 
 // Gather for the compacted records in chunk-of-4 feature-major order:
@@ -651,9 +729,15 @@ __global__ void __launch_bounds__(128, SAMP == kSampLoad ? 1 : 6)
     k_gather_fm(Tables t, const float* __restrict__ stencil, const float* __restrict__ h0s, Records rec, int cap, F3 L,
                 float alpha, float g, F3 srp, float* __restrict__ desc, float* __restrict__ aux) {
   const unsigned n = min(*rec.count, (unsigned)cap);
-  // a resident grid strides over the records (the record count is known on
-  // the device only)
-  for (unsigned k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+  if (n == 0) return;
+  // a resident grid strides over the (group of points, tile of records) items,
+  // group by group (the record count is known on the device only)
+  const int groups = gather_groups(n, gridDim.x * blockDim.x, SAMP == kSampTex), per = kPoints / groups;
+  const unsigned tiles = (n + blockDim.x - 1) / blockDim.x;
+  for (unsigned w = blockIdx.x; w < tiles * groups; w += gridDim.x) {
+    const int grp = w / tiles;
+    const unsigned k = (w - grp * tiles) * blockDim.x + threadIdx.x;
+    if (k >= n) continue;
     F3 pos = f3(rec.pos[3 * (size_t)k], rec.pos[3 * (size_t)k + 1], rec.pos[3 * (size_t)k + 2]);
     Frame f = load_frame(rec.frame + 12 * (size_t)k);
     // chunk-of-4 feature-major: features 4j..4j+3 of record k are the float4
@@ -671,12 +755,14 @@ __global__ void __launch_bounds__(128, SAMP == kSampLoad ? 1 : 6)
         d[(96 + (i >> 2)) * c] = bh;
       }
     };
-    gather_fast<SAMP>(t, stencil, pos, L, f, alpha, g, h0s, sink);
-    aux[k] = g;
-    aux[c + k] = acosf(dot(f.X, f.LX));
-    aux[2 * c + k] = srp.x;
-    aux[3 * c + k] = srp.y;
-    aux[4 * c + k] = srp.z;
+    gather_points<SAMP, kBoxSingle>(t, stencil, pixel_gather(pos, L, f, alpha, g), h0s, grp * per, grp * per + per, sink);
+    if (grp == 0) {
+      aux[k] = g;
+      aux[c + k] = acosf(dot(f.X, f.LX));
+      aux[2 * c + k] = srp.x;
+      aux[3 * c + k] = srp.y;
+      aux[4 * c + k] = srp.z;
+    }
   }
 }
 
@@ -888,7 +974,7 @@ static int neural_passes(Volume* v, const Network* net, const mr_render_params* 
         128, 0);
     return std::max(1, n);
   });
-  const unsigned ggrid = (unsigned)std::min<size_t>((npx + 127) / 128, (size_t)per_sm * sm_count());
+  const unsigned ggrid = (unsigned)std::min<size_t>((npx + 127) / 128 * 24, (size_t)per_sm * sm_count());
   if (samp == kSampTex)
     k_gather_fm<kSampTex><<<ggrid, 128, 0, s>>>(tabs, net->stencil, h0s, rec, (int)npx, L, p->alpha, p->g,
                                                srp_of(sr), desc, aux);
@@ -938,9 +1024,11 @@ extern "C" int mr_gather_descriptors(const mr_volume* h, const mr_network* nh, c
   if (!v->mips_valid || !v->tr_valid || !v->lut_valid)
     return set_error(MR_ERR_STATE, "gather needs mr_volume_update, _update_tr and _update_hglut first");
   F3 sr = to_f3(scatter_rate) / 1.001f;
-  k_gather<<<(n + 127) / 128, 128, 0, (cudaStream_t)stream>>>(Tables{v->mips, v->tr, v->lut, {}, {}, 0}, nh->n.stencil,
-                                                            dev_pos, dev_frame, n, v->tr_light, alpha, g,
-                                                            srp_of(sr), dev_desc, dev_aux);
+  const int groups = gather_groups((unsigned)n, (unsigned)sm_count() * 640u, false);
+  const long long blocks = (long long)((n + 127) / 128) * groups;
+  k_gather<<<(unsigned)blocks, 128, 0, (cudaStream_t)stream>>>(
+      Tables{v->mips, v->tr, v->lut, {}, {}, 0}, nh->n.stencil, dev_pos, dev_frame, n, v->tr_light, alpha, g,
+      srp_of(sr), dev_desc, dev_aux, groups, (reinterpret_cast<uintptr_t>(dev_desc) & 15) == 0);
   MR_CUDA(cudaGetLastError());
   return MR_OK;
 }
@@ -1168,13 +1256,21 @@ __global__ void k_sphere_h0_batch(const BatchJob* __restrict__ jobs, const float
   point_table<SAMP>(jobs[blockIdx.x].tabs, stencil, h0 + (size_t)blockIdx.x * kPtTable);
 }
 
+// Groups of points per record in the batched gather (gather_groups' largest
+// gains need no more; a launch covers the wave's pixels, of which the records
+// are a part, so more groups would mostly add empty blocks). Batch of 8 views,
+// texture filter: 1097 us at one group, 1033 at three.
+constexpr int kBatchGroups = 3;
 template <int SAMP>
 __global__ void __launch_bounds__(256, 3) k_gather_batch(const BatchJob* __restrict__ jobs,
                                                       const float* __restrict__ stencil,
                                                       const float* __restrict__ h0, Records rec, int cap,
                                                       float* __restrict__ desc, float* __restrict__ aux) {
-  const unsigned k = blockIdx.x * blockDim.x + threadIdx.x;
   const unsigned n = min(*rec.count, (unsigned)cap);
+  const unsigned tiles = (n + blockDim.x - 1) / blockDim.x;
+  if (blockIdx.x >= tiles * kBatchGroups) return;
+  const unsigned grp = blockIdx.x / tiles;
+  const unsigned k = (blockIdx.x - grp * tiles) * blockDim.x + threadIdx.x;
   const bool valid = k < n;
   const int job = valid ? rec.job[k] : -1;
   // One job at a time per warp. The texture handles of a fetch must be the
@@ -1203,12 +1299,16 @@ __global__ void __launch_bounds__(256, 3) k_gather_batch(const BatchJob* __restr
           d[(96 + (i >> 2)) * c] = bh;
         }
       };
-      gather_fast<SAMP>(j.tabs, stencil, pos, j.sc.L, f, j.sc.alpha, j.sc.g, h0 + (size_t)jj * kPtTable, sink);
-      aux[k] = j.sc.g;
-      aux[c + k] = acosf(dot(f.X, f.LX));
-      aux[2 * c + k] = j.srp.x;
-      aux[3 * c + k] = j.srp.y;
-      aux[4 * c + k] = j.srp.z;
+      gather_points<SAMP, box_batch(SAMP)>(j.tabs, stencil, pixel_gather(pos, j.sc.L, f, j.sc.alpha, j.sc.g),
+                                           h0 + (size_t)jj * kPtTable, grp * (kPoints / kBatchGroups), (grp + 1) * (kPoints / kBatchGroups),
+                                           sink);
+      if (grp == 0) {
+        aux[k] = j.sc.g;
+        aux[c + k] = acosf(dot(f.X, f.LX));
+        aux[2 * c + k] = j.srp.x;
+        aux[3 * c + k] = j.srp.y;
+        aux[4 * c + k] = j.srp.z;
+      }
     }
     todo &= ~__ballot_sync(0xffffffffu, mine);
   }
@@ -1317,7 +1417,7 @@ static int batch_launches(Batch& b, const Network* net, cudaStream_t s) {
     const unsigned tgrid = (unsigned)((w1 - w0 + b.trace_block - 1) / b.trace_block);
     k_trace_batch<<<tgrid, b.trace_block, kRingWords * sizeof(uint32_t) * b.trace_block, s>>>(b.d_jobs, nj, w0, w1, b.d_out, rec, b.counters);
     MR_CUDA(cudaGetLastError());
-    const unsigned ggrid = (unsigned)((w1 - w0 + b.gather_block - 1) / b.gather_block);
+    const unsigned ggrid = kBatchGroups * (unsigned)((w1 - w0 + b.gather_block - 1) / b.gather_block);
     if (hw)
       k_gather_batch<kSampTex><<<ggrid, b.gather_block, 0, s>>>(b.d_jobs, net->stencil, b.d_h0, rec, (int)cap, desc,
                                                                 aux);

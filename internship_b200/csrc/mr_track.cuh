@@ -23,26 +23,6 @@ __device__ __forceinline__ float fetch_density(const Medium& m, F3 pos, TrackSta
   return m.tex ? tri_border_tex(m.tex, m.res, pos + 0.5f) : tri_border(m.density, m.res, pos + 0.5f);
 }
 
-// x / y for a fixed y, correctly rounded like the division itself: two
-// residual corrections with r = RN(1 / y) (Markstein, IBM J. Res. Dev. 34,
-// 1990: a faithful quotient corrected once with a correctly rounded
-// reciprocal is the correctly rounded quotient). Needs y, x / y and their
-// residuals in the normal range, so y far from it (fast == false) takes the
-// division (1.5e8 quotients over 40 divisors equal the division's). A tiny or
-// infinite x only gives quotients that compare and accumulate like the
-// division's. In run_paths: sphere scene 2.90 ms with the division, 2.57 ms.
-struct DivBy {
-  float y, r;
-  bool fast;
-  __device__ __forceinline__ explicit DivBy(float y_) : y(y_), r(1.0f / y_), fast(y_ > 1e-18f && y_ < 1e18f) {}
-  __device__ __forceinline__ float operator()(float x) const {
-    if (!fast) return x / y;
-    float q = __fmul_rn(x, r);
-    q = __fmaf_rn(__fmaf_rn(-q, y, x), r, q);
-    return __fmaf_rn(__fmaf_rn(-q, y, x), r, q);
-  }
-};
-
 // DeterminateNextVertex (core/render.cuh:138-172). R is Rng or RngRing;
 // prime() keeps the lanes' Philox calls at the same iterations.
 template <class R>
