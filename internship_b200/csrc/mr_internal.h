@@ -105,6 +105,12 @@ struct Volume {
   cudaStream_t copy_stream = nullptr;
   cudaEvent_t rendered[2] = {}, copied[2] = {};
   long long frame_seq = 0;  // frames issued so far; frame t uses frame[t % 2]
+  // Device frame of mr_render_host, kept for the next call: a call takes it
+  // (or allocates one) and puts it back, so that calls from several threads
+  // never share it.
+  std::mutex host_frame_mu;
+  float* host_frame = nullptr;
+  size_t host_frame_bytes = 0;
   // Side stream of a neural render (the per-point table beside the trace),
   // forked from and joined back to the caller's stream by events.
   cudaStream_t side_stream = nullptr;
@@ -180,6 +186,15 @@ void clear_error();
   } while (0)
 
 inline F3 to_f3(const mr_float3& a) { return F3{a.x, a.y, a.z}; }
+
+// Stream-ordered temporary memory from a pool of the library's own on the
+// current device. Up to kPoolKeep bytes stay with the pool between calls (the
+// runtime's default pool returns everything to the device at each
+// synchronisation and maps it again on the next call); network_pool_trim gives
+// unused memory back.
+constexpr size_t kPoolKeep = (size_t)256 << 20;
+cudaError_t pool_alloc(void** p, size_t bytes, cudaStream_t s);
+void network_pool_trim();
 
 // Grows v->scratch to at least `bytes` (stream-ordered free of the old block).
 int ensure_scratch(Volume* v, size_t bytes, cudaStream_t s);

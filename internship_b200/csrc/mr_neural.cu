@@ -1108,27 +1108,34 @@ extern "C" int mr_radiance_predict(const mr_network* nh, int32_t precision, cons
   if (n == 0) return MR_OK;
   if (reinterpret_cast<uintptr_t>(dev_desc) & 15)
     return set_error(MR_ERR_ARG, "mr_radiance_predict: dev_desc must be 16-byte aligned");
-  if (precision == MR_PREC_BF16 || precision == MR_PREC_FP8) {
-    // rows may carry distinct albedo channels: spill space for further heads
-    cudaStream_t s = (cudaStream_t)stream;
-    float* spill = nullptr;
-    cudaError_t e = cudaMallocAsync(&spill, (size_t)n * 120 * sizeof(float), s);
-    if (e != cudaSuccess) return set_error(MR_ERR_NOMEM, "spill allocation failed: %s", cudaGetErrorString(e));
-    int rc = launch_mlp_tc(&nh->n, dev_desc, dev_aux, 576, 4, 5, 1, n, dev_out, nullptr, nullptr, nullptr,
-                           f3(1, 1, 1), f3(1, 1, 1), spill, precision == MR_PREC_FP8, s);
-    MR_CUDA(cudaFreeAsync(spill, s));
-    return rc;
-  }
-  if (precision != MR_PREC_FP32) return set_error(MR_ERR_ARG, "unknown precision %d", precision);
-  // the caller's descriptors stay untouched: trunk outputs (152) and the
-  // head's LC2 outputs (96) of a row go to a temporary
   cudaStream_t s = (cudaStream_t)stream;
-  float* tout = nullptr;
-  cudaError_t e = cudaMallocAsync(&tout, (size_t)n * 248 * sizeof(float), s);
-  if (e != cudaSuccess) return set_error(MR_ERR_NOMEM, "trunk buffer: %s", cudaGetErrorString(e));
-  int rc = launch_mlp_simt(&nh->n, dev_desc, dev_aux, 576, 4, 5, 1, n, nullptr, dev_out, nullptr, nullptr,
-                           f3(1, 1, 1), f3(1, 1, 1), s, nullptr, nullptr, tout, 248, 4, tout + 152, 248, 4);
-  MR_CUDA(cudaFreeAsync(tout, s));
+  const bool tc = precision == MR_PREC_BF16 || precision == MR_PREC_FP8;
+  if (!tc && precision != MR_PREC_FP32) return set_error(MR_ERR_ARG, "unknown precision %d", precision);
+  // The caller's descriptors stay untouched. fp32: trunk outputs (152) and the
+  // head's LC2 outputs (96) of a row go to a temporary; tensor cores: spill
+  // space for further heads, as rows may carry distinct albedo channels. Long
+  // tables run in pieces whose temporary the pool keeps (265 k rows, 251 MiB
+  // in fp32): 262 k rows took 1.20 ms in one piece, 1.26 in three, 1.31 in
+  // five (one wave of the trunk each, its outputs in L2).
+  const size_t per_row = tc ? 120 : 248;
+  const int piece = std::min(n, sm_count() * (tc ? 2048 : 14 * 128));
+  float* tmp = nullptr;
+  cudaError_t e = pool_alloc((void**)&tmp, (size_t)piece * per_row * sizeof(float), s);
+  if (e != cudaSuccess) return set_error(MR_ERR_NOMEM, "network temporary: %s", cudaGetErrorString(e));
+  int rc = MR_OK;
+  for (int r0 = 0; r0 < n && rc == MR_OK; r0 += piece) {
+    const int m = std::min(piece, n - r0);
+    const float* d = dev_desc + (size_t)r0 * 576;
+    const float* a = dev_aux + (size_t)r0 * 5;
+    float* o = dev_out + (size_t)r0 * 3;
+    if (tc)
+      rc = launch_mlp_tc(&nh->n, d, a, 576, 4, 5, 1, m, o, nullptr, nullptr, nullptr, f3(1, 1, 1), f3(1, 1, 1), tmp,
+                         precision == MR_PREC_FP8, s);
+    else
+      rc = launch_mlp_simt(&nh->n, d, a, 576, 4, 5, 1, m, nullptr, o, nullptr, nullptr, f3(1, 1, 1), f3(1, 1, 1), s,
+                           nullptr, nullptr, tmp, 248, 4, tmp + 152, 248, 4);
+  }
+  MR_CUDA(cudaFreeAsync(tmp, s));
   return rc;
 }
 

@@ -550,6 +550,37 @@ void destroy_textures(Volume* v) {
   if (v->lut_arr) cudaFreeArray(v->lut_arr);
 }
 
+// One pool per device, created on first use.
+static std::mutex g_pool_mu;
+static cudaMemPool_t g_pool[kMaxDevices];
+static cudaMemPool_t device_pool(bool create) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return nullptr;
+  std::lock_guard<std::mutex> lock(g_pool_mu);
+  if (!g_pool[dev] && create) {
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    cudaMemPool_t pool = nullptr;
+    if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
+    unsigned long long keep = kPoolKeep;
+    cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    g_pool[dev] = pool;
+  }
+  return g_pool[dev];
+}
+cudaError_t pool_alloc(void** p, size_t bytes, cudaStream_t s) {
+  cudaMemPool_t pool = device_pool(true);
+  return pool ? cudaMallocFromPoolAsync(p, bytes, pool, s) : cudaMallocAsync(p, bytes, s);
+}
+void network_pool_trim() {
+  if (cudaMemPool_t pool = device_pool(false)) cudaMemPoolTrimTo(pool, 0);
+}
+
 int ensure_scratch(Volume* v, size_t bytes, cudaStream_t s) {
   if (v->scratch_bytes >= bytes) return MR_OK;
   if (v->scratch) MR_CUDA(cudaFreeAsync(v->scratch, s));
@@ -621,6 +652,7 @@ int mr_volume_destroy(mr_volume* h) {
   }
   for (int i = 0; i < 2; ++i)
     if (v->frame[i]) cudaFree(v->frame[i]);
+  if (v->host_frame) cudaFree(v->host_frame);
   if (v->side_stream) {
     cudaStreamSynchronize(v->side_stream);
     cudaEventDestroy(v->side_fork);
