@@ -44,6 +44,7 @@ struct Volume {
   int res = 0;
   int device = 0;
   float* density = nullptr;  // res^3
+  float* tables = nullptr;   // one allocation: the tables below, the majorant and the counters
   float* mips = nullptr;     // kMipTotal
   float* var = nullptr;      // kMipTotal
   float* tr = nullptr;       // kTrTotal
