@@ -22,8 +22,7 @@ struct DTArgs {
   unsigned long long* counters;     // [0] fetches, [1] paths, [2] loop caps
   float* store;                     // W*H*3 (nullable): one path per pixel, its radiance written, no sums
   int checker, flip;                // store only: half the pixels, those with (row + flip) & 1 == col & 1
-  float* sum32;                     // W*H*3 (nullable)
-  double* sum64;                    // W*H*3 (nullable)
+  double* sum64;                    // W*H*3 (unless store)
   double* sumsq64;                  // W*H*3 (nullable)
 };
 
@@ -37,16 +36,10 @@ __device__ __forceinline__ void add_path(const DTArgs& a, unsigned pix, F3 L) {
     a.store[o + 2] = L.z;
     return;
   }
-  if (a.sum32) {
-    atomicAdd(a.sum32 + o, L.x);
-    atomicAdd(a.sum32 + o + 1, L.y);
-    atomicAdd(a.sum32 + o + 2, L.z);
-  }
-  if (a.sum64) {
-    atomicAdd(a.sum64 + o, (double)L.x);
-    atomicAdd(a.sum64 + o + 1, (double)L.y);
-    atomicAdd(a.sum64 + o + 2, (double)L.z);
-  }
+  if (L.x == 0.0f && L.y == 0.0f && L.z == 0.0f) return;  // nothing to add (a ray beside the volume)
+  atomicAdd(a.sum64 + o, (double)L.x);
+  atomicAdd(a.sum64 + o + 1, (double)L.y);
+  atomicAdd(a.sum64 + o + 2, (double)L.z);
   if (a.sumsq64) {
     atomicAdd(a.sumsq64 + o, (double)L.x * L.x);
     atomicAdd(a.sumsq64 + o + 1, (double)L.y * L.y);
@@ -125,9 +118,10 @@ __global__ void __launch_bounds__(128) k_delta_track(const __grid_constant__ DTA
   }
 }
 
-__global__ void k_scale(float* x, size_t n, float s) {
+// The mean of spp samples from their FP64 sum.
+__global__ void k_mean(const double* __restrict__ sum, float* __restrict__ x, size_t n, double spp) {
   size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  if (i < n) x[i] *= s;
+  if (i < n) x[i] = (float)(sum[i] / spp);
 }
 
 // SM count of the current device.
@@ -251,9 +245,9 @@ int check_params(const mr_render_params* p) {
   return MR_OK;
 }
 
-// Launch the tracer; exactly one of sum32 / sum64 is non-null.
-int launch_delta_track(Volume* v, const mr_render_params* p, float* sum32, double* sum64, double* sumsq64,
-                       cudaStream_t s) {
+// Launch the tracer: adds the samples' radiance to sum64 and, unless null,
+// its square to sumsq64.
+int launch_delta_track(Volume* v, const mr_render_params* p, double* sum64, double* sumsq64, cudaStream_t s) {
   if (!v->data_set) return set_error(MR_ERR_STATE, "render before mr_volume_set_data");
   if (!v->mips_valid) return set_error(MR_ERR_STATE, "render before mr_volume_update");
   DTArgs a;
@@ -273,7 +267,6 @@ int launch_delta_track(Volume* v, const mr_render_params* p, float* sum32, doubl
   a.counters = v->d_counters;
   a.store = nullptr;
   a.checker = a.flip = 0;
-  a.sum32 = sum32;
   a.sum64 = sum64;
   a.sumsq64 = sumsq64;
   MR_CUDA(cudaMemsetAsync(v->d_counters, 0, kCounters * sizeof(unsigned long long), s));
@@ -305,7 +298,6 @@ int launch_path_frame(Volume* v, const mr_render_params* p, uint32_t sample, int
   a.store = dev_rgb;
   a.checker = checker;
   a.flip = flip;
-  a.sum32 = nullptr;
   a.sum64 = a.sumsq64 = nullptr;
   MR_CUDA(cudaMemsetAsync(a.queue, 0, sizeof(unsigned long long), s));
   k_delta_track<<<dt_grid(), 128, 0, s>>>(a);
@@ -313,14 +305,25 @@ int launch_path_frame(Volume* v, const mr_render_params* p, uint32_t sample, int
   return MR_OK;
 }
 
+// A pixel's samples finish in any order. Their FP64 sum is exact for all but
+// extreme ranges of radiance, so two renders of one request agree, which fp32
+// sums in the order of the atomics did only by timing.
 int render_pt(Volume* v, const mr_render_params* p, float* dev_rgb, cudaStream_t s) {
-  size_t n = (size_t)p->width * p->height * 3;
-  MR_CUDA(cudaMemsetAsync(dev_rgb, 0, n * sizeof(float), s));
-  int rc = launch_delta_track(v, p, dev_rgb, nullptr, nullptr, s);
-  if (rc) return rc;
-  k_scale<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(dev_rgb, n, 1.0f / (float)p->spp);
-  MR_CUDA(cudaGetLastError());
-  return MR_OK;
+  const size_t n = (size_t)p->width * p->height * 3;
+  double* sum = nullptr;
+  cudaError_t e = pool_alloc((void**)&sum, n * sizeof(double), s);
+  if (e != cudaSuccess) return set_error(MR_ERR_NOMEM, "sample sums of %zu bytes: %s", n * sizeof(double), cudaGetErrorString(e));
+  int rc = MR_OK;
+  e = cudaMemsetAsync(sum, 0, n * sizeof(double), s);
+  if (e != cudaSuccess) rc = cuda_error(e, "cudaMemsetAsync(sample sums)");
+  if (rc == MR_OK) rc = launch_delta_track(v, p, sum, nullptr, s);
+  if (rc == MR_OK) {
+    k_mean<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(sum, dev_rgb, n, (double)p->spp);
+    e = cudaGetLastError();
+    if (e != cudaSuccess) rc = cuda_error(e, "k_mean");
+  }
+  MR_CUDA(cudaFreeAsync(sum, s));
+  return rc;
 }
 
 }  // namespace mr
@@ -333,5 +336,5 @@ extern "C" int mr_render_accumulate_f64(mr_volume* h, const mr_render_params* p,
   if (!h || !dev_sum) return set_error(MR_ERR_ARG, "mr_render_accumulate_f64: NULL argument");
   int rc = check_params(p);
   if (rc) return rc;
-  return launch_delta_track(&h->v, p, nullptr, dev_sum, dev_sumsq, (cudaStream_t)stream);
+  return launch_delta_track(&h->v, p, dev_sum, dev_sumsq, (cudaStream_t)stream);
 }
