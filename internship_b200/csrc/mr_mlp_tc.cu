@@ -831,8 +831,10 @@ __global__ void __launch_bounds__(128 * kGroups, 1) k_mlp_tc(const __grid_consta
   const uint32_t tcomb = c.tmem + c.tlane + 96;
 
   for (int it = 0;; ++it) {
-    // static tile striding over (CTA, group)
-    const int tile = (it * (int)gridDim.x + (int)blockIdx.x) * kGroups + g;
+    // static tile striding, over the CTAs first: few tiles, or the last ones,
+    // take an SM each instead of sharing one between four groups (8 tiles: 92 us
+    // on two SMs, 60 on eight; a batch of 8 views 2.90 -> 2.52 ms)
+    const int tile = (it * kGroups + g) * (int)gridDim.x + (int)blockIdx.x;
     if (tile * 128 >= n) break;  // group-uniform exit
     const int row = tile * 128 + t;
     const int kk = row < n ? row : n - 1;
@@ -1380,7 +1382,7 @@ int launch_mlp_tc(const Network* net, const float* desc, const float* aux, long 
   for (int i = 0; i < kTcLayers; ++i) a.winv[i] = f8 ? net->h_winv8[i] : 1.0f;
   a.err = (int*)((uint8_t*)net->packed + kWBytes);
   int tiles = (n + 127) / 128;
-  int grid = std::min(sm_count(), std::max(1, (tiles + kGroups - 1) / kGroups));
+  int grid = std::min(sm_count(), std::max(1, tiles));
   if (f8) k_mlp_tc<true><<<grid, 128 * kGroups, smem_bytes<true>(), s>>>(a);
   else k_mlp_tc<false><<<grid, 128 * kGroups, smem_bytes<false>(), s>>>(a);
   MR_CUDA(cudaGetLastError());

@@ -1100,6 +1100,27 @@ extern "C" int mr_sampler_selftest(int32_t n, const float* host_table, const flo
   return rc;
 }
 
+namespace mr {
+// n rows of 576 features -> chunks of 4 features: chunk j of row k at
+// out[(j * n + k) * 4]. A block moves 32 rows x 16 chunks through shared
+// memory: 256-byte row pieces in, 512-byte chunk pieces out.
+__global__ void __launch_bounds__(128) k_rows_to_chunks(const float* __restrict__ rows, int n, float* __restrict__ out) {
+  __shared__ float4 t[32][17];
+  const int r0 = blockIdx.x * 32, j0 = blockIdx.y * 16;
+#pragma unroll
+  for (int i = threadIdx.x; i < 32 * 16; i += 128) {
+    const int r = i >> 4, j = i & 15;
+    if (r0 + r < n) t[r][j] = __ldg(reinterpret_cast<const float4*>(rows + (size_t)(r0 + r) * 576) + j0 + j);
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = threadIdx.x; i < 32 * 16; i += 128) {
+    const int j = i >> 5, r = i & 31;
+    if (r0 + r < n) reinterpret_cast<float4*>(out)[(size_t)(j0 + j) * n + r0 + r] = t[r][j];
+  }
+}
+}  // namespace mr
+
 extern "C" int mr_radiance_predict(const mr_network* nh, int32_t precision, const float* dev_desc,
                                    const float* dev_aux, int32_t n, float* dev_out, void* stream) {
   clear_error();
@@ -1111,29 +1132,36 @@ extern "C" int mr_radiance_predict(const mr_network* nh, int32_t precision, cons
   cudaStream_t s = (cudaStream_t)stream;
   const bool tc = precision == MR_PREC_BF16 || precision == MR_PREC_FP8;
   if (!tc && precision != MR_PREC_FP32) return set_error(MR_ERR_ARG, "unknown precision %d", precision);
-  // The caller's descriptors stay untouched. fp32: trunk outputs (152) and the
-  // head's LC2 outputs (96) of a row go to a temporary; tensor cores: spill
-  // space for further heads, as rows may carry distinct albedo channels. Long
-  // tables run in pieces whose temporary the pool keeps (265 k rows, 251 MiB
-  // in fp32): 262 k rows took 1.20 ms in one piece, 1.26 in three, 1.31 in
-  // five (one wave of the trunk each, its outputs in L2).
-  const size_t per_row = tc ? 120 : 248;
-  const int piece = std::min(n, sm_count() * (tc ? 2048 : 14 * 128));
+  // The kernels read descriptors in chunks of 4 features, one row per thread:
+  // rows of 2304 bytes would cost a sector per thread and chunk, so a piece of
+  // the table is first brought into the render path's layout (k_rows_to_chunks).
+  // The caller's descriptors stay untouched. As in a render the fp32 network
+  // writes its trunk and LC2 outputs over consumed chunks; the tensor-core one
+  // has spill space for further heads, as rows may carry distinct albedo
+  // channels. Pieces are whole waves of the network's first kernel that the
+  // pool keeps (up to 250 MiB). 262 k fp32 rows: 1.20 ms reading rows, 0.98 ms
+  // in pieces of two waves, 1.07 in pieces of one; 1000 BF16 rows: 198 us, 66
+  // with their tiles on an SM each.
+  const size_t per_row = tc ? 576 + 120 : 576;
+  const int piece = std::min(n, sm_count() * (tc ? 512 : 2 * 3 * 128));
   float* tmp = nullptr;
   cudaError_t e = pool_alloc((void**)&tmp, (size_t)piece * per_row * sizeof(float), s);
   if (e != cudaSuccess) return set_error(MR_ERR_NOMEM, "network temporary: %s", cudaGetErrorString(e));
   int rc = MR_OK;
   for (int r0 = 0; r0 < n && rc == MR_OK; r0 += piece) {
     const int m = std::min(piece, n - r0);
-    const float* d = dev_desc + (size_t)r0 * 576;
+    const long long cs = 4ll * m;
     const float* a = dev_aux + (size_t)r0 * 5;
     float* o = dev_out + (size_t)r0 * 3;
-    if (tc)
-      rc = launch_mlp_tc(&nh->n, d, a, 576, 4, 5, 1, m, o, nullptr, nullptr, nullptr, f3(1, 1, 1), f3(1, 1, 1), tmp,
-                         precision == MR_PREC_FP8, s);
+    k_rows_to_chunks<<<dim3((unsigned)((m + 31) / 32), 576 / 4 / 16), 128, 0, s>>>(dev_desc + (size_t)r0 * 576, m, tmp);
+    e = cudaGetLastError();
+    if (e != cudaSuccess) rc = cuda_error(e, "k_rows_to_chunks");
+    else if (tc)
+      rc = launch_mlp_tc(&nh->n, tmp, a, 4, cs, 5, 1, m, o, nullptr, nullptr, nullptr, f3(1, 1, 1), f3(1, 1, 1),
+                         tmp + (size_t)m * 576, precision == MR_PREC_FP8, s);
     else
-      rc = launch_mlp_simt(&nh->n, d, a, 576, 4, 5, 1, m, nullptr, o, nullptr, nullptr, f3(1, 1, 1), f3(1, 1, 1), s,
-                           nullptr, nullptr, tmp, 248, 4, tmp + 152, 248, 4);
+      rc = launch_mlp_simt(&nh->n, tmp, a, 4, cs, 5, 1, m, nullptr, o, nullptr, nullptr, f3(1, 1, 1), f3(1, 1, 1), s,
+                           nullptr, nullptr, tmp, 4, cs, tmp + 48 * cs, 4, cs);
   }
   MR_CUDA(cudaFreeAsync(tmp, s));
   return rc;
