@@ -429,6 +429,8 @@ static int fwd_bwd(Trainer& t, const float* desc, const float* aux, const float*
   a.wk.dsp = take(12);
   a.wk.a3 = take(32);
   a.wk.da3 = take(32);
+  a.wk.xs = take(3 * kTrunkSaved);
+  a.wk.mask = reinterpret_cast<uint16_t*>(take(kTrunkMaskFloats));
   const bool tc = t.precision == MR_PREC_BF16;
   int rc = tc ? launch_head_pack(t.w, t.img, s) : (int)MR_OK;
   for (int r0 = 0; r0 < n && !rc; r0 += kStepRows) {

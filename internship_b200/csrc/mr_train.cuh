@@ -80,8 +80,16 @@ struct TrainWork {
   float* dsp;    // 2 x 6: gradients of the output gates, two partial sums
   float* a3;     // BF16 step: LC2 output after ReLU, rows x 32
   float* da3;    // BF16 step: its gradient, 0 where a3 is 0
+  // For the trunks' backward, per tile of kTrainRows rows and branch:
+  float* xs;       // [kTrunkSaved][kTrainRows]: every layer's input, then the two outputs
+  uint16_t* mask;  // kTrunkMask bytes: the signs of every layer's outputs
 };
-constexpr size_t kTrainWorkFloats = 128 + 128 + 72 + 36 + 6 + 72 + 12 + 32 + 32;  // per row
+constexpr int kTrunkSaved = 232 + 40;         // features
+constexpr int kTrunkMask = 14 * 128 * 2;      // bytes: layers, threads
+static_assert(3 * kTrunkMask % (4 * kTrainRows) == 0, "whole floats per row");
+constexpr size_t kTrunkMaskFloats = 3 * kTrunkMask / (4 * kTrainRows);  // per row
+constexpr size_t kTrainWorkFloats =           // per row
+    128 + 128 + 72 + 36 + 6 + 72 + 12 + 32 + 32 + 3 * kTrunkSaved + kTrunkMaskFloats;
 
 struct TrainArgs {
   const float* w;       // fp32 master weights (blob layout)

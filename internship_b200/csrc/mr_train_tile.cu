@@ -4,9 +4,10 @@
 //
 //   k_train_stats   pooled descriptor statistics, the squeeze-excitation
 //                   gates of every block, the trunk-output gates and LGGS
-//   k_train_trunk   the trunks of one branch (density, transmittance or
-//                   phase): forward to the head input, or, with the forward
-//                   recomputed, backward from its gradient
+//   k_train_trunk_fwd, k_train_trunk_bwd
+//                   the trunks of one branch (density, transmittance or
+//                   phase): forward to the head input, backward from its
+//                   gradient
 //   k_train_head    LC0 / LC1 / LC2, the tail and the loss, forward and
 //                   backward (fp32 step)
 //   k_train_tail    the tail and the loss alone (BF16 step, between the
@@ -15,8 +16,7 @@
 //
 // The gates depend on descriptor statistics alone, so the three branches of
 // the trunks are independent of one another given the gates, and each CTA
-// runs one branch: its weights (25 KB) and a tile's layer inputs (63 KB) stay
-// in shared memory, two CTAs per SM.
+// runs one branch with its weights (25 KB) in shared memory.
 //
 // A tile's activations are stored feature-major, 64 rows padded to 68 floats:
 // a thread's 4 x 4 (or 4 x 8) piece of a layer reads four rows of a feature
@@ -139,7 +139,13 @@ __global__ void __launch_bounds__(256) k_train_stats(TrainArgs a) {
 // each layer's weights, rows padded by 4 floats and stored in the order
 // slot(o) = o / NC + 8 (o % NC) (NC = S / 8 columns per thread), which puts
 // the rows that the four column groups of a warp read at once into distinct
-// banks; and each layer's input tile.
+// banks; and the input tiles of two layers in turn.
+//
+// The forward kernel writes every layer's input, the trunks' outputs and the
+// signs of all outputs to memory (wk.xs, wk.mask); the backward kernel copies
+// the inputs back one layer ahead. 65,536 rows: forward 226 -> 180 us and
+// backward 502 -> 287 us against keeping a tile's 232 inputs in shared memory
+// and running the forward again (two CTAs per SM; now five and three).
 constexpr int kTrunkThreads = 128;
 __host__ __device__ constexpr int layer_width(int l) {
   return l < 2 ? 8 : l < 5 ? 16 : l < 9 ? 32 : 8;
@@ -155,8 +161,11 @@ __host__ __device__ constexpr int layer_x(int l) {  // first feature of layer l'
   return o;
 }
 constexpr int kLayers = 14, kTrunkW = layer_w(kLayers), kTrunkX = layer_x(kLayers);
-static_assert(kTrunkX == 232 && layer_x(8) == 160 && layer_x(9) == 192, "descriptor features sit at their own offset");
-constexpr int kTrunkSmem = (kTrunkW + kTrunkX + (kTrunkX + 64) * kRS) * 4 + kLayers * kTrunkThreads * 2;
+static_assert(kTrunkX + 40 == kTrunkSaved && kLayers * kTrunkThreads * 2 == kTrunkMask, "the sizes in mr_train.cuh");
+// forward: weights, biases, two input tiles of 32 features; backward: weights,
+// two input tiles and two gradient buffers
+constexpr int kFwdSmem = (kTrunkW + kTrunkX + 64 * kRS) * 4;
+constexpr int kBwdSmem = (kTrunkW + 128 * kRS) * 4;
 
 // Blob offsets of layer l of branch br.
 __device__ __forceinline__ int layer_wg(const TrainTables& T, int l, int br) {
@@ -167,19 +176,65 @@ __device__ __forceinline__ int layer_bg(const TrainTables& T, int l, int br) {
 }
 
 struct TrunkCtx {
-  float *Ws, *Bs, *X, *D;  // weights, biases, layer inputs, two gradient buffers of 32 features
-  uint16_t* mask;          // [layer][thread]: pre-activation > 0, bit 4 j + r
+  float *Ws, *Bs, *X, *D;  // weights, biases, input tiles, gradient buffers (two of 32 features each)
+  float* xs;               // the tile's and branch's piece of wk.xs
+  uint16_t* mask;          // and of wk.mask: [layer][thread], pre-activation > 0, bit 4 j + r
   const TrainArgs* a;
   int br, r0, rg, c, t;
-  float inv;
 };
 
-// Rows 4 rg .. 4 rg + 3, outputs c NC .. c NC + NC - 1 of layer l: bias after
-// the sum over ascending inputs.
+__device__ __forceinline__ void trunk_ctx(TrunkCtx& k, const TrainArgs& a) {
+  k.a = &a;
+  k.br = blockIdx.x % 3;
+  k.t = threadIdx.x;
+  const int warp = k.t >> 5, lane = k.t & 31;
+  k.rg = (lane & 7) + 8 * (warp & 1);
+  k.c = (lane >> 3) + 4 * (warp >> 1);
+}
+__device__ __forceinline__ void trunk_tile(TrunkCtx& k, int tile) {
+  k.r0 = tile * kR;
+  const size_t q = (size_t)tile * 3 + k.br;
+  k.xs = k.a->wk.xs + q * (kTrunkSaved * kR);
+  k.mask = k.a->wk.mask + q * (kTrunkMask / 2);
+}
+__device__ __forceinline__ void trunk_weights(const TrunkCtx& k, bool biases) {
+#pragma unroll 1
+  for (int l = 0; l < kLayers; ++l) {
+    const int S = layer_width(l), nc = S / 8, wg = layer_wg(c_tt, l, k.br), bg = layer_bg(c_tt, l, k.br);
+    for (int i = k.t; i < S * S; i += kTrunkThreads) {
+      const int o = i / S, c = i - o * S;
+      k.Ws[layer_w(l) + (o / nc + 8 * (o % nc)) * (S + 4) + c] = __ldg(k.a->w + wg + i);
+    }
+    if (biases && k.t < S) k.Bs[layer_x(l) + k.t] = __ldg(k.a->w + bg + k.t);
+  }
+}
+
+// The descriptor features of layer l (a block's) at the caller's rows and
+// columns: s[r][j].
 template <int NC>
-__device__ __forceinline__ void tile_fwd(const TrunkCtx& k, int l, float (&y)[NC][4]) {
+__device__ __forceinline__ void load_features(const TrunkCtx& k, int block, float (&s)[4][NC]) {
+  const int f = k.br * 192 + c_tt.from[block] + k.c * NC;
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    const float* p = k.a->desc + (size_t)min(k.r0 + 4 * k.rg + r, k.a->n - 1) * 576 + f;
+    if constexpr (NC == 4) {
+      const float4 v = __ldg(reinterpret_cast<const float4*>(p));
+      s[r][0] = v.x; s[r][1] = v.y; s[r][2] = v.z; s[r][3] = v.w;
+    } else if constexpr (NC == 2) {
+      const float2 v = __ldg(reinterpret_cast<const float2*>(p));
+      s[r][0] = v.x; s[r][1] = v.y;
+    } else {
+      s[r][0] = __ldg(p);
+    }
+  }
+}
+
+// Rows 4 rg .. 4 rg + 3, outputs c NC .. c NC + NC - 1 of layer l from the
+// input tile x: bias after the sum over ascending inputs.
+template <int NC>
+__device__ __forceinline__ void tile_fwd(const TrunkCtx& k, int l, const float* x, float (&y)[NC][4]) {
   constexpr int S = 8 * NC;
-  const float* x = k.X + layer_x(l) * kRS + 4 * k.rg;
+  x += 4 * k.rg;
   const float* w = k.Ws + layer_w(l) + k.c * (S + 4);
 #pragma unroll
   for (int j = 0; j < NC; ++j)
@@ -217,65 +272,138 @@ __device__ __forceinline__ void tile_fwd(const TrunkCtx& k, int l, float (&y)[NC
   k.mask[l * kTrunkThreads + k.t] = (uint16_t)m;
 }
 
-// Blocks l .. l + COUNT - 1 of one width (l counts layers; the block is
-// l - shift). y: the running output, in and out; with `rep` the last block
-// doubles the width (REP3) and leaves its output in the next layer's input
-// tile. The tile's descriptor features sit in the layers' input slots and are
-// replaced there by the layer inputs.
+// A layer's input, the caller's piece, to its tile and to memory.
 template <int NC>
-__device__ __forceinline__ void blocks_fwd(const TrunkCtx& k, int l, int count, int shift, bool rep, float (&y)[NC][4]) {
+__device__ __forceinline__ void put_input(const TrunkCtx& k, int l, float* x, int j, float a, float b, float c, float d) {
+  st4(x + (k.c * NC + j) * kRS + 4 * k.rg, a, b, c, d);
+  st4(k.xs + (layer_x(l) + k.c * NC + j) * kR + 4 * k.rg, a, b, c, d);
+}
+
+// Blocks l .. l + count - 1 of one width (l counts layers; the block is
+// l - shift). y: the running output, in and out; with `rep` the last block
+// doubles the width (REP3) and leaves its output in the next input tile for
+// take_wide. buf: the input tile to use, alternating (one barrier a layer).
+template <int NC>
+__device__ __forceinline__ void blocks_fwd(const TrunkCtx& k, int l, int count, int shift, bool rep, int& buf,
+                                           float (&y)[NC][4]) {
   constexpr int S = 8 * NC;
+  auto gate = [&](int l) {
+    return ld4(k.a->wk.gate + (size_t)(3 * (l - shift) + k.br) * k.a->wk.rows + k.r0 + 4 * k.rg);
+  };
+  float s[4][NC];
+  load_features<NC>(k, l - shift, s);
+  float4 g = gate(l);
 #pragma unroll 1
   for (int n = 0; n < count; ++n, ++l) {
-    const float4 g = ld4(k.a->wk.gate + (size_t)(3 * (l - shift) + k.br) * k.a->wk.rows + k.r0 + 4 * k.rg);
-    float* x = k.X + (layer_x(l) + k.c * NC) * kRS + 4 * k.rg;
-    float4 s[NC];
+    float* x = k.X + buf * 32 * kRS;
+    buf ^= 1;
 #pragma unroll
-    for (int j = 0; j < NC; ++j) {
-      s[j] = ld4(x + j * kRS);
-      st4(x + j * kRS, fmaf(s[j].x, g.x, y[j][0]), fmaf(s[j].y, g.y, y[j][1]), fmaf(s[j].z, g.z, y[j][2]),
-          fmaf(s[j].w, g.w, y[j][3]));
-    }
+    for (int j = 0; j < NC; ++j)
+      put_input<NC>(k, l, x, j, fmaf(s[0][j], g.x, y[j][0]), fmaf(s[1][j], g.y, y[j][1]), fmaf(s[2][j], g.z, y[j][2]),
+                    fmaf(s[3][j], g.w, y[j][3]));
     __syncthreads();
-    tile_fwd<NC>(k, l, y);
+    float sn[4][NC];
+    if (n + 1 < count) {  // lands during the products
+      load_features<NC>(k, l + 1 - shift, sn);
+      g = gate(l + 1);
+    }
+    tile_fwd<NC>(k, l, x, y);
     if (rep && n == count - 1) {
-      // the next layer's slots still hold its descriptor features: the wider
-      // y goes through the gradient buffers
+      float* o = k.X + buf * 32 * kRS;
 #pragma unroll
       for (int j = 0; j < NC; ++j) {
-        st4(k.D + (k.c * NC + j) * kRS + 4 * k.rg, y[j]);
-        *reinterpret_cast<float4*>(k.D + (S + k.c * NC + j) * kRS + 4 * k.rg) = s[j];
+        st4(o + (k.c * NC + j) * kRS + 4 * k.rg, y[j]);
+        st4(o + (S + k.c * NC + j) * kRS + 4 * k.rg, s[0][j], s[1][j], s[2][j], s[3][j]);
       }
     } else {
 #pragma unroll
-      for (int j = 0; j < NC; ++j) {
-        y[j][0] += s[j].x; y[j][1] += s[j].y; y[j][2] += s[j].z; y[j][3] += s[j].w;
-      }
+      for (int j = 0; j < NC; ++j)
+#pragma unroll
+        for (int r = 0; r < 4; ++r) y[j][r] += s[r][j];
     }
+    if (n + 1 < count)
+#pragma unroll
+      for (int j = 0; j < NC; ++j)
+#pragma unroll
+        for (int r = 0; r < 4; ++r) s[r][j] = sn[r][j];
   }
 }
+// The wide output in the wider column split. The tile it sits in is the next
+// layer's: every thread overwrites the piece it read.
 template <int NC>
-__device__ __forceinline__ void take_wide(const TrunkCtx& k, float (&y)[NC][4]) {
+__device__ __forceinline__ void take_wide(const TrunkCtx& k, int buf, float (&y)[NC][4]) {
   __syncthreads();
 #pragma unroll
   for (int j = 0; j < NC; ++j) {
-    const float4 v = ld4(k.D + (k.c * NC + j) * kRS + 4 * k.rg);
+    const float4 v = ld4(k.X + buf * 32 * kRS + (k.c * NC + j) * kRS + 4 * k.rg);
     y[j][0] = v.x; y[j][1] = v.y; y[j][2] = v.z; y[j][3] = v.w;
   }
 }
-// y into layer l's input tile (L81, LD41), then the layer.
+// L81 and LD41: y is the layer's input.
 template <int NC>
-__device__ __forceinline__ void last_fwd(const TrunkCtx& k, int l, float (&y)[NC][4]) {
+__device__ __forceinline__ void last_fwd(const TrunkCtx& k, int l, int& buf, float (&y)[NC][4]) {
+  float* x = k.X + buf * 32 * kRS;
+  buf ^= 1;
 #pragma unroll
-  for (int j = 0; j < NC; ++j) st4(k.X + (layer_x(l) + k.c * NC + j) * kRS + 4 * k.rg, y[j]);
+  for (int j = 0; j < NC; ++j) put_input<NC>(k, l, x, j, y[j][0], y[j][1], y[j][2], y[j][3]);
   __syncthreads();
-  tile_fwd<NC>(k, l, y);
+  tile_fwd<NC>(k, l, x, y);
 }
 
-// Weight gradient of layer l, dW[o][i] += sum over rows of D[o] X[i], and the
+// Head-input columns of a trunk: y = relu(L81 or LD41) times its output gate.
+// y itself is kept as feature kTrunkX + at + column, for the gate's gradient.
+template <int NC>
+__device__ __forceinline__ void put_h0(const TrunkCtx& k, int col, int at, const float4 sp, const float (&y)[NC][4]) {
+#pragma unroll
+  for (int j = 0; j < NC; ++j) st4(k.xs + (kTrunkX + at + k.c * NC + j) * kR + 4 * k.rg, y[j]);
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    float* p = k.a->wk.h0 + (size_t)(k.r0 + 4 * k.rg + r) * 128 + col + k.c * NC;
+    const float g = (&sp.x)[r];
+    if constexpr (NC == 4)
+      st4(p, y[0][r] * g, y[1][r] * g, y[2][r] * g, y[3][r] * g);
+    else
+      p[0] = y[0][r] * g;
+  }
+}
+
+// CTA b: branch b % 3, tiles b / 3, b / 3 + gridDim / 3, ...
+__global__ void __launch_bounds__(kTrunkThreads, 5) k_train_trunk_fwd(const __grid_constant__ TrainArgs a) {
+  extern __shared__ __align__(16) float sm[];
+  TrunkCtx k;
+  trunk_ctx(k, a);
+  k.Ws = sm;
+  k.Bs = k.Ws + kTrunkW;
+  k.X = k.Bs + kTrunkX;
+  trunk_weights(k, true);
+  __syncthreads();
+  const int tiles = (a.n + kR - 1) / kR;
+  const size_t N = a.wk.rows;
+  int buf = 0;
+  for (int tile = blockIdx.x / 3; tile < tiles; tile += gridDim.x / 3) {
+    trunk_tile(k, tile);
+    {
+      float y1[1][4] = {}, y2[2][4], y4[4][4];
+      blocks_fwd<1>(k, 0, 2, 0, true, buf, y1);
+      take_wide<2>(k, buf, y2);
+      blocks_fwd<2>(k, 2, 3, 0, true, buf, y2);
+      take_wide<4>(k, buf, y4);
+      blocks_fwd<4>(k, 5, 3, 0, false, buf, y4);
+      last_fwd<4>(k, 8, buf, y4);
+      put_h0<4>(k, 32 * k.br, 0, ld4(a.wk.sp + (size_t)k.br * N + k.r0 + 4 * k.rg), y4);
+    }
+    float yl[1][4] = {};
+    blocks_fwd<1>(k, 9, 4, 1, false, buf, yl);
+    last_fwd<1>(k, 13, buf, yl);
+    put_h0<1>(k, 96 + 8 * k.br, 32, ld4(a.wk.sp + (size_t)(3 + k.br) * N + k.r0 + 4 * k.rg), yl);
+  }
+}
+
+// Weight gradient of layer l, dW[o][i] += sum over rows of D[o] x[i], and the
 // bias gradient from the caller's own rows of D.
 template <int NC>
-__device__ __forceinline__ void tile_dw(const TrunkCtx& k, int l, const float* D, const float (&dp)[NC][4]) {
+__device__ __forceinline__ void tile_dw(const TrunkCtx& k, int l, const float* x, const float* D,
+                                        const float (&dp)[NC][4]) {
   constexpr int S = 8 * NC;
   float* G = k.a->grad;
   const int wg = layer_wg(c_tt, l, k.br), bg = layer_bg(c_tt, l, k.br);
@@ -287,7 +415,7 @@ __device__ __forceinline__ void tile_dw(const TrunkCtx& k, int l, const float* D
     if ((k.t & 7) == 0) add_grad(G + bg + k.c * NC + j, s);
   }
   const int ig = k.t & 7, og = k.t >> 3;
-  const float* x = k.X + (layer_x(l) + ig) * kRS;
+  x += ig * kRS;
   if constexpr (NC == 1) {  // 64 weights: each half of the threads sums half the rows
     const float* d = D + (og & 7) * kRS;
     const int k0 = (k.t >> 6) * (kR / 2);
@@ -321,21 +449,62 @@ __device__ __forceinline__ void tile_dw(const TrunkCtx& k, int l, const float* D
   }
 }
 
-// Backward of layer l: d = gradient of its ReLU output in, of its input out.
-// buf: which gradient buffer to use (alternating layers, one barrier each).
+// The backward pass takes the layers in the order 8 (L81), 7 .. 0, 13 (LD41),
+// 12 .. 9: step i is layer bwd_layer(i).
+__device__ __forceinline__ int bwd_layer(int i) { return i < 9 ? 8 - i : 22 - i; }
+
+struct BwdState {
+  int step;       // layers of the tile done
+  int buf;        // gradient buffer to use next
+  int next;       // the CTA's next tile, or -1
+  uint32_t mask;  // the next layer's signs
+};
+
+// Starts the copy of a step's layer inputs into input tile step & 1 and loads
+// its signs; step kLayers is the next tile's first.
+__device__ __forceinline__ void fetch_step(const TrunkCtx& k, BwdState& b, int step) {
+  const float* xs = k.xs;
+  const uint16_t* mask = k.mask;
+  if (step == kLayers) {
+    if (b.next < 0) return;
+    const size_t q = (size_t)b.next * 3 + k.br;
+    xs = k.a->wk.xs + q * (kTrunkSaved * kR);
+    mask = k.a->wk.mask + q * (kTrunkMask / 2);
+    step = 0;
+  }
+  const int l = bwd_layer(step), at = layer_x(l);
+  const uint32_t dst = (uint32_t)__cvta_generic_to_shared(k.X + (step & 1) * 32 * kRS);
+  for (int i = k.t; i < layer_width(l) * (kR / 4); i += kTrunkThreads) {
+    const int f = i / (kR / 4), q = i % (kR / 4);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + (f * kRS + 4 * q) * 4),
+                 "l"(xs + (at + f) * kR + 4 * q)
+                 : "memory");
+  }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  b.mask = mask[l * kTrunkThreads + k.t];
+}
+
+// Backward of the next layer in order (l): d = gradient of its ReLU output in,
+// of its input out. One barrier: the gradient buffers and the input tiles
+// alternate, and a tile is refilled only after the barrier behind its last
+// reads.
 template <int NC>
-__device__ __forceinline__ void tile_bwd(const TrunkCtx& k, int l, int buf, float (&d)[NC][4]) {
+__device__ __forceinline__ void tile_bwd(const TrunkCtx& k, BwdState& b, int l, float (&d)[NC][4]) {
   constexpr int S = 8 * NC;
-  const uint32_t m = k.mask[l * kTrunkThreads + k.t];
-  float* D = k.D + buf * 32 * kRS;
+  const uint32_t m = b.mask;
+  const int i = b.step++;
+  float* D = k.D + b.buf * 32 * kRS;
+  b.buf ^= 1;
 #pragma unroll
   for (int j = 0; j < NC; ++j) {
 #pragma unroll
     for (int r = 0; r < 4; ++r) d[j][r] = (m >> (4 * j + r)) & 1u ? d[j][r] : 0.0f;
     st4(D + (k.c * NC + j) * kRS + 4 * k.rg, d[j]);
   }
+  asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
-  tile_dw<NC>(k, l, D, d);
+  fetch_step(k, b, i + 1);
+  tile_dw<NC>(k, l, k.X + (i & 1) * 32 * kRS, D, d);
 #pragma unroll
   for (int j = 0; j < NC; ++j)
 #pragma unroll
@@ -379,29 +548,14 @@ __device__ __forceinline__ void row_sums(const TrunkCtx& k, float* half0, size_t
   if ((k.t & 31) < 8) st4(half0 + (k.t >> 6) * half_stride + k.r0 + 4 * k.rg, s);
 }
 
-// Blocks l, l - 1, ..., l - COUNT + 1 backward; d as in tile_bwd.
+// Blocks l, l - 1, ..., l - count + 1 backward; d as in tile_bwd.
 template <int NC>
-__device__ __forceinline__ void blocks_bwd(const TrunkCtx& k, int l, int count, int shift, int& buf, float (&d)[NC][4]) {
+__device__ __forceinline__ void blocks_bwd(const TrunkCtx& k, BwdState& b, int l, int count, int shift, float (&d)[NC][4]) {
 #pragma unroll 1
   for (int n = 0; n < count; ++n, --l) {
-    // this block's descriptor features, for the gate's gradient
-    const int f = k.br * 192 + c_tt.from[l - shift] + k.c * NC;
     float s[4][NC];
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      const float* p = k.a->desc + (size_t)min(k.r0 + 4 * k.rg + r, k.a->n - 1) * 576 + f;
-      if constexpr (NC == 4) {
-        const float4 v = __ldg(reinterpret_cast<const float4*>(p));
-        s[r][0] = v.x; s[r][1] = v.y; s[r][2] = v.z; s[r][3] = v.w;
-      } else if constexpr (NC == 2) {
-        const float2 v = __ldg(reinterpret_cast<const float2*>(p));
-        s[r][0] = v.x; s[r][1] = v.y;
-      } else {
-        s[r][0] = __ldg(p);
-      }
-    }
-    tile_bwd<NC>(k, l, buf, d);
-    buf ^= 1;
+    load_features<NC>(k, l - shift, s);  // for the gate's gradient; lands during the products
+    tile_bwd<NC>(k, b, l, d);
     float dg[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
     for (int r = 0; r < 4; ++r)
@@ -414,9 +568,9 @@ __device__ __forceinline__ void blocks_bwd(const TrunkCtx& k, int l, int count, 
 // The first half of a wide gradient (the ReLU part of REP3's output) in the
 // narrower column split.
 template <int NC>
-__device__ __forceinline__ void narrow(const TrunkCtx& k, int& buf, const float (&w)[2 * NC][4], float (&d)[NC][4]) {
-  float* D = k.D + buf * 32 * kRS;
-  buf ^= 1;
+__device__ __forceinline__ void narrow(const TrunkCtx& k, BwdState& b, const float (&w)[2 * NC][4], float (&d)[NC][4]) {
+  float* D = k.D + b.buf * 32 * kRS;
+  b.buf ^= 1;
 #pragma unroll
   for (int j = 0; j < 2 * NC; ++j) st4(D + (k.c * 2 * NC + j) * kRS + 4 * k.rg, w[j]);
   __syncthreads();
@@ -427,23 +581,16 @@ __device__ __forceinline__ void narrow(const TrunkCtx& k, int& buf, const float 
   }
 }
 
-// Head-input columns of a trunk: y = relu(L81 or LD41) times its output gate.
+// The head input's gradient at a trunk's columns: d = dh0 * gate, and the
+// gate's own gradient sum(dh0 * y).
 template <int NC>
-__device__ __forceinline__ void put_h0(const TrunkCtx& k, int col, const float4 sp, const float (&y)[NC][4]) {
+__device__ __forceinline__ void take_dh0(const TrunkCtx& k, int col, int at, const float4 sp, float* dsp, float (&d)[NC][4]) {
+  float y[NC][4];
 #pragma unroll
-  for (int r = 0; r < 4; ++r) {
-    float* p = k.a->wk.h0 + (size_t)(k.r0 + 4 * k.rg + r) * 128 + col + k.c * NC;
-    const float g = (&sp.x)[r];
-    if constexpr (NC == 4)
-      st4(p, y[0][r] * g, y[1][r] * g, y[2][r] * g, y[3][r] * g);
-    else
-      p[0] = y[0][r] * g;
+  for (int j = 0; j < NC; ++j) {
+    const float4 v = ld4(k.xs + (kTrunkX + at + k.c * NC + j) * kR + 4 * k.rg);
+    y[j][0] = v.x; y[j][1] = v.y; y[j][2] = v.z; y[j][3] = v.w;
   }
-}
-// Its gradient: d = dh0 * gate, and the gate's own gradient sum(dh0 * y).
-template <int NC>
-__device__ __forceinline__ void take_dh0(const TrunkCtx& k, int col, const float4 sp, float* dsp, const float (&y)[NC][4],
-                                         float (&d)[NC][4]) {
   float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
   for (int r = 0; r < 4; ++r) {
@@ -465,81 +612,38 @@ __device__ __forceinline__ void take_dh0(const TrunkCtx& k, int col, const float
   row_sums(k, dsp, (size_t)6 * k.a->wk.rows, s);
 }
 
-// CTA b: branch b % 3, tiles b / 3, b / 3 + gridDim / 3, ...
-template <bool BWD>
-__global__ void __launch_bounds__(kTrunkThreads, 2) k_train_trunk(const __grid_constant__ TrainArgs a) {
+__global__ void __launch_bounds__(kTrunkThreads, 3) k_train_trunk_bwd(const __grid_constant__ TrainArgs a) {
   extern __shared__ __align__(16) float sm[];
   TrunkCtx k;
+  trunk_ctx(k, a);
   k.Ws = sm;
-  k.Bs = k.Ws + kTrunkW;
-  k.X = k.Bs + kTrunkX;
-  k.D = k.X + kTrunkX * kRS;
-  k.mask = reinterpret_cast<uint16_t*>(k.D + 64 * kRS);
-  k.a = &a;
-  k.br = blockIdx.x % 3;
-  k.t = threadIdx.x;
-  const int warp = k.t >> 5, lane = k.t & 31;
-  k.rg = (lane & 7) + 8 * (warp & 1);
-  k.c = (lane >> 3) + 4 * (warp >> 1);
-#pragma unroll 1
-  for (int l = 0; l < kLayers; ++l) {
-    const int S = layer_width(l), nc = S / 8, wg = layer_wg(c_tt, l, k.br), bg = layer_bg(c_tt, l, k.br);
-    for (int i = k.t; i < S * S; i += kTrunkThreads) {
-      const int o = i / S, c = i - o * S;
-      k.Ws[layer_w(l) + (o / nc + 8 * (o % nc)) * (S + 4) + c] = __ldg(a.w + wg + i);
-    }
-    if (k.t < S) k.Bs[layer_x(l) + k.t] = __ldg(a.w + bg + k.t);
-  }
-  const int tiles = (a.n + kR - 1) / kR;
+  k.Bs = nullptr;
+  k.X = k.Ws + kTrunkW;
+  k.D = k.X + 64 * kRS;
+  const int tiles = (a.n + kR - 1) / kR, stride = gridDim.x / 3;
   const size_t N = a.wk.rows;
-  for (int tile = blockIdx.x / 3; tile < tiles; tile += gridDim.x / 3) {
-    k.r0 = tile * kR;
-    __syncthreads();  // the previous tile's reads of X
-    // descriptor features into the layers' input slots, transposed 4 x 4
-    for (int i = k.t; i < 48 * 16; i += kTrunkThreads) {
-      const int rg = i & 15, cg = i >> 4;
-      float4 v[4];
-#pragma unroll
-      for (int r = 0; r < 4; ++r)
-        v[r] = __ldg(reinterpret_cast<const float4*>(a.desc + (size_t)min(k.r0 + 4 * rg + r, a.n - 1) * 576 +
-                                                     k.br * 192) + cg);
-      float* x = k.X + (4 * cg + (cg >= 40 ? 32 : 0)) * kRS + 4 * rg;
-      st4(x, v[0].x, v[1].x, v[2].x, v[3].x);
-      st4(x + kRS, v[0].y, v[1].y, v[2].y, v[3].y);
-      st4(x + 2 * kRS, v[0].z, v[1].z, v[2].z, v[3].z);
-      st4(x + 3 * kRS, v[0].w, v[1].w, v[2].w, v[3].w);
-    }
-    __syncthreads();
-    const float4 spm = ld4(a.wk.sp + (size_t)k.br * N + k.r0 + 4 * k.rg);
-    const float4 spl = ld4(a.wk.sp + (size_t)(3 + k.br) * N + k.r0 + 4 * k.rg);
-    float y1[1][4] = {}, y2[2][4], y4[4][4], yl[1][4] = {};
-    blocks_fwd<1>(k, 0, 2, 0, true, y1);
-    take_wide<2>(k, y2);
-    blocks_fwd<2>(k, 2, 3, 0, true, y2);
-    take_wide<4>(k, y4);
-    blocks_fwd<4>(k, 5, 3, 0, false, y4);
-    last_fwd<4>(k, 8, y4);
-    blocks_fwd<1>(k, 9, 4, 1, false, yl);
-    last_fwd<1>(k, 13, yl);
-    if constexpr (!BWD) {
-      put_h0<4>(k, 32 * k.br, spm, y4);
-      put_h0<1>(k, 96 + 8 * k.br, spl, yl);
-    } else {
-      int buf = 0;
+  BwdState b{0, 0, (int)blockIdx.x / 3, 0};
+  if (b.next < tiles) fetch_step(k, b, kLayers);
+  trunk_weights(k, false);  // the first layer's barrier is behind them
+  for (int tile = blockIdx.x / 3; tile < tiles; tile += stride) {
+    trunk_tile(k, tile);
+    b.step = 0;
+    b.next = tile + stride < tiles ? tile + stride : -1;
+    {
       float d4[4][4], d2[2][4], d1[1][4];
-      take_dh0<4>(k, 32 * k.br, spm, a.wk.dsp + (size_t)k.br * N, y4, d4);
-      tile_bwd<4>(k, 8, buf, d4);
-      buf ^= 1;
-      blocks_bwd<4>(k, 7, 3, 0, buf, d4);
-      narrow<2>(k, buf, d4, d2);
-      blocks_bwd<2>(k, 4, 3, 0, buf, d2);
-      narrow<1>(k, buf, d2, d1);
-      blocks_bwd<1>(k, 1, 2, 0, buf, d1);
-      take_dh0<1>(k, 96 + 8 * k.br, spl, a.wk.dsp + (size_t)(3 + k.br) * N, yl, d1);
-      tile_bwd<1>(k, 13, buf, d1);
-      buf ^= 1;
-      blocks_bwd<1>(k, 12, 4, 1, buf, d1);
+      take_dh0<4>(k, 32 * k.br, 0, ld4(a.wk.sp + (size_t)k.br * N + k.r0 + 4 * k.rg), a.wk.dsp + (size_t)k.br * N, d4);
+      tile_bwd<4>(k, b, 8, d4);
+      blocks_bwd<4>(k, b, 7, 3, 0, d4);
+      narrow<2>(k, b, d4, d2);
+      blocks_bwd<2>(k, b, 4, 3, 0, d2);
+      narrow<1>(k, b, d2, d1);
+      blocks_bwd<1>(k, b, 1, 2, 0, d1);
     }
+    float dl[1][4];
+    take_dh0<1>(k, 96 + 8 * k.br, 32, ld4(a.wk.sp + (size_t)(3 + k.br) * N + k.r0 + 4 * k.rg),
+                a.wk.dsp + (size_t)(3 + k.br) * N, dl);
+    tile_bwd<1>(k, b, 13, dl);
+    blocks_bwd<1>(k, b, 12, 4, 1, dl);
   }
 }
 
@@ -1139,17 +1243,17 @@ __global__ void __launch_bounds__(256, 2) k_train_gates(const __grid_constant__ 
 static int tile_attrs() {
   static DeviceCache attr;
   return attr.once([] {
-    MR_CUDA(cudaFuncSetAttribute(k_train_trunk<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTrunkSmem));
-    MR_CUDA(cudaFuncSetAttribute(k_train_trunk<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTrunkSmem));
+    MR_CUDA(cudaFuncSetAttribute(k_train_trunk_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, kFwdSmem));
+    MR_CUDA(cudaFuncSetAttribute(k_train_trunk_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, kBwdSmem));
     MR_CUDA(cudaFuncSetAttribute(k_train_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailSmem));
     MR_CUDA(cudaFuncSetAttribute(k_train_head, cudaFuncAttributeMaxDynamicSharedMemorySize, kHeadSmem2));
     MR_CUDA(cudaFuncSetAttribute(k_train_gates, cudaFuncAttributeMaxDynamicSharedMemorySize, kGatesSmem));
     return (int)MR_OK;
   });
 }
-static unsigned trunk_grid(int n) {
+static unsigned trunk_grid(int n, int per_sm) {
   const int tiles = (n + kR - 1) / kR;
-  return 3u * (unsigned)std::min(tiles, std::max(1, 2 * sm_count() / 3));
+  return 3u * (unsigned)std::min(tiles, std::max(1, per_sm * sm_count() / 3));
 }
 
 // Statistics, gates and the trunks' forward: wk.h0 of the rows.
@@ -1158,7 +1262,7 @@ int launch_train_trunk_fwd(const TrainArgs& a, cudaStream_t s) {
   if (rc) return rc;
   k_train_stats<<<(a.n + kR - 1) / kR, 256, (75 + 16) * kRS * 4, s>>>(a);
   MR_CUDA(cudaGetLastError());
-  k_train_trunk<false><<<trunk_grid(a.n), kTrunkThreads, kTrunkSmem, s>>>(a);
+  k_train_trunk_fwd<<<trunk_grid(a.n, 5), kTrunkThreads, kFwdSmem, s>>>(a);
   MR_CUDA(cudaGetLastError());
   return MR_OK;
 }
@@ -1176,7 +1280,7 @@ int launch_train_tail(const TrainArgs& a, cudaStream_t s) {
 }
 // The trunks and the gates backward from wk.dh0.
 int launch_train_trunk_bwd(const TrainArgs& a, cudaStream_t s) {
-  k_train_trunk<true><<<trunk_grid(a.n), kTrunkThreads, kTrunkSmem, s>>>(a);
+  k_train_trunk_bwd<<<trunk_grid(a.n, 3), kTrunkThreads, kBwdSmem, s>>>(a);
   MR_CUDA(cudaGetLastError());
   k_train_gates<<<(a.n + kR - 1) / kR, 256, kGatesSmem, s>>>(a);
   MR_CUDA(cudaGetLastError());
