@@ -128,6 +128,7 @@ struct Network {
   std::vector<float> h_se;       // per-block squeeze-excitation records of the tensor-core trunk (mr_mlp_tc.cu)
   float* simt_img = nullptr;     // weight image of the fp32 network kernels (simt_weight_image)
   std::vector<float> h_tail;     // LXW .. LX12B, kernel parameters of the fp32 head's tail (mr_mlp_simt.cu)
+  std::vector<float> h_trunk;    // kernel parameters of the fp32 trunk (mr_mlp_simt.cu)
   std::vector<float> h_light;    // kernel parameters of the fp32 light-direction trunk (mr_mlp_simt.cu)
   float h_stencil[MR_STENCIL_POINTS * 3];
 };

@@ -207,28 +207,15 @@ struct YS {
   __device__ __forceinline__ float& at(int b, int i) const { return p[(b * 32 + i) * kTile]; }
 };
 
-// yn = ReLU(B + W x) for one branch, S x S (bias stored after W): bias first,
-// then ascending inputs (LinearReLU<S> order), four outputs interleaved.
-template <int S>
-__device__ __forceinline__ void dense1(const float* x, float* yn, const float* __restrict__ W) {
+// 8 -> 8 layer, bias first then ascending inputs, weights from the parameter
+// space.
+__device__ __forceinline__ void dense8p(const float (&x)[8], float (&y)[8], const float* W) {
 #pragma unroll
-  for (int i0 = 0; i0 < S; i0 += 4) {
-    float acc[4];
+  for (int q = 0; q < 8; ++q) {
+    float acc = W[64 + q];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) acc[q] = __ldg(W + S * S + i0 + q);
-#pragma unroll
-    for (int j = 0; j < S; j += 4) {
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const float4 wv = ldg4(W + (i0 + q) * S + j);
-        acc[q] += x[j] * wv.x;
-        acc[q] += x[j + 1] * wv.y;
-        acc[q] += x[j + 2] * wv.z;
-        acc[q] += x[j + 3] * wv.w;
-      }
-    }
-#pragma unroll
-    for (int q = 0; q < 4; ++q) yn[i0 + q] = relu0(acc[q]);
+    for (int j = 0; j < 8; ++j) acc += x[j] * W[q * 8 + j];
+    y[q] = relu0(acc);
   }
 }
 
@@ -237,7 +224,7 @@ __device__ __forceinline__ void dense1(const float* x, float* yn, const float* _
 // straight into the 16 LSEFin1 sums `fin` (pool[pid+b], pool[36+pid+b]), and
 // the three branch gates.
 template <int S>
-__device__ __forceinline__ void se_gates(const RowIO& in, const float* __restrict__ sw, int from, float g,
+__device__ __forceinline__ void se_gates(const RowIO& in, const float* sw, int from, float g,
                                          float gamma, float (&fin)[16], float (&gate)[3]) {
   float st[6];  // mean b0, max b0, mean b1, max b1, mean b2, max b2
 #pragma unroll
@@ -256,39 +243,21 @@ __device__ __forceinline__ void se_gates(const RowIO& in, const float* __restric
 #pragma unroll
   for (int k = 0; k < 6; ++k)
 #pragma unroll
-    for (int j = 0; j < 16; j += 4) {
-      const float4 f = ldg4(sw + k * 16 + j);
-      fin[j] += st[k] * f.x;
-      fin[j + 1] += st[k] * f.y;
-      fin[j + 2] += st[k] * f.z;
-      fin[j + 3] += st[k] * f.w;
-    }
+    for (int j = 0; j < 16; ++j) fin[j] += st[k] * sw[k * 16 + j];
   const float tmp[8] = {st[0], st[2], st[4], st[1], st[3], st[5], g, gamma};
   float h[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     float a = 0.0f;
 #pragma unroll
-    for (int j = 0; j < 8; j += 4) {
-      const float4 q = ldg4(sw + 96 + i * 8 + j);
-      a += tmp[j] * q.x;
-      a += tmp[j + 1] * q.y;
-      a += tmp[j + 2] * q.z;
-      a += tmp[j + 3] * q.w;
-    }
+    for (int j = 0; j < 8; ++j) a += tmp[j] * sw[96 + i * 8 + j];
     h[i] = relu0(a);
   }
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
     float a = 0.0f;
 #pragma unroll
-    for (int j = 0; j < 8; j += 4) {
-      const float4 q = ldg4(sw + 160 + i * 8 + j);
-      a += h[j] * q.x;
-      a += h[j + 1] * q.y;
-      a += h[j + 2] * q.z;
-      a += h[j + 3] * q.w;
-    }
+    for (int j = 0; j < 8; ++j) a += h[j] * sw[160 + i * 8 + j];
     gate[i] = 1.0f / (1.0f + expf(-a));
   }
 }
@@ -297,15 +266,13 @@ __device__ __forceinline__ void se_gates(const RowIO& in, const float* __restric
 // REP3. Weight offsets are runtime values so that blocks of equal mode share
 // this code.
 template <int MODE>
-__device__ __forceinline__ void row_block8(const RowIO& in, const float* __restrict__ w, const float* __restrict__ sw,
-                                           int from, int wa, int wb, int wc, float g, float gamma, const YS& y,
-                                           float (&fin)[16]) {
+__device__ __forceinline__ void row_block8(const RowIO& in, const float (*W)[72], const float* sw, int from, float g,
+                                           float gamma, const YS& y, float (&fin)[16]) {
   float gate[3];
   se_gates<8>(in, sw, from, g, gamma, fin, gate);
-#pragma unroll 1
+#pragma unroll
   for (int b = 0; b < 3; ++b) {
-    const int wo = b == 0 ? wa : b == 1 ? wb : wc;
-    const float gb = b == 0 ? gate[0] : b == 1 ? gate[1] : gate[2];
+    const float gb = gate[b];
     float x[8], yn[8];
 #pragma unroll
     for (int i = 0; i < 8; i += 4) {
@@ -317,7 +284,7 @@ __device__ __forceinline__ void row_block8(const RowIO& in, const float* __restr
         x[i + u] = MODE == 0 ? v : v + y.at(b, i + u);
       }
     }
-    dense1<8>(x, yn, w + wo);
+    dense8p(x, yn, W[b]);
 #pragma unroll
     for (int i = 0; i < 8; i += 4) {
       const float4 q = in.ld4(b * 192 + from + i);
@@ -338,7 +305,7 @@ __device__ __forceinline__ void row_block8(const RowIO& in, const float* __restr
 // Per-row half of a width-S SERES block run as a block GEMM: gates, then the
 // layer input x = in * gate + y written over y in the tile.
 template <int S>
-__device__ __forceinline__ void row_gate_input(const RowIO& in, const float* __restrict__ sw, int from, float g,
+__device__ __forceinline__ void row_gate_input(const RowIO& in, const float* sw, int from, float g,
                                                float gamma, const YS& y, float (&fin)[16]) {
   float gate[3];
   se_gates<S>(in, sw, from, g, gamma, fin, gate);
@@ -465,16 +432,40 @@ __device__ __forceinline__ void desc_prefetch(const TrunkArgs& a, int row0, int 
 
 constexpr int kTrunkSmem = (96 * kTile + 2 * 3 * (32 * 32 + 32)) * (int)sizeof(float);
 
+// Weights of the trunk's per-row parts: kernel parameters, uniform
+// constant-bank operands (as loads they took 476 of a thread's L1 requests;
+// a 1080p frame's trunk 513 -> 469 us, 262,144 rows of the whole network 985
+// -> 945 us). The loop over the stages is not unrolled: with a copy of the
+// code per stage the frame took 2,183 us instead of 1,985. So is the GEMM's
+// split of 4 columns a thread: 8 x 8 pieces, 64 threads per branch and the
+// three branches at once load a third less from shared memory, but leave a
+// third of the threads idle in the per-row parts (frame 2,057 us).
+struct TrunkParams {
+  float se[8][kSeFloats];
+  float dense[2][3][72];  // blocks 0 and 1, the three branches
+  float gg[16][2];        // LSEFin1's g and gamma columns (pool[72], pool[73])
+};
+
+void trunk_param_image(const float* w, const std::vector<float>& img, std::vector<float>& out) {
+  out.assign(sizeof(TrunkParams) / sizeof(float), 0.0f);
+  std::copy(img.begin() + kSeOff, img.begin() + kSeOff + 8 * kSeFloats, out.begin());
+  const WeightTable wt = make_weight_table();
+  const int ids[6] = {MR_W_L01W, MR_W_L_Tr01W, MR_W_L_Hg01W, MR_W_L11W, MR_W_L_Tr11W, MR_W_L_Hg11W};
+  for (int d = 0; d < 6; ++d)
+    std::copy(w + wt.off[ids[d]], w + wt.off[ids[d]] + 72, out.begin() + 8 * kSeFloats + 72 * d);
+  for (int j = 0; j < 16; ++j)
+    for (int k = 0; k < 2; ++k) out[8 * kSeFloats + 6 * 72 + 2 * j + k] = w[wt.off[MR_W_LSEFin1W] + j * 75 + 72 + k];
+}
+
 // Trunks of RadiancePredict (radiancePredict.cu:385-437) for a tile of 128
 // rows, one thread per row in the per-row parts.
-__device__ __forceinline__ void trunk_tile(const TrunkArgs& a, const TrunkOut& to, float* tile, float* ring, int row0,
-                                           int n) {
+__device__ __forceinline__ void trunk_tile(const TrunkArgs& a, const TrunkOut& to, const TrunkParams& P, float* tile,
+                                           float* ring, int row0, int n) {
   trunk_stage_issue(a.img, ring, 0);
   trunk_stage_issue(a.img, ring, 1);
   desc_prefetch(a, row0, n, 0, 48);  // blocks 0..3; each stage prefetches the block two stages ahead
   const int r = threadIdx.x, row = row0 + r;
   const int kr = row < n ? row : n - 1;
-  const float* __restrict__ w = a.w;
   RowIO in{a.desc + (long long)kr * a.rs, (int)(a.cs * 4)};
   const float* ax = a.aux + (long long)kr * a.ars;
   const float g = __ldg(ax), gamma = __ldg(ax + a.afs);
@@ -483,13 +474,12 @@ __device__ __forceinline__ void trunk_tile(const TrunkArgs& a, const TrunkOut& t
   for (int j = 0; j < 16; ++j) fin[j] = 0.0f;
   const YS y{tile + r};
   // main trunk (radiancePredict.cu:396-421): blocks 0, 1 per row, 2..7 as GEMMs
-  const float* __restrict__ sw = a.img + kSeOff;  // squeeze-excitation block weights
-  row_block8<0>(in, w, sw, 0, WOFF(L01W), WOFF(L_Tr01W), WOFF(L_Hg01W), g, gamma, y, fin);
-  row_block8<2>(in, w, sw + kSeFloats, 8, WOFF(L11W), WOFF(L_Tr11W), WOFF(L_Hg11W), g, gamma, y, fin);
+  row_block8<0>(in, P.dense[0], P.se[0], 0, g, gamma, y, fin);
+  row_block8<2>(in, P.dense[1], P.se[1], 8, g, gamma, y, fin);
 #pragma unroll 1
   for (int st = 0; st < 6; ++st) {
     const int S = stage_width(st), from = st < 3 ? 16 + 16 * st : 64 + 32 * (st - 3);
-    const float* sws = sw + (2 + st) * kSeFloats;
+    const float* sws = P.se[2 + st];
     if (st < 4) desc_prefetch(a, row0, n, st == 0 ? 48 : 32 * st + 32, st == 0 ? 64 : 32 * st + 64);
     if (S == 16)
       row_gate_input<16>(in, sws, from, g, gamma, y, fin);
@@ -522,18 +512,18 @@ __device__ __forceinline__ void trunk_tile(const TrunkArgs& a, const TrunkOut& t
   // added per channel by the head
 #pragma unroll
   for (int j = 0; j < 16; ++j)
-    fin[j] += g * __ldg(w + WOFF(LSEFin1W) + j * 75 + 72) + gamma * __ldg(w + WOFF(LSEFin1W) + j * 75 + 73);
+    fin[j] += g * P.gg[j][0] + gamma * P.gg[j][1];
 #pragma unroll
   for (int j0 = 0; j0 < 16; j0 += 4) put4(30 + j0 / 4, fin[j0], fin[j0 + 1], fin[j0 + 2], fin[j0 + 3]);
 }
 
 // One tile per block (a resident grid striding over the tiles measured
 // slower: 0.948 against 0.930 ms for the network).
-__global__ void __launch_bounds__(kTile, 3) k_simt_trunk(TrunkArgs a, TrunkOut to) {
+__global__ void __launch_bounds__(kTile, 3) k_simt_trunk(TrunkArgs a, TrunkOut to, const __grid_constant__ TrunkParams P) {
   extern __shared__ __align__(16) float tsm[];
   const int n = a.count ? (int)min(*a.count, (unsigned)a.n) : a.n;
   const int row0 = blockIdx.x * kTile;
-  if (row0 < n) trunk_tile(a, to, tsm, tsm + 96 * kTile, row0, n);  // block-uniform
+  if (row0 < n) trunk_tile(a, to, P, tsm, tsm + 96 * kTile, row0, n);  // block-uniform
 }
 
 // ---- light-direction trunk --------------------------------------------------------------
@@ -560,18 +550,6 @@ void light_param_image(const float* w, const std::vector<float>& img, std::vecto
   for (int d = 0; d < 15; ++d)
     std::copy(w + wt.off[ids[d]], w + wt.off[ids[d]] + 72, out.begin() + 4 * kSeFloats + 72 * d);
   std::copy(img.begin() + kHeadRowOff, img.begin() + kHeadRowOff + 144, out.begin() + 4 * kSeFloats + 15 * 72);
-}
-
-// 8 -> 8 layer, bias first then ascending inputs (dense1's order), weights
-// from the parameter space.
-__device__ __forceinline__ void dense8p(const float (&x)[8], float (&y)[8], const float* W) {
-#pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    float acc = W[64 + q];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) acc += x[j] * W[q * 8 + j];
-    y[q] = relu0(acc);
-  }
 }
 
 template <int B>
@@ -1144,7 +1122,8 @@ int launch_mlp_simt(const Network* net, const float* desc, const float* aux, lon
                     const BatchOut* bout, float* tout, long long trs, long long tcs, float* stg, long long srs,
                     long long scs, StageTimer* timer) {
   if (!tout || !stg) return set_error(MR_ERR_ARG, "fp32 network: no buffer for the trunk or LC2 outputs");
-  if (net->h_tail.size() != (size_t)kTailFloats || net->h_light.size() * sizeof(float) != sizeof(LightParams))
+  if (net->h_tail.size() != (size_t)kTailFloats || net->h_light.size() * sizeof(float) != sizeof(LightParams) ||
+      net->h_trunk.size() * sizeof(float) != sizeof(TrunkParams))
     return set_error(MR_ERR_STATE, "network not packed");
   static DeviceCache attr;  // the attributes belong to each device's context
   int rc = attr.once([] {
@@ -1165,7 +1144,11 @@ int launch_mlp_simt(const Network* net, const float* desc, const float* aux, lon
   a.n = n;
   a.count = count;
   if (timer) timer->mark(ST_NN_TRUNK, s);
-  k_simt_trunk<<<(unsigned)((n + kTile - 1) / kTile), kTile, kTrunkSmem, s>>>(a, TrunkOut{tout, trs, tcs});
+  {
+    TrunkParams P;
+    std::memcpy(&P, net->h_trunk.data(), sizeof(P));
+    k_simt_trunk<<<(unsigned)((n + kTile - 1) / kTile), kTile, kTrunkSmem, s>>>(a, TrunkOut{tout, trs, tcs}, P);
+  }
   if (timer) timer->mark(ST_NN_TRUNK, s);
   MR_CUDA(cudaGetLastError());
   {

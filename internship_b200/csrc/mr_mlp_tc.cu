@@ -1256,6 +1256,7 @@ static uint8_t to_e4m3(float f) {
 
 void simt_weight_image(const float* w, std::vector<float>& img);  // mr_mlp_simt.cu
 void tail_param_image(const float* w, std::vector<float>& out);   // mr_mlp_simt.cu
+void trunk_param_image(const float* w, const std::vector<float>& img, std::vector<float>& out);
 void light_param_image(const float* w, const std::vector<float>& img, std::vector<float>& out);
 
 int pack_network(Network* n) {
@@ -1313,6 +1314,7 @@ int pack_network(Network* n) {
     std::vector<float> si;
     simt_weight_image(w.data(), si);
     tail_param_image(w.data(), n->h_tail);
+    trunk_param_image(w.data(), si, n->h_trunk);
     light_param_image(w.data(), si, n->h_light);
     cudaError_t e = cudaMalloc(&n->simt_img, si.size() * sizeof(float));
     if (e == cudaSuccess) e = cudaMemcpy(n->simt_img, si.data(), si.size() * sizeof(float), cudaMemcpyHostToDevice);

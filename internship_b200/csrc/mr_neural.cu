@@ -1251,7 +1251,10 @@ struct BatchJob {
   int npx;
 };
 
-__global__ void __launch_bounds__(256) k_trace_batch(const BatchJob* __restrict__ jobs, int njobs, long long w0,
+// Registers for 1,024 threads per SM (64 each; 78 without the bound, and 48 as
+// in k_nn_trace, with its spills): eight views, 1.83 M pixels, 663 us, without
+// the bound 757 and at 48 registers 728.
+__global__ void __launch_bounds__(256, 4) k_trace_batch(const BatchJob* __restrict__ jobs, int njobs, long long w0,
                                                      long long w1, const BatchOut* __restrict__ bout, Records rec,
                                                      unsigned long long* counters) {
   extern __shared__ uint32_t ring[];  // kRingWords * blockDim.x
