@@ -178,19 +178,19 @@ TRAINED = os.path.join(ROOT, "internship_b200", "data", "mrpnn_trained.npy")
 
 # DRAM bytes (read + write) per unit from one ncu capture of each kernel on the
 # 960x540 case of this frame (ncu --set full, one launch each): per active pixel
-# for the gathers and networks (the fp32 network: k_simt_trunk + k_light_trunk +
+# for the gathers and networks (the fp32 network: k_tc32_trunk + k_light_trunk +
 # k_tc32_head + k_tc32_tail),
 # per density fetch for the trace. A launch's traffic = this figure x the
 # launch's units.
-TRAFFIC_PER_UNIT = {"k_simt": 3377.8, "k_simt_trunk": 2103.4, "k_mlp_tc": 2456.3, "k_gather_fm_exact": 2463.2,
+TRAFFIC_PER_UNIT = {"k_simt": 3377.8, "k_tc32_trunk": 2103.4, "k_mlp_tc": 2456.3, "k_gather_fm_exact": 2463.2,
                     "k_gather_fm_texture": 2447.0, "k_nn_trace": 52.56}
 # k_nn_trace: dram__bytes_read + write of one launch of the 1080p bench frame
 # (759.9 MB for 14.46 M density fetches); the others at 960x540 per active pixel.
-SIMT_KERNELS = ("k_simt_trunk + k_light_trunk + k_tc32_head + k_tc32_tail (fp32 network: CUDA-core trunks, "
-                "tcgen05 head with fp32-accurate three-term TF32 products, CUDA-core tail)")
+SIMT_KERNELS = ("k_tc32_trunk + k_light_trunk + k_tc32_head + k_tc32_tail (fp32 network: tcgen05 trunk in "
+                "BF16 parts and head in three-term TF32 products, fp32-accurate; CUDA-core light trunk and tail)")
 # The library's kernels of one fp32 / exact-sampler frame, in launch order
 # (as an ncu launch list of this command shows them).
-FP32_FRAME_KERNELS = ("k_sphere_h0", "k_nn_trace", "k_gather_fm", "k_simt_trunk", "k_light_trunk", "k_tc32_head",
+FP32_FRAME_KERNELS = ("k_sphere_h0", "k_nn_trace", "k_gather_fm", "k_tc32_trunk", "k_light_trunk", "k_tc32_head",
                       "k_tc32_tail")
 # algorithmic FLOPs per active pixel of the fp32 main-trunk kernel (blocks 0..7 and L81)
 TRUNK_FLOP_PER_PIXEL = 32.9e3
@@ -740,17 +740,17 @@ def main():
     trunk_ms = head["stage"][7]
     kernels = {"k_nn_trace": dict(stages["nn_trace"], stage="nn_trace"),
                "k_gather_fm": dict(stages["nn_gather"], stage="nn_gather"),
-               "k_simt_trunk": {"bound": "fp32", "kernel": "k_simt_trunk (fp32 main trunk on the CUDA cores)",
+               "k_tc32_trunk": {"bound": "fp32", "kernel": "k_tc32_trunk (fp32 main trunk: layers on the tensor cores in BF16 parts, per-row code on the CUDA cores)",
                                 "ms": trunk_ms,
                                 "achieved": TRUNK_FLOP_PER_PIXEL * active / (trunk_ms / 1e3) / 1e12,
                                 "peak": FP32_PEAK_TFLOPS, "unit": "TFLOP/s",
                                 "peak_source": "nominal fp32 FMA rate (148 SMs x 128 lanes x 2 x 1.965 GHz)",
                                 "stage": "nn_network"}}
-    kernels["k_simt_trunk"]["frac"] = kernels["k_simt_trunk"]["achieved"] / FP32_PEAK_TFLOPS
-    kernels["k_simt_trunk"]["traffic"] = TRAFFIC_PER_UNIT["k_simt_trunk"] * active
+    kernels["k_tc32_trunk"]["frac"] = kernels["k_tc32_trunk"]["achieved"] / FP32_PEAK_TFLOPS
+    kernels["k_tc32_trunk"]["traffic"] = TRAFFIC_PER_UNIT["k_tc32_trunk"] * active
     dom = max(kernels, key=lambda k: kernels[k]["ms"])
     roofline = kernels[dom]
-    stages["nn_network"]["largest_kernel"] = {"kernel": "k_simt_trunk", "ms": trunk_ms}
+    stages["nn_network"]["largest_kernel"] = {"kernel": "k_tc32_trunk", "ms": trunk_ms}
     variants = {}
     for name, lg in legs.items():
         g_ms, m_ms = lg["stage"][2], lg["stage"][6]

@@ -6,14 +6,11 @@
 // feature-major columns (rs = 4, cs = 4*capacity) so that a warp's 32 loads
 // of one chunk are one coalesced transaction.
 //
-//  * k_simt_trunk (CUDA cores): the main trunk over a shared-memory tile,
-//    column-major (feature f of tile row r at [f*128 + r]). The
-//    squeeze-excitation statistics and gates and blocks 0 and 1 run per row
-//    (one thread per row); the width-16 and width-32 layers and L81 (89 % of
-//    the kernel's multiply-adds) run as register-tiled block GEMMs over the
-//    tile, starting at the bias and adding the inputs in ascending order as
-//    LinearReLU does, with their weights pre-transposed and double-buffered
-//    in shared memory by cp.async.
+//  * k_tc32_trunk (tensor cores): the main trunk. The squeeze-excitation
+//    statistics and gates and blocks 0 and 1 run per row (one thread per row);
+//    the width-16 and width-32 layers and L81 (89 % of the kernel's
+//    multiply-adds) as tcgen05 MMAs over operands in three BF16 parts
+//    (fp32-accurate).
 //  * k_light_trunk (CUDA cores): the light-direction trunk and LD41, one
 //    thread per row, weights as kernel parameters.
 //  * k_tc32_head (tensor cores): the head. LC0 / LC1 / LC2 (53 % of all
@@ -43,14 +40,15 @@ __device__ __forceinline__ void cp_async16(float* dst, const float* src) {
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 
 // ---- weight image of the fp32 kernels -------------------------------------------------
-// [trunk stages 0..6: blocks 2..7 of the main trunk and L81; per stage the
-//  three branches' [in][out] weights, each followed by its bias]
+// [trunk stages 0..6: blocks 2..7 of the main trunk and L81; per stage and
+//  branch the weights' three BF16 parts (split_bf16), each S x S in the
+//  canonical K-major layout (canon_off)]
 constexpr int kTrunkStages = 7;
 __host__ __device__ constexpr int stage_width(int g) { return g < 3 ? 16 : 32; }
-__host__ __device__ constexpr int stage_floats(int g) { return 3 * (stage_width(g) * stage_width(g) + stage_width(g)); }
-__host__ __device__ constexpr int stage_offset(int g) { return g <= 3 ? 816 * g : 2448 + 3168 * (g - 3); }
-static_assert(stage_offset(1) == stage_floats(0) && stage_offset(4) == stage_offset(3) + stage_floats(3),
-              "stage offsets");
+__host__ __device__ constexpr int stage_bytes(int g) { return 9 * stage_width(g) * stage_width(g) * 2; }
+__host__ __device__ constexpr int stage_offset(int g) {  // in floats
+  return g <= 3 ? stage_bytes(0) / 4 * g : 3 * (stage_bytes(0) / 4) + stage_bytes(3) / 4 * (g - 3);
+}
 // [squeeze-excitation blocks 0..11 (main trunk 0..7, light trunk 8..11): per
 //  block kSeFloats = the LSEFin1 weights of its pool entries as [6][16] (mean
 //  b0, max b0, mean b1, max b1, mean b2, max b2; 16 outputs), then SE1 8x8 and
@@ -88,29 +86,37 @@ static float tf32_rna(float x) {
 }
 static_assert(kSeOff % 4 == 0 && kSeFloats % 4 == 0 && kHeadRowOff % 4 == 0, "float4 alignment");
 
+// fp32 -> BF16 rounded to nearest even, as the upper half of an fp32, for
+// finite x (cvt.rn.bf16.f32 on the device).
+static uint32_t bf16_rn(float x) {
+  uint32_t u;
+  std::memcpy(&u, &x, 4);
+  return (u + 0x7FFFu + ((u >> 16) & 1u)) & 0xFFFF0000u;
+}
+
 void simt_weight_image(const float* w, std::vector<float>& img) {
   const WeightTable wt = make_weight_table();
   img.assign(kSimtImage, 0.0f);
-  auto put_t = [&](size_t o, int id, int N, int K) {  // W[N][K] -> [K][N] at o
-    const float* W = w + wt.off[id];
-    for (int k = 0; k < K; ++k)
-      for (int c = 0; c < N; ++c) img[o + (size_t)k * N + c] = W[(size_t)c * K + k];
-  };
-  const int ids[kTrunkStages][3][2] = {
-      {{MR_W_L21W, MR_W_L21B}, {MR_W_L_Tr21W, MR_W_L_Tr21B}, {MR_W_L_Hg21W, MR_W_L_Hg21B}},
-      {{MR_W_L31W, MR_W_L31B}, {MR_W_L_Tr31W, MR_W_L_Tr31B}, {MR_W_L_Hg31W, MR_W_L_Hg31B}},
-      {{MR_W_L41W, MR_W_L41B}, {MR_W_L_Tr41W, MR_W_L_Tr41B}, {MR_W_L_Hg41W, MR_W_L_Hg41B}},
-      {{MR_W_L51W, MR_W_L51B}, {MR_W_L_Tr51W, MR_W_L_Tr51B}, {MR_W_L_Hg51W, MR_W_L_Hg51B}},
-      {{MR_W_L61W, MR_W_L61B}, {MR_W_L_Tr61W, MR_W_L_Tr61B}, {MR_W_L_Hg61W, MR_W_L_Hg61B}},
-      {{MR_W_L71W, MR_W_L71B}, {MR_W_L_Tr71W, MR_W_L_Tr71B}, {MR_W_L_Hg71W, MR_W_L_Hg71B}},
-      {{MR_W_L81W, MR_W_L81B}, {MR_W_L_Tr81W, MR_W_L_Tr81B}, {MR_W_L_Hg81W, MR_W_L_Hg81B}}};
+  const int ids[kTrunkStages][3] = {{MR_W_L21W, MR_W_L_Tr21W, MR_W_L_Hg21W}, {MR_W_L31W, MR_W_L_Tr31W, MR_W_L_Hg31W},
+                                    {MR_W_L41W, MR_W_L_Tr41W, MR_W_L_Hg41W}, {MR_W_L51W, MR_W_L_Tr51W, MR_W_L_Hg51W},
+                                    {MR_W_L61W, MR_W_L_Tr61W, MR_W_L_Hg61W}, {MR_W_L71W, MR_W_L_Tr71W, MR_W_L_Hg71W},
+                                    {MR_W_L81W, MR_W_L_Tr81W, MR_W_L_Hg81W}};
   for (int g = 0; g < kTrunkStages; ++g) {
     const int S = stage_width(g);
-    size_t o = stage_offset(g);
     for (int b = 0; b < 3; ++b) {
-      put_t(o, ids[g][b][0], S, S);
-      for (int c = 0; c < S; ++c) img[o + S * S + c] = w[wt.off[ids[g][b][1]] + c];
-      o += S * S + S;
+      uint8_t* o = reinterpret_cast<uint8_t*>(img.data() + stage_offset(g)) + 3 * b * S * S * 2;
+      const float* W = w + wt.off[ids[g][b]];  // W[out][in]
+      for (int i = 0; i < S * S; ++i) {
+        float x = W[i];
+        for (int part = 0; part < 3; ++part) {
+          const uint32_t h = bf16_rn(x);
+          float v;
+          std::memcpy(&v, &h, 4);
+          const uint16_t e = (uint16_t)(h >> 16);
+          std::memcpy(o + part * S * S * 2 + canon_off(i / S, i % S, S), &e, 2);
+          x -= v;
+        }
+      }
     }
   }
   const int se[kSeBlocks][2] = {{MR_W_LSE01W, MR_W_LSE02W}, {MR_W_LSE11W, MR_W_LSE12W}, {MR_W_LSE21W, MR_W_LSE22W},
@@ -163,7 +169,6 @@ void simt_weight_image(const float* w, std::vector<float>& img) {
 // ---- trunk ---------------------------------------------------------------------------
 
 struct TrunkArgs {
-  const float* __restrict__ w;
   const float* __restrict__ img;  // simt_weight_image
   const float* __restrict__ desc;
   const float* __restrict__ aux;
@@ -171,6 +176,7 @@ struct TrunkArgs {
   long long ars, afs;  // aux strides
   int n;
   const unsigned* __restrict__ count;  // device row count (render path) or null
+  int* err;                            // set when a bounded wait gave up
 };
 
 // Trunk outputs per row, handed from the trunk kernels to the head kernel:
@@ -198,13 +204,6 @@ struct RowIO {
         : "r"(i >> 2), "r"(cs16), "l"(d));
     return v;
   }
-};
-
-// The running trunk state y of a row (3 branches x up to 32 values) in the
-// tile, one column per thread: conflict-free.
-struct YS {
-  float* p;  // tile base + row
-  __device__ __forceinline__ float& at(int b, int i) const { return p[(b * 32 + i) * kTile]; }
 };
 
 // 8 -> 8 layer, bias first then ascending inputs, weights from the parameter
@@ -262,156 +261,31 @@ __device__ __forceinline__ void se_gates(const RowIO& in, const float* sw, int f
   }
 }
 
-// Block of width 8, per row. MODE 0: SE + ADD3, 1: SERES + ADD3, 2: SERES +
-// REP3. Weight offsets are runtime values so that blocks of equal mode share
-// this code.
+// Block of width 8, per row, y in and out. MODE 0: SE + ADD3 (y[b][0..8)); 2:
+// SERES + REP3 (the outputs, then the block input).
 template <int MODE>
 __device__ __forceinline__ void row_block8(const RowIO& in, const float (*W)[72], const float* sw, int from, float g,
-                                           float gamma, const YS& y, float (&fin)[16]) {
+                                           float gamma, float (&y)[3][16], float (&fin)[16]) {
   float gate[3];
   se_gates<8>(in, sw, from, g, gamma, fin, gate);
 #pragma unroll
   for (int b = 0; b < 3; ++b) {
-    const float gb = gate[b];
-    float x[8], yn[8];
+    float v[8], x[8], yn[8];
 #pragma unroll
     for (int i = 0; i < 8; i += 4) {
       const float4 q = in.ld4(b * 192 + from + i);
-      const float qv[4] = {q.x, q.y, q.z, q.w};
+      v[i] = q.x; v[i + 1] = q.y; v[i + 2] = q.z; v[i + 3] = q.w;
+    }
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const float v = qv[u] * gb;
-        x[i + u] = MODE == 0 ? v : v + y.at(b, i + u);
-      }
+    for (int i = 0; i < 8; ++i) {
+      const float xv = v[i] * gate[b];
+      x[i] = MODE == 0 ? xv : xv + y[b][i];
     }
     dense8p(x, yn, W[b]);
 #pragma unroll
-    for (int i = 0; i < 8; i += 4) {
-      const float4 q = in.ld4(b * 192 + from + i);
-      const float qv[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        if (MODE == 2) {
-          y.at(b, i + u) = yn[i + u];
-          y.at(b, 8 + i + u) = qv[u];
-        } else {
-          y.at(b, i + u) = yn[i + u] + qv[u];
-        }
-      }
-    }
-  }
-}
-
-// Per-row half of a width-S SERES block run as a block GEMM: gates, then the
-// layer input x = in * gate + y written over y in the tile.
-template <int S>
-__device__ __forceinline__ void row_gate_input(const RowIO& in, const float* sw, int from, float g,
-                                               float gamma, const YS& y, float (&fin)[16]) {
-  float gate[3];
-  se_gates<S>(in, sw, from, g, gamma, fin, gate);
-#pragma unroll
-  for (int b = 0; b < 3; ++b) {
-#pragma unroll 4
-    for (int i = 0; i < S; i += 4) {
-      const float4 q = in.ld4(b * 192 + from + i);
-      const float qv[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const float v = qv[u] * gate[b];
-        y.at(b, i + u) = v + y.at(b, i + u);
-      }
-    }
-  }
-}
-
-// Trunk weight stage g into ring buffer g % 2 (one commit group per call,
-// empty past the last stage).
-__device__ __forceinline__ void trunk_stage_issue(const float* __restrict__ img, float* ring, int g) {
-  if (g < kTrunkStages) {
-    const float* src = img + stage_offset(g);
-    float* dst = ring + (g & 1) * stage_floats(kTrunkStages - 1);
-    const int pieces = stage_floats(g) / 4;
-    for (int i = threadIdx.x; i < pieces; i += kTile) cp_async16(dst + 4 * i, src + 4 * i);
-  }
-  cp_async_commit();
-}
-
-// The three branch layers of a trunk stage of width S as block GEMMs over the
-// tile: out_b = ReLU(B_b + W_b x_b), x_b = tile columns [32b, 32b+S). Thread
-// t owns 4 consecutive columns (c0) and S/4 rows in quads: for S = 32 rows
-// 4g..4g+3 and 64+4g..64+4g+3 (g = t % 16, c0 = 4 (t / 16)); for S = 16
-// rows 4g..4g+3 (g = t % 32, c0 = 4 (t / 32)). Epilogue EPI 0: y = out + in
-// (SERES + ADD3); 1: y[0..S) = out, y[S..2S) = in (SERES + REP3); 2: the
-// outputs go to comb (L81).
-template <int S, int EPI>
-__device__ __forceinline__ void trunk_gemm(float* tile, const float* W, const float* __restrict__ desc, long long rs,
-                                           long long cs, int row0, int n, int from, const TrunkOut& to) {
-  constexpr int NQ = S / 16;            // row quads per thread
-  constexpr int G = 32 / NQ;            // row groups
-  constexpr int QS = kTile / NQ;        // distance between a thread's quads
-  const int t = threadIdx.x, r0 = 4 * (t % G), c0 = 4 * (t / G);
-#pragma unroll 1
-  for (int b = 0; b < 3; ++b) {
-    const float* X = tile + b * 32 * kTile;
-    const float* Wb = W + b * (S * S + S);
-    float acc[4 * NQ][4];
-    {
-      const float4 bias = *reinterpret_cast<const float4*>(Wb + S * S + c0);
-#pragma unroll
-      for (int i = 0; i < 4 * NQ; ++i) {
-        acc[i][0] = bias.x; acc[i][1] = bias.y; acc[i][2] = bias.z; acc[i][3] = bias.w;
-      }
-    }
-#pragma unroll 8
-    for (int k = 0; k < S; ++k) {
-      const float4 wv = *reinterpret_cast<const float4*>(Wb + k * S + c0);
-      const float wa[4] = {wv.x, wv.y, wv.z, wv.w};
-#pragma unroll
-      for (int q = 0; q < NQ; ++q) {
-        const float4 xv = *reinterpret_cast<const float4*>(X + k * kTile + q * QS + r0);
-        const float xa[4] = {xv.x, xv.y, xv.z, xv.w};
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) acc[4 * q + i][j] = fmaf(xa[i], wa[j], acc[4 * q + i][j]);
-      }
-    }
-    if (EPI != 2) __syncthreads();  // every read of x_b is done before y_b overwrites it
-#pragma unroll
-    for (int q = 0; q < NQ; ++q) {
-      const int rq = q * QS + r0;  // first of the quad's 4 rows
-      float o[4][4];               // [row][column]
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) o[i][j] = relu0(acc[4 * q + i][j]);
-      if (EPI == 2) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-          if (row0 + rq + i < n)
-            *reinterpret_cast<float4*>(to.t + (long long)(row0 + rq + i) * to.rs + (8 * b + c0 / 4) * to.cs) =
-                make_float4(o[i][0], o[i][1], o[i][2], o[i][3]);
-      } else {
-        float iv[4][4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int row = row0 + rq + i, kr = row < n ? row : n - 1;
-          const float4 v = ldg4(desc + (long long)kr * rs + ((b * 192 + from + c0) >> 2) * cs);
-          iv[i][0] = v.x; iv[i][1] = v.y; iv[i][2] = v.z; iv[i][3] = v.w;
-        }
-        // one float4 of 4 rows per column: a quarter warp stores 128 contiguous bytes
-        float* yc = tile + (b * 32 + c0) * kTile + rq;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          if (EPI == 0) {
-            *reinterpret_cast<float4*>(yc + j * kTile) =
-                make_float4(o[0][j] + iv[0][j], o[1][j] + iv[1][j], o[2][j] + iv[2][j], o[3][j] + iv[3][j]);
-          } else {
-            *reinterpret_cast<float4*>(yc + j * kTile) = make_float4(o[0][j], o[1][j], o[2][j], o[3][j]);
-            *reinterpret_cast<float4*>(yc + (S + j) * kTile) = make_float4(iv[0][j], iv[1][j], iv[2][j], iv[3][j]);
-          }
-        }
-      }
+    for (int i = 0; i < 8; ++i) {
+      y[b][i] = MODE == 2 ? yn[i] : yn[i] + v[i];
+      if (MODE == 2) y[b][8 + i] = v[i];
     }
   }
 }
@@ -430,20 +304,14 @@ __device__ __forceinline__ void desc_prefetch(const TrunkArgs& a, int row0, int 
                : "memory");
 }
 
-constexpr int kTrunkSmem = (96 * kTile + 2 * 3 * (32 * 32 + 32)) * (int)sizeof(float);
-
 // Weights of the trunk's per-row parts: kernel parameters, uniform
-// constant-bank operands (as loads they took 476 of a thread's L1 requests;
-// a 1080p frame's trunk 513 -> 469 us, 262,144 rows of the whole network 985
-// -> 945 us). The loop over the stages is not unrolled: with a copy of the
-// code per stage the frame took 2,183 us instead of 1,985. So is the GEMM's
-// split of 4 columns a thread: 8 x 8 pieces, 64 threads per branch and the
-// three branches at once load a third less from shared memory, but leave a
-// third of the threads idle in the per-row parts (frame 2,057 us).
+// constant-bank operands (as loads they took 476 of a thread's L1 requests and
+// 44 us of a 1080p frame).
 struct TrunkParams {
   float se[8][kSeFloats];
   float dense[2][3][72];  // blocks 0 and 1, the three branches
   float gg[16][2];        // LSEFin1's g and gamma columns (pool[72], pool[73])
+  float bias[kTrunkStages][3][32];
 };
 
 void trunk_param_image(const float* w, const std::vector<float>& img, std::vector<float>& out) {
@@ -451,57 +319,192 @@ void trunk_param_image(const float* w, const std::vector<float>& img, std::vecto
   std::copy(img.begin() + kSeOff, img.begin() + kSeOff + 8 * kSeFloats, out.begin());
   const WeightTable wt = make_weight_table();
   const int ids[6] = {MR_W_L01W, MR_W_L_Tr01W, MR_W_L_Hg01W, MR_W_L11W, MR_W_L_Tr11W, MR_W_L_Hg11W};
-  for (int d = 0; d < 6; ++d)
-    std::copy(w + wt.off[ids[d]], w + wt.off[ids[d]] + 72, out.begin() + 8 * kSeFloats + 72 * d);
+  float* o = out.data() + 8 * kSeFloats;
+  for (int d = 0; d < 6; ++d, o += 72) std::copy(w + wt.off[ids[d]], w + wt.off[ids[d]] + 72, o);
   for (int j = 0; j < 16; ++j)
-    for (int k = 0; k < 2; ++k) out[8 * kSeFloats + 6 * 72 + 2 * j + k] = w[wt.off[MR_W_LSEFin1W] + j * 75 + 72 + k];
+    for (int k = 0; k < 2; ++k) *o++ = w[wt.off[MR_W_LSEFin1W] + j * 75 + 72 + k];
+  const int bias[kTrunkStages][3] = {
+      {MR_W_L21B, MR_W_L_Tr21B, MR_W_L_Hg21B}, {MR_W_L31B, MR_W_L_Tr31B, MR_W_L_Hg31B},
+      {MR_W_L41B, MR_W_L_Tr41B, MR_W_L_Hg41B}, {MR_W_L51B, MR_W_L_Tr51B, MR_W_L_Hg51B},
+      {MR_W_L61B, MR_W_L_Tr61B, MR_W_L_Hg61B}, {MR_W_L71B, MR_W_L_Tr71B, MR_W_L_Hg71B},
+      {MR_W_L81B, MR_W_L_Tr81B, MR_W_L_Hg81B}};
+  for (int g = 0; g < kTrunkStages; ++g)
+    for (int b = 0; b < 3; ++b, o += 32) std::copy(w + wt.off[bias[g][b]], w + wt.off[bias[g][b]] + stage_width(g), o);
+}
+
+constexpr int kTrunkA = 3 * kTile * 32 * 2;  // bytes of one branch's input: three BF16 parts
+constexpr int kTrunkSmem = kTrunkA + stage_bytes(kTrunkStages - 1) + 64;
+
+struct TrunkTile {
+  uint8_t* sm;        // a branch's input tile, the stage's weights, the mbarrier
+  uint32_t tmem, tl;  // accumulators (branch b: columns 32 b ..), this warp's lanes of them
+  uint32_t bar;       // completes once per branch and stage, with its MMAs
+  uint32_t parity;    // of the next wait
+  bool ok;
+};
+
+// Stage g's weights into shared memory (every thread its share; not waited for).
+__device__ __forceinline__ void trunk_weights(const TrunkTile& k, const float* __restrict__ img, int g) {
+  float* dst = reinterpret_cast<float*>(k.sm + kTrunkA);
+  const float* src = img + stage_offset(g);
+  for (int i = threadIdx.x; i < stage_bytes(g) / 16; i += kTile) cp_async16(dst + 4 * i, src + 4 * i);
+  cp_async_commit();
+}
+
+// 8 inputs of row r at columns k0..k0+7 as three BF16 parts into a branch's
+// tiles (S columns each).
+template <int S>
+__device__ __forceinline__ void put_split8(uint8_t* A, int r, int k0, const float* x) {
+  uint4 p[3];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    float a = x[2 * i], b = x[2 * i + 1];
+#pragma unroll
+    for (int part = 0; part < 3; ++part) {
+      const uint32_t h = pack_bf16(a, b);
+      (&p[part].x)[i] = h;
+      a -= __uint_as_float(h << 16);
+      b -= __uint_as_float(h & 0xFFFF0000u);
+    }
+  }
+#pragma unroll
+  for (int part = 0; part < 3; ++part)
+    *reinterpret_cast<uint4*>(A + part * (kTile * S * 2) + canon_off(r, k0, S)) = p[part];
+}
+
+// Branch b's layer of a stage, D = A W^T, from the input tile that the callers
+// have written: the six products of BF16 parts above 2^-24 of the result, the
+// smallest first.
+template <int S>
+__device__ __forceinline__ void trunk_mma(TrunkTile& k, int b) {
+  fence_async_smem();
+  tc_fence_before();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    tc_fence_after();
+    constexpr uint32_t id = idesc_bf16(kTile, S), sbo = (S / 8) * 128;
+    const uint32_t A = smem_u32(k.sm);
+    const uint32_t W = smem_u32(k.sm + kTrunkA) + 3 * b * (S * S * 2);
+    const int pa[6] = {2, 0, 1, 1, 0, 0}, pb[6] = {0, 2, 1, 0, 1, 0};
+#pragma unroll
+    for (int t = 0; t < 6; ++t)
+#pragma unroll
+      for (int q = 0; q < S / 16; ++q)
+        umma_bf16(k.tmem + 32 * b, sdesc(A + pa[t] * (kTile * S * 2) + 256 * q, 128, sbo),
+                  sdesc(W + pb[t] * (S * S * 2) + 256 * q, 128, sbo), id, (t | q) ? 1u : 0u);
+    umma_commit(k.bar);
+  }
+}
+
+// All threads: the MMAs issued so far are complete (bounded wait).
+__device__ __forceinline__ void trunk_wait(TrunkTile& k) {
+  if (k.ok && !mbar_wait(k.bar, k.parity)) k.ok = false;
+  k.parity ^= 1u;
+  tc_fence_after();
+}
+
+// Stage st from stage st - 1's accumulators: y = ReLU(D + bias) + the previous
+// block's input (ADD3), or those two side by side where the width doubles
+// (REP3, PS < S); the layer input is this block's input * gate + y (GATED), or
+// y (L81). PS, S: the widths of the previous stage and of this one.
+template <int PS, int S, bool GATED>
+__device__ __forceinline__ void trunk_stage(TrunkTile& k, const RowIO& in, const TrunkParams& P, int st, int pfrom,
+                                            int from, const float (&gate)[3], const float* __restrict__ img) {
+  constexpr int H = S / 16, N = 3 * H;  // pieces of 16 columns
+  const int r = threadIdx.x;
+  trunk_wait(k);
+  trunk_weights(k, img, st);
+#pragma unroll 1
+  for (int i = 0; i < N; ++i) {
+    const int b = i / H, c = 16 * (i % H);
+    float4 np[4], nc[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      if (PS == S || c == 16) np[q] = in.ld4(b * 192 + pfrom + (PS == S ? c : 0) + 4 * q);
+      if (GATED) nc[q] = in.ld4(b * 192 + from + c + 4 * q);
+    }
+    float y[16];
+    if (PS == S || c == 0) {
+      tmem_ld16(k.tl + 32 * b + c, y);
+      const float* bias = P.bias[st - 1][b] + c;
+#pragma unroll
+      for (int j = 0; j < 16; ++j) y[j] = fmaxf(y[j] + bias[j], 0.0f);
+      if (PS == S)
+#pragma unroll
+        for (int j = 0; j < 16; ++j) y[j] += (&np[j / 4].x)[j % 4];
+    } else {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) y[j] = (&np[j / 4].x)[j % 4];
+    }
+    if (GATED) {
+      const float gb = b == 0 ? gate[0] : b == 1 ? gate[1] : gate[2];
+#pragma unroll
+      for (int j = 0; j < 16; ++j) y[j] = (&nc[j / 4].x)[j % 4] * gb + y[j];
+    }
+    if (i > 0 && c == 0) trunk_wait(k);  // the previous branch's MMAs are done with the input tile
+    uint8_t* A = k.sm;
+    put_split8<S>(A, r, c, y);
+    put_split8<S>(A, r, c + 8, y + 8);
+    if (c == S - 16) {
+      if (b == 0) asm volatile("cp.async.wait_all;\n" ::: "memory");
+      trunk_mma<S>(k, b);
+    }
+  }
 }
 
 // Trunks of RadiancePredict (radiancePredict.cu:385-437) for a tile of 128
-// rows, one thread per row in the per-row parts.
-__device__ __forceinline__ void trunk_tile(const TrunkArgs& a, const TrunkOut& to, const TrunkParams& P, float* tile,
-                                           float* ring, int row0, int n) {
-  trunk_stage_issue(a.img, ring, 0);
-  trunk_stage_issue(a.img, ring, 1);
+// rows, one thread per row (its TMEM lane).
+__device__ __forceinline__ void trunk_tile(const TrunkArgs& a, const TrunkOut& to, const TrunkParams& P, TrunkTile& k,
+                                           int row0, int n) {
+  trunk_weights(k, a.img, 0);
   desc_prefetch(a, row0, n, 0, 48);  // blocks 0..3; each stage prefetches the block two stages ahead
   const int r = threadIdx.x, row = row0 + r;
   const int kr = row < n ? row : n - 1;
   RowIO in{a.desc + (long long)kr * a.rs, (int)(a.cs * 4)};
   const float* ax = a.aux + (long long)kr * a.ars;
   const float g = __ldg(ax), gamma = __ldg(ax + a.afs);
-  float fin[16];
+  float fin[16], gate[3];
 #pragma unroll
   for (int j = 0; j < 16; ++j) fin[j] = 0.0f;
-  const YS y{tile + r};
-  // main trunk (radiancePredict.cu:396-421): blocks 0, 1 per row, 2..7 as GEMMs
-  row_block8<0>(in, P.dense[0], P.se[0], 0, g, gamma, y, fin);
-  row_block8<2>(in, P.dense[1], P.se[1], 8, g, gamma, y, fin);
-#pragma unroll 1
-  for (int st = 0; st < 6; ++st) {
-    const int S = stage_width(st), from = st < 3 ? 16 + 16 * st : 64 + 32 * (st - 3);
-    const float* sws = P.se[2 + st];
-    if (st < 4) desc_prefetch(a, row0, n, st == 0 ? 48 : 32 * st + 32, st == 0 ? 64 : 32 * st + 64);
-    if (S == 16)
-      row_gate_input<16>(in, sws, from, g, gamma, y, fin);
-    else
-      row_gate_input<32>(in, sws, from, g, gamma, y, fin);
-    asm volatile("cp.async.wait_group 1;\n" ::: "memory");
-    __syncthreads();  // stage st's weights and every row's input are in the tile
-    const float* W = ring + (st & 1) * stage_floats(kTrunkStages - 1);
-    if (st < 2)
-      trunk_gemm<16, 0>(tile, W, a.desc, a.rs, a.cs, row0, n, from, to);
-    else if (st == 2)
-      trunk_gemm<16, 1>(tile, W, a.desc, a.rs, a.cs, row0, n, from, to);
-    else
-      trunk_gemm<32, 0>(tile, W, a.desc, a.rs, a.cs, row0, n, from, to);
-    trunk_stage_issue(a.img, ring, st + 2);  // ring buffer st % 2 is free: every thread passed the GEMM's barriers
-    __syncthreads();                          // y complete for the per-row part
+  // main trunk (radiancePredict.cu:396-421): blocks 0, 1 per row, 2..7 as MMAs
+  {
+    float y[3][16];
+    row_block8<0>(in, P.dense[0], P.se[0], 0, g, gamma, y, fin);
+    row_block8<2>(in, P.dense[1], P.se[1], 8, g, gamma, y, fin);
+    desc_prefetch(a, row0, n, 48, 64);
+    se_gates<16>(in, P.se[2], 16, g, gamma, fin, gate);
+#pragma unroll
+    for (int b = 0; b < 3; ++b) {
+#pragma unroll
+      for (int i = 0; i < 16; i += 4) {
+        const float4 q = in.ld4(b * 192 + 16 + i);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) y[b][i + u] = (&q.x)[u] * gate[b] + y[b][i + u];
+      }
+      if (b > 0) trunk_wait(k);
+      uint8_t* A = k.sm;
+      put_split8<16>(A, r, 0, y[b]);
+      put_split8<16>(A, r, 8, y[b] + 8);
+      if (b == 0) asm volatile("cp.async.wait_all;\n" ::: "memory");
+      trunk_mma<16>(k, b);
+    }
   }
-  // L81 -> comb[0..96)
-  asm volatile("cp.async.wait_group 1;\n" ::: "memory");
-  __syncthreads();
-  trunk_gemm<32, 2>(tile, ring + (6 & 1) * stage_floats(kTrunkStages - 1), a.desc, a.rs, a.cs, row0, n, 0, to);
-  asm volatile("cp.async.wait_all;\n" ::: "memory");
+#pragma unroll 1
+  for (int st = 1; st < 6; ++st) {
+    const int from = st < 3 ? 16 + 16 * st : 64 + 32 * (st - 3);
+    if (st < 4) desc_prefetch(a, row0, n, 32 * st + 32, 32 * st + 64);
+    if (st < 3) {
+      se_gates<16>(in, P.se[2 + st], from, g, gamma, fin, gate);
+      trunk_stage<16, 16, true>(k, in, P, st, from - 16, from, gate, a.img);
+    } else {
+      se_gates<32>(in, P.se[2 + st], from, g, gamma, fin, gate);
+      if (st == 3)
+        trunk_stage<16, 32, true>(k, in, P, st, from - 16, from, gate, a.img);
+      else
+        trunk_stage<32, 32, true>(k, in, P, st, from - 32, from, gate, a.img);
+    }
+  }
+  trunk_stage<32, 32, false>(k, in, P, 6, 128, 0, gate, a.img);
   const bool valid = row < n;
   float* orow = to.t + (long long)row * to.rs;
   auto put4 = [&](int c, float x0, float x1, float x2, float x3) {
@@ -511,24 +514,72 @@ __device__ __forceinline__ void trunk_tile(const TrunkArgs& a, const TrunkOut& t
   // LSEFin1's g and gamma columns (pool[72], pool[73]); the albedo column is
   // added per channel by the head
 #pragma unroll
-  for (int j = 0; j < 16; ++j)
-    fin[j] += g * P.gg[j][0] + gamma * P.gg[j][1];
+  for (int j = 0; j < 16; ++j) fin[j] += g * P.gg[j][0] + gamma * P.gg[j][1];
 #pragma unroll
   for (int j0 = 0; j0 < 16; j0 += 4) put4(30 + j0 / 4, fin[j0], fin[j0 + 1], fin[j0 + 2], fin[j0 + 3]);
+  // L81 -> comb[0..96)
+  trunk_wait(k);
+#pragma unroll 1
+  for (int i = 0; i < 6; ++i) {
+    float y[16];
+    tmem_ld16(k.tl + 16 * i, y);
+    const float* bias = P.bias[6][0] + 16 * i;
+#pragma unroll
+    for (int j = 0; j < 16; j += 4)
+      put4(4 * i + j / 4, relu0(y[j] + bias[j]), relu0(y[j + 1] + bias[j + 1]), relu0(y[j + 2] + bias[j + 2]),
+           relu0(y[j + 3] + bias[j + 3]));
+  }
 }
 
-// One tile per block (a resident grid striding over the tiles measured
-// slower: 0.948 against 0.930 ms for the network).
-__global__ void __launch_bounds__(kTile, 3) k_simt_trunk(TrunkArgs a, TrunkOut to, const __grid_constant__ TrunkParams P) {
-  extern __shared__ __align__(16) float tsm[];
+// A tile of 128 rows per CTA. fp32 operands are split into three BF16 parts (8
+// bits each, 24 together), so that a product is exact to 2^-26 and six MMAs
+// carry it.
+//
+// Bound by the per-row parts: gates, splitting, residuals (issue active 52 %,
+// 16.8 k instructions a row; stalls on loads, instruction fetch and barriers).
+// One input tile per CTA and four CTAs per SM, where the other CTAs' row parts
+// cover a branch's MMAs: a 1080p fp32 frame 1,875 us, with two tiles and three
+// CTAs per SM 1,898. On the CUDA cores, as register-tiled GEMMs over the tile
+// (bound by shared-memory loads), the trunk took 469 us and now takes 329; with
+// 8 x 8 register tiles it took longer (2,057 us a frame against 1,985).
+__global__ void __launch_bounds__(kTile, 4) k_tc32_trunk(TrunkArgs a, TrunkOut to, const __grid_constant__ TrunkParams P) {
+  extern __shared__ __align__(1024) uint8_t ttsm[];
   const int n = a.count ? (int)min(*a.count, (unsigned)a.n) : a.n;
   const int row0 = blockIdx.x * kTile;
-  if (row0 < n) trunk_tile(a, to, P, tsm, tsm + 96 * kTile, row0, n);  // block-uniform
+  if (row0 >= n) return;  // block-uniform
+  uint64_t* mb = reinterpret_cast<uint64_t*>(ttsm + kTrunkA + stage_bytes(kTrunkStages - 1));
+  uint32_t* holder = reinterpret_cast<uint32_t*>(mb + 1);
+  const int warp = threadIdx.x >> 5;
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(holder)),
+                 "r"(128));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  if (threadIdx.x == 0) mbar_init(smem_u32(mb), 1);
+  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  TrunkTile k;
+  k.sm = ttsm;
+  k.tmem = *holder;
+  k.tl = k.tmem + ((uint32_t)(32 * warp) << 16);
+  k.bar = smem_u32(mb);
+  k.parity = 0;
+  k.ok = true;
+  trunk_tile(a, to, P, k, row0, n);
+  if (!k.ok && a.err) atomicExch(a.err, 1);
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(k.tmem), "r"(128));
+  }
 }
 
 // ---- light-direction trunk --------------------------------------------------------------
 // Blocks 8..11 (SE + ADD3, then SERES + ADD3, width 8) and LD41
-// (radiancePredict.cu:424-437) per row, after k_simt_trunk: comb[96..120)
+// (radiancePredict.cu:424-437) per row, after k_tc32_trunk: comb[96..120)
 // into trunk-output chunks 24..29 and the blocks' LSEFin1 terms added to the
 // sums in chunks 30..33. One thread per row; the weights (squeeze-excitation
 // of the four blocks, then the fifteen 8 -> 8 layers with their biases) are
@@ -697,8 +748,14 @@ struct HeadArgs {
 // LC0 / LC1 / LC2 as M = 128 tcgen05 MMAs of kind::tf32 with FP32 accumulators
 // in TMEM: every product is the sum of three TF32 products (A_hi W_hi + A_hi
 // W_lo + A_lo W_hi, split_tf32), which carries about 22 bits of each operand,
-// the accuracy of an fp32 dot product. Activations live in two canonical
-// K-major tiles (TF32 part and fp32 remainder, 128 rows x K <= 128).
+// the accuracy of an fp32 dot product. An MMA cuts its sum off to 24 bits; in
+// one accumulator all 48 sums of a K = 128 layer lose at the size of the
+// result. In LC1 and LC2 the two remainder products therefore have an
+// accumulator of their own: the network's error against 64 bits, over 300
+// random networks, 0.73 times as large at the same time. (In LC0 as well: 0.50
+// times, but then outputs differ by up to 1.7e-5 from those with one
+// accumulator.) Activations live in two canonical K-major tiles (TF32 part and
+// fp32 remainder, 128 rows x K <= 128).
 // Persistent blocks (one per SM) walk the row tiles. Thread 0 streams the
 // split weight chunks (32 input columns each, the same 10-chunk sequence for
 // every albedo channel) into a 3-slot shared-memory ring with bulk copies two
@@ -725,12 +782,14 @@ struct TcFeed {  // thread 0's view of the weight ring
   }
 };
 
-// Thread 0: the MMAs of one head layer D[tmem] = A (128 x K) W^T (K -> N),
-// K / 32 chunks of three TF32 products (4 MMAs of K = 8 each), refilling
-// each consumed slot with the chunk three places later; then a commit on
-// `done` that completes when every MMA of the layer has.
+// Thread 0: the MMAs of one head layer D = A (128 x K) W^T (K -> N), at tmem or
+// (N < 128) the sum of that and the columns from tmem + 128: K / 32 chunks of
+// three TF32 products (4 MMAs of K = 8 each), refilling each consumed slot with
+// the chunk three places later; then a commit on `done` that completes when
+// every MMA of the layer has.
 template <int N, int K>
 __device__ __forceinline__ void tc_issue_layer(TcFeed& f, uint32_t tmem, uint32_t ahi, uint32_t alo, uint32_t done) {
+  constexpr bool sep = N < 128;  // the remainder products' own accumulator
   constexpr uint32_t id = idesc_tf32(128, N), sbo_a = (K / 4) * 128, sbo_b = (kTcKC / 4) * 128;
 #pragma unroll 1
   for (int j = 0; j < K / kTcKC; ++j) {
@@ -740,12 +799,12 @@ __device__ __forceinline__ void tc_issue_layer(TcFeed& f, uint32_t tmem, uint32_
     if (f.ok) {
       const uint32_t bh = f.ring + (uint32_t)(s * kTcStage * 4), bl = bh + N * kTcKC * 4;
 #pragma unroll
-      for (int term = 0; term < 3; ++term) {  // remainder terms first, then TF32 x TF32
+      for (int term = 0; term < 3; ++term) {  // remainder terms, then TF32 x TF32
         const uint32_t a = (term == 1 ? alo : ahi) + j * (kTcKC / 4) * 128, b = term == 0 ? bl : bh;
 #pragma unroll
         for (int k8 = 0; k8 < kTcKC / 8; ++k8)
-          umma_tf32(tmem, sdesc(a + k8 * 256, 128, sbo_a), sdesc(b + k8 * 256, 128, sbo_b), id,
-                    (j | term | k8) ? 1u : 0u);
+          umma_tf32(tmem + (sep && term < 2 ? 128 : 0), sdesc(a + k8 * 256, 128, sbo_a),
+                    sdesc(b + k8 * 256, 128, sbo_b), id, (j | (sep ? term == 1 : term) | k8) ? 1u : 0u);
       }
     }
     umma_commit(f.empty + 8 * s);
@@ -787,8 +846,17 @@ __device__ __forceinline__ void tc_epi_split(uint32_t tl, const float* __restric
   static_assert(N % 64 == 0, "pairs of 16-column loads per thread");
 #pragma unroll
   for (int q = 0; q < N / 32; q += 2) {  // two TMEM loads under one wait
-    float v[2][16];
-    tmem_ld16x2(tl + h * (N / 2) + 16 * q, tl + h * (N / 2) + 16 * (q + 1), v[0], v[1]);
+    float v[2][16], u[2][16];
+    const uint32_t t0 = tl + h * (N / 2) + 16 * q;
+    tmem_ld16x2(t0, t0 + 16, v[0], v[1]);
+    if (N < 128) {
+      tmem_ld16x2(t0 + 128, t0 + 144, u[0], u[1]);
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        v[0][i] += u[0][i];
+        v[1][i] += u[1][i];
+      }
+    }
 #pragma unroll
     for (int p = 0; p < 2; ++p) {
       const int c0 = h * (N / 2) + 16 * (q + p);
@@ -840,7 +908,7 @@ __global__ void __launch_bounds__(kHeadThreads, 1) k_tc32_head(HeadArgs a) {
   const uint32_t done = smem_u32(mb + 2 * kTcSlots);
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(holder)),
-                 "r"(128));
+                 "r"(256));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   if (threadIdx.x == 0) {
@@ -966,15 +1034,16 @@ __global__ void __launch_bounds__(kHeadThreads, 1) k_tc32_head(HeadArgs a) {
       // LC2 outputs (bias, ReLU) of this channel to the staging columns; the
       // tail runs in k_tc32_tail
       {
-        float v[16];
-        tmem_ld16(tl + 16 * half, v);
+        float v[16], u[16];
+        tmem_ld16x2(tl + 16 * half, tl + 128 + 16 * half, v, u);
         if (valid) {
           float* srow = a.stg + (long long)row * a.srs;
 #pragma unroll
           for (int i = 0; i < 16; i += 4) {
             const float4 b = ldg4(bias + 192 + 16 * half + i);
             *reinterpret_cast<float4*>(srow + (8 * ch + (16 * half + i) / 4) * a.scs) =
-                make_float4(relu0(v[i] + b.x), relu0(v[i + 1] + b.y), relu0(v[i + 2] + b.z), relu0(v[i + 3] + b.w));
+                make_float4(relu0(v[i] + u[i] + b.x), relu0(v[i + 1] + u[i + 1] + b.y),
+                            relu0(v[i + 2] + u[i + 2] + b.z), relu0(v[i + 3] + u[i + 3] + b.w));
           }
         }
       }
@@ -991,7 +1060,7 @@ __global__ void __launch_bounds__(kHeadThreads, 1) k_tc32_head(HeadArgs a) {
   __syncthreads();
   if (warp == 0) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(128));
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(256));
   }
 }
 
@@ -1128,12 +1197,11 @@ int launch_mlp_simt(const Network* net, const float* desc, const float* aux, lon
   static DeviceCache attr;  // the attributes belong to each device's context
   int rc = attr.once([] {
     MR_CUDA(cudaFuncSetAttribute(k_tc32_head, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcHeadSmem));
-    MR_CUDA(cudaFuncSetAttribute(k_simt_trunk, cudaFuncAttributeMaxDynamicSharedMemorySize, kTrunkSmem));
+    MR_CUDA(cudaFuncSetAttribute(k_tc32_trunk, cudaFuncAttributeMaxDynamicSharedMemorySize, kTrunkSmem));
     return (int)MR_OK;
   });
   if (rc) return rc;
   TrunkArgs a;
-  a.w = net->w;
   a.img = net->simt_img;
   a.desc = desc;
   a.aux = aux;
@@ -1143,11 +1211,12 @@ int launch_mlp_simt(const Network* net, const float* desc, const float* aux, lon
   a.afs = afs;
   a.n = n;
   a.count = count;
+  a.err = mlp_error_word(net);
   if (timer) timer->mark(ST_NN_TRUNK, s);
   {
     TrunkParams P;
     std::memcpy(&P, net->h_trunk.data(), sizeof(P));
-    k_simt_trunk<<<(unsigned)((n + kTile - 1) / kTile), kTile, kTrunkSmem, s>>>(a, TrunkOut{tout, trs, tcs}, P);
+    k_tc32_trunk<<<(unsigned)((n + kTile - 1) / kTile), kTile, kTrunkSmem, s>>>(a, TrunkOut{tout, trs, tcs}, P);
   }
   if (timer) timer->mark(ST_NN_TRUNK, s);
   MR_CUDA(cudaGetLastError());

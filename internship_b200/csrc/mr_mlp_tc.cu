@@ -143,10 +143,6 @@ static_assert(kSmemBytes <= 232448, "shared memory budget");
 
 __device__ __forceinline__ void group_bar(int g) { asm volatile("bar.sync %0, 128;" ::"r"(g + 1) : "memory"); }
 
-__device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
-  __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-  return *reinterpret_cast<uint32_t*>(&h);
-}
 // Row `row` of a K-major tile with KP columns from x[0..KP) (fp32 -> bf16).
 template <int KP>
 __device__ __forceinline__ void store_row(uint8_t* tile, int row, const float* x) {

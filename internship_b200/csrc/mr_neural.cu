@@ -6,7 +6,7 @@
 //     list with warp-aggregated atomics, inactive ones get the environment.
 //  2. k_gather_fm: per active record, the 192-point multi-scale descriptor
 //     gather (core/radiancePredict.cu:319-368) into feature-major columns.
-//  3. the network body: k_simt_trunk, k_light_trunk, k_tc32_head and
+//  3. the network body: k_tc32_trunk, k_light_trunk, k_tc32_head and
 //     k_tc32_tail (fp32, mr_mlp_simt.cu) or k_mlp_tc (BF16 / E4M3 tcgen05,
 //     mr_mlp_tc.cu); the last kernel also writes the pixel.
 // The gather's per-point table (k_sphere_h0) runs on a side stream beside
@@ -1139,11 +1139,11 @@ extern "C" int mr_radiance_predict(const mr_network* nh, int32_t precision, cons
   // writes its trunk and LC2 outputs over consumed chunks; the tensor-core one
   // has spill space for further heads, as rows may carry distinct albedo
   // channels. Pieces are whole waves of the network's first kernel that the
-  // pool keeps (up to 250 MiB). 262 k fp32 rows: 1.20 ms reading rows, 0.98 ms
-  // in pieces of two waves, 1.07 in pieces of one; 1000 BF16 rows: 198 us, 66
-  // with their tiles on an SM each.
+  // pool keeps (up to 210 MB; the fp32 trunk's four tiles of 128 rows per SM;
+  // one and a half waves take the same time). 1000 BF16 rows: 198 us reading
+  // rows, 66 with their tiles on an SM each.
   const size_t per_row = tc ? 576 + 120 : 576;
-  const int piece = std::min(n, sm_count() * (tc ? 512 : 2 * 3 * 128));
+  const int piece = std::min(n, sm_count() * 512);
   float* tmp = nullptr;
   cudaError_t e = pool_alloc((void**)&tmp, (size_t)piece * per_row * sizeof(float), s);
   if (e != cudaSuccess) return set_error(MR_ERR_NOMEM, "network temporary: %s", cudaGetErrorString(e));

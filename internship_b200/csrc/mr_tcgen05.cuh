@@ -120,6 +120,13 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
   for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+// a and b rounded to BF16 (nearest even), a in the lower half.
+__device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
+  uint32_t h;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(h) : "f"(b), "f"(a));
+  return h;
+}
+
 // ---- fp32-accurate products from TF32 operands --------------------------------
 // Canonical K-major no-swizzle offset of element (row, k) of a 4-byte-element
 // tile with KP columns: core matrices of 8 rows x 16 B (4 elements), adjacent
