@@ -54,6 +54,47 @@ __device__ __forceinline__ void add_grad(float* g, float v) {
 }
 
 // ---- statistics and gates ------------------------------------------------------
+// Per-row layers of the gates, four rows (4 rg ..) per thread: a weight load
+// serves four multiply-adds. (One row per thread: bound by those loads;
+// 65,536 rows, k_train_stats 93 -> 67 us, k_train_gates 115 -> 91.)
+__device__ __forceinline__ void fma4(float4& s, const float4 x, float w) {
+  s.x = fmaf(x.x, w, s.x);
+  s.y = fmaf(x.y, w, s.y);
+  s.z = fmaf(x.z, w, s.z);
+  s.w = fmaf(x.w, w, s.w);
+}
+__device__ __forceinline__ float4 relu4(const float4 s) { return make_float4(relu(s.x), relu(s.y), relu(s.z), relu(s.w)); }
+__device__ __forceinline__ float4 sigmoid4(const float4 s) {
+  return make_float4(sigmoid(s.x), sigmoid(s.y), sigmoid(s.z), sigmoid(s.w));
+}
+__device__ __forceinline__ void st4(float* p, const float4 v) { *reinterpret_cast<float4*>(p) = v; }
+
+// Squeeze-excitation inputs of block b: means, maxima, g, gamma (P: 75 pooled features).
+__device__ __forceinline__ void se_inputs(const float* P, int b, int rg, float4 (&t)[8]) {
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    t[k] = ld4(P + (3 * b + k) * kRS + 4 * rg);
+    t[3 + k] = ld4(P + (36 + 3 * b + k) * kRS + 4 * rg);
+  }
+  t[6] = ld4(P + 72 * kRS + 4 * rg);
+  t[7] = ld4(P + 73 * kRS + 4 * rg);
+}
+// Hidden unit o, before its ReLU.
+__device__ __forceinline__ float4 se_hidden(const float* __restrict__ W, const float4 (&t)[8], int o) {
+  float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+  for (int j = 0; j < 8; ++j) fma4(s, t[j], __ldg(W + j + o * 8));
+  return s;
+}
+// LSEFin1's 16 sums over the 75 features, after the ReLU, to SW: 256 threads,
+// one output and four rows each.
+__device__ __forceinline__ void fin1(const float* P, const float* __restrict__ W, float* SW) {
+  const int rg = threadIdx.x & 15, o = threadIdx.x >> 4;
+  float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll 15
+  for (int j = 0; j < 75; ++j) fma4(s, ld4(P + j * kRS + 4 * rg), __ldg(W + o * 75 + j));
+  st4(SW + o * kRS + 4 * rg, relu4(s));
+}
 
 __global__ void __launch_bounds__(256) k_train_stats(TrainArgs a) {
   extern __shared__ __align__(16) float sm[];
@@ -85,45 +126,24 @@ __global__ void __launch_bounds__(256) k_train_stats(TrainArgs a) {
     const int f = i / kR, row = i % kR;
     a.wk.pool[(size_t)f * a.wk.rows + r0 + row] = P[f * kRS + row];
   }
-  for (int i = threadIdx.x; i < 12 * kR; i += 256) {
-    const int b = i / kR, row = i % kR;
-    float t[8], h[8];
+  if (threadIdx.x < 12 * 16) {
+    const int b = threadIdx.x >> 4, rg = threadIdx.x & 15;
+    float4 t[8], h[8];
+    se_inputs(P, b, rg, t);
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      t[k] = P[(3 * b + k) * kRS + row];
-      t[3 + k] = P[(36 + 3 * b + k) * kRS + row];
-    }
-    t[6] = P[72 * kRS + row];
-    t[7] = P[73 * kRS + row];
+    for (int o = 0; o < 8; ++o) h[o] = relu4(se_hidden(W + T.se0[b], t, o));
 #pragma unroll
-    for (int o = 0; o < 8; ++o) {
-      float s = 0.0f;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) s += t[j] * __ldg(W + T.se0[b] + j + o * 8);
-      h[o] = relu(s);
-    }
-#pragma unroll
-    for (int o = 0; o < 3; ++o) {
-      float s = 0.0f;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) s += h[j] * __ldg(W + T.se1[b] + j + o * 8);
-      a.wk.gate[(size_t)(3 * b + o) * a.wk.rows + r0 + row] = sigmoid(s);
-    }
+    for (int o = 0; o < 3; ++o)
+      st4(a.wk.gate + (size_t)(3 * b + o) * a.wk.rows + r0 + 4 * rg, sigmoid4(se_hidden(W + T.se1[b], h, o)));
   }
-  for (int i = threadIdx.x; i < 16 * kR; i += 256) {
-    const int o = i / kR, row = i % kR;
-    float s = 0.0f;
-#pragma unroll 5
-    for (int j = 0; j < 75; ++j) s += P[j * kRS + row] * __ldg(W + T.f1 + o * 75 + j);
-    SW[o * kRS + row] = relu(s);
-  }
+  fin1(P, W + T.f1, SW);
   __syncthreads();
-  for (int i = threadIdx.x; i < 6 * kR; i += 256) {
-    const int o = i / kR, row = i % kR;
-    float s = 0.0f;
+  if (threadIdx.x < 6 * 16) {
+    const int o = threadIdx.x >> 4, rg = threadIdx.x & 15;
+    float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll
-    for (int j = 0; j < 16; ++j) s += SW[j * kRS + row] * __ldg(W + T.f2 + o * 16 + j);
-    a.wk.sp[(size_t)o * a.wk.rows + r0 + row] = sigmoid(s);
+    for (int j = 0; j < 16; ++j) fma4(s, ld4(SW + j * kRS + 4 * rg), __ldg(W + T.f2 + o * 16 + j));
+    st4(a.wk.sp + (size_t)o * a.wk.rows + r0 + 4 * rg, sigmoid4(s));
   }
   for (int i = threadIdx.x; i < 8 * kR; i += 256) {
     const int row = i / 8, o = i % 8;
@@ -740,6 +760,44 @@ __device__ __forceinline__ void head_dw(const HeadCtx& k, const float* D, const 
 #pragma unroll
     for (int j = 0; j < NI; ++j) add_grad(G + (og + 16 * u) * (16 * NI) + ig + 16 * j, s[u][j]);
 }
+// dW[o][i] of a 16 x 16 NI layer: two outputs and 2 NI inputs per thread over a
+// quarter of the rows (row quads k, k + 4, ... of lane k % 4), summed over the
+// four lanes. A warp's lanes hold the inputs in an order that spreads the
+// eight loads of a phase over all banks. (One weight per thread over all rows
+// takes twice the shared-memory loads: k_train_tail, 65,536 rows, 143 -> 130
+// us.)
+template <int NI>
+__device__ __forceinline__ void tail_dw(const HeadCtx& k, const float* D, const float* X, float* G) {
+  const int warp = k.t >> 5, q0 = k.t & 3, m = (k.t & 31) >> 2, ig = (m & 1) * 4 + (m >> 1);
+  float s[2][2 * NI];
+#pragma unroll
+  for (int u = 0; u < 2; ++u)
+#pragma unroll
+    for (int j = 0; j < 2 * NI; ++j) s[u][j] = 0.0f;
+#pragma unroll
+  for (int q = 4 * q0; q < kR; q += 16) {
+    const float4 d0 = ld4(D + warp * kRS + q), d1 = ld4(D + (warp + 8) * kRS + q);
+#pragma unroll
+    for (int j = 0; j < 2 * NI; ++j) {
+      const float4 x = ld4(X + (ig + 8 * j) * kRS + q);
+      s[0][j] = dot4(d0, x, s[0][j]);
+      s[1][j] = dot4(d1, x, s[1][j]);
+    }
+  }
+  // lane bit 0 keeps one output, bit 1 one half of the inputs
+  float h[2 * NI];
+#pragma unroll
+  for (int j = 0; j < 2 * NI; ++j) {
+    const float mine = q0 & 1 ? s[1][j] : s[0][j], other = q0 & 1 ? s[0][j] : s[1][j];
+    h[j] = mine + __shfl_xor_sync(0xffffffffu, other, 1);
+  }
+#pragma unroll
+  for (int j = 0; j < NI; ++j) {
+    const float mine = q0 & 2 ? h[NI + j] : h[j], other = q0 & 2 ? h[j] : h[NI + j];
+    add_grad(G + (warp + 8 * (q0 & 1)) * (16 * NI) + ig + 8 * ((q0 & 2 ? NI : 0) + j),
+             mine + __shfl_xor_sync(0xffffffffu, other, 2));
+  }
+}
 // Bias gradient of column o from the caller's rows of it.
 __device__ __forceinline__ void head_db(const HeadCtx& k, float* g, const float (&d)[4]) {
   float s = (d[0] + d[1]) + (d[2] + d[3]);
@@ -824,7 +882,7 @@ __device__ __forceinline__ void tail_tile(const HeadCtx& k, const float* A3, flo
     st4(D1 + own, e);
     head_db(k, a.grad + T.lxrb[2 * l + 1] + k.c, e);
     __syncthreads();
-    head_dw<1, 1>(k, D1, TT + 16 * l * kRS, a.grad + T.lxrw[2 * l + 1]);
+    tail_dw<1>(k, D1, TT + 16 * l * kRS, a.grad + T.lxrw[2 * l + 1]);
     col16<20>(k, D1, w + 320, k.c, e);
     const float4 tt = ld4(TT + 16 * l * kRS + own);
     e[0] = tt.x > 0.0f ? e[0] : 0.0f;
@@ -834,7 +892,7 @@ __device__ __forceinline__ void tail_tile(const HeadCtx& k, const float* A3, flo
     st4(D2 + own, e);
     head_db(k, a.grad + T.lxrb[2 * l] + k.c, e);
     __syncthreads();
-    head_dw<1, 1>(k, D2, AR + 16 * l * kRS, a.grad + T.lxrw[2 * l]);
+    tail_dw<1>(k, D2, AR + 16 * l * kRS, a.grad + T.lxrw[2 * l]);
     col16<20>(k, D2, w, k.c, e);
 #pragma unroll
     for (int r = 0; r < 4; ++r) v[r] += e[r];
@@ -849,7 +907,7 @@ __device__ __forceinline__ void tail_tile(const HeadCtx& k, const float* A3, flo
     head_db(k, a.grad + T.lxb + k.c, v);
   }
   __syncthreads();
-  head_dw<1, 2>(k, D1, A3, a.grad + T.lxw);
+  tail_dw<2>(k, D1, A3, a.grad + T.lxw);
   col16<36>(k, D1, k.tw, 2 * k.c, d[0]);
   col16<36>(k, D1, k.tw, 2 * k.c + 1, d[1]);
 #pragma unroll
@@ -1165,38 +1223,30 @@ __global__ void __launch_bounds__(256, 2) k_train_gates(const __grid_constant__ 
     for (int i = 0; i < 3; ++i) F[(72 + i) * kRS + t] = x[i];
   }
   __syncthreads();
-  for (int i = t; i < 12 * kR; i += 256) {
-    const int b = i / kR, row = i % kR;
-    float x[8], dg[3], dh[8] = {};
+  if (t < 12 * 16) {
+    const int b = t >> 4, rg = t & 15;
+    float4 x[8], dg[3];
+    se_inputs(F, b, rg, x);
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-      x[k] = F[(3 * b + k) * kRS + row];
-      x[3 + k] = F[(36 + 3 * b + k) * kRS + row];
-      const size_t at = (size_t)(3 * b + k) * N + r0 + row;
-      const float g = a.wk.gate[at];
-      dg[k] = (a.wk.dgate[at] + a.wk.dgate[36 * N + at]) * g * (1.0f - g);
-      F[(kGDG + 3 * b + k) * kRS + row] = dg[k];
+      const size_t at = (size_t)(3 * b + k) * N + r0 + 4 * rg;
+      const float4 g = ld4(a.wk.gate + at), d0 = ld4(a.wk.dgate + at), d1 = ld4(a.wk.dgate + 36 * N + at);
+      dg[k] = make_float4((d0.x + d1.x) * g.x * (1.0f - g.x), (d0.y + d1.y) * g.y * (1.0f - g.y),
+                          (d0.z + d1.z) * g.z * (1.0f - g.z), (d0.w + d1.w) * g.w * (1.0f - g.w));
+      st4(F + (kGDG + 3 * b + k) * kRS + 4 * rg, dg[k]);
     }
-    x[6] = F[72 * kRS + row];
-    x[7] = F[73 * kRS + row];
 #pragma unroll
     for (int o = 0; o < 8; ++o) {
-      float s = 0.0f;
+      const float4 s = se_hidden(W + T.se0[b], x, o);
+      float4 dh = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) s += x[j] * __ldg(W + T.se0[b] + j + o * 8);
-#pragma unroll
-      for (int j = 0; j < 3; ++j) dh[o] += __ldg(W + T.se1[b] + j * 8 + o) * dg[j];
-      F[(kGH + 8 * b + o) * kRS + row] = relu(s);
-      F[(kGDH + 8 * b + o) * kRS + row] = s > 0.0f ? dh[o] : 0.0f;
+      for (int j = 0; j < 3; ++j) fma4(dh, dg[j], __ldg(W + T.se1[b] + j * 8 + o));
+      st4(F + (kGH + 8 * b + o) * kRS + 4 * rg, relu4(s));
+      st4(F + (kGDH + 8 * b + o) * kRS + 4 * rg, s.x > 0.0f ? dh.x : 0.0f, s.y > 0.0f ? dh.y : 0.0f,
+          s.z > 0.0f ? dh.z : 0.0f, s.w > 0.0f ? dh.w : 0.0f);
     }
   }
-  for (int i = t; i < 16 * kR; i += 256) {
-    const int o = i / kR, row = i % kR;
-    float s = 0.0f;
-#pragma unroll 5
-    for (int j = 0; j < 75; ++j) s += F[j * kRS + row] * __ldg(W + T.f1 + o * 75 + j);
-    F[(kGSW + o) * kRS + row] = relu(s);
-  }
+  fin1(F, W + T.f1, F + kGSW * kRS);
   for (int i = t; i < 6 * kR; i += 256) {
     const int o = i / kR, row = i % kR;
     const size_t at = (size_t)o * N + r0 + row;
