@@ -163,9 +163,12 @@ __global__ void __launch_bounds__(256) k_train_stats(TrainArgs a) {
 //
 // The forward kernel writes every layer's input, the trunks' outputs and the
 // signs of all outputs to memory (wk.xs, wk.mask); the backward kernel copies
-// the inputs back one layer ahead. 65,536 rows: forward 226 -> 180 us and
-// backward 502 -> 287 us against keeping a tile's 232 inputs in shared memory
-// and running the forward again (two CTAs per SM; now five and three).
+// the inputs back one layer ahead. 65,536 rows: forward 226 -> 187 us and
+// backward 502 -> 278 us against keeping a tile's 232 inputs in shared memory
+// and running the forward again. A CTA has the weights once for two tiles,
+// which go their own ways: 16 warps per SM for the backward where one tile per
+// CTA allows 12 (20,011 rows: 110 us, with one tile 122). The forward gains
+// nothing from more warps (three CTAs per SM: 192 us).
 constexpr int kTrunkThreads = 128;
 __host__ __device__ constexpr int layer_width(int l) {
   return l < 2 ? 8 : l < 5 ? 16 : l < 9 ? 32 : 8;
@@ -184,8 +187,9 @@ constexpr int kLayers = 14, kTrunkW = layer_w(kLayers), kTrunkX = layer_x(kLayer
 static_assert(kTrunkX + 40 == kTrunkSaved && kLayers * kTrunkThreads * 2 == kTrunkMask, "the sizes in mr_train.cuh");
 // forward: weights, biases, two input tiles of 32 features; backward: weights,
 // two input tiles and two gradient buffers
-constexpr int kFwdSmem = (kTrunkW + kTrunkX + 64 * kRS) * 4;
-constexpr int kBwdSmem = (kTrunkW + 128 * kRS) * 4;
+constexpr int kTrunkTiles = 2;  // tiles of a CTA, 128 threads each
+constexpr int kFwdSmem = (kTrunkW + kTrunkX + kTrunkTiles * 64 * kRS) * 4;
+constexpr int kBwdSmem = (kTrunkW + kTrunkTiles * 128 * kRS) * 4;
 
 // Blob offsets of layer l of branch br.
 __device__ __forceinline__ int layer_wg(const TrainTables& T, int l, int br) {
@@ -200,13 +204,22 @@ struct TrunkCtx {
   float* xs;               // the tile's and branch's piece of wk.xs
   uint16_t* mask;          // and of wk.mask: [layer][thread], pre-activation > 0, bit 4 j + r
   const TrainArgs* a;
-  int br, r0, rg, c, t;
+  int br, r0, rg, c, t, g;  // branch, first row, row and column group, thread of the tile, tile of the CTA
 };
+
+// Barrier of a tile's threads.
+__device__ __forceinline__ void tile_sync(const TrunkCtx& k) {
+  if (k.g == 0)
+    asm volatile("bar.sync 1, %0;" ::"n"(kTrunkThreads) : "memory");
+  else
+    asm volatile("bar.sync 2, %0;" ::"n"(kTrunkThreads) : "memory");
+}
 
 __device__ __forceinline__ void trunk_ctx(TrunkCtx& k, const TrainArgs& a) {
   k.a = &a;
   k.br = blockIdx.x % 3;
-  k.t = threadIdx.x;
+  k.t = threadIdx.x % kTrunkThreads;
+  k.g = threadIdx.x / kTrunkThreads;
   const int warp = k.t >> 5, lane = k.t & 31;
   k.rg = (lane & 7) + 8 * (warp & 1);
   k.c = (lane >> 3) + 4 * (warp >> 1);
@@ -221,11 +234,11 @@ __device__ __forceinline__ void trunk_weights(const TrunkCtx& k, bool biases) {
 #pragma unroll 1
   for (int l = 0; l < kLayers; ++l) {
     const int S = layer_width(l), nc = S / 8, wg = layer_wg(c_tt, l, k.br), bg = layer_bg(c_tt, l, k.br);
-    for (int i = k.t; i < S * S; i += kTrunkThreads) {
+    for (int i = threadIdx.x; i < S * S; i += blockDim.x) {
       const int o = i / S, c = i - o * S;
       k.Ws[layer_w(l) + (o / nc + 8 * (o % nc)) * (S + 4) + c] = __ldg(k.a->w + wg + i);
     }
-    if (biases && k.t < S) k.Bs[layer_x(l) + k.t] = __ldg(k.a->w + bg + k.t);
+    if (biases && threadIdx.x < S) k.Bs[layer_x(l) + threadIdx.x] = __ldg(k.a->w + bg + threadIdx.x);
   }
 }
 
@@ -321,7 +334,7 @@ __device__ __forceinline__ void blocks_fwd(const TrunkCtx& k, int l, int count, 
     for (int j = 0; j < NC; ++j)
       put_input<NC>(k, l, x, j, fmaf(s[0][j], g.x, y[j][0]), fmaf(s[1][j], g.y, y[j][1]), fmaf(s[2][j], g.z, y[j][2]),
                     fmaf(s[3][j], g.w, y[j][3]));
-    __syncthreads();
+    tile_sync(k);
     float sn[4][NC];
     if (n + 1 < count) {  // lands during the products
       load_features<NC>(k, l + 1 - shift, sn);
@@ -352,7 +365,7 @@ __device__ __forceinline__ void blocks_fwd(const TrunkCtx& k, int l, int count, 
 // layer's: every thread overwrites the piece it read.
 template <int NC>
 __device__ __forceinline__ void take_wide(const TrunkCtx& k, int buf, float (&y)[NC][4]) {
-  __syncthreads();
+  tile_sync(k);
 #pragma unroll
   for (int j = 0; j < NC; ++j) {
     const float4 v = ld4(k.X + buf * 32 * kRS + (k.c * NC + j) * kRS + 4 * k.rg);
@@ -366,7 +379,7 @@ __device__ __forceinline__ void last_fwd(const TrunkCtx& k, int l, int& buf, flo
   buf ^= 1;
 #pragma unroll
   for (int j = 0; j < NC; ++j) put_input<NC>(k, l, x, j, y[j][0], y[j][1], y[j][2], y[j][3]);
-  __syncthreads();
+  tile_sync(k);
   tile_fwd<NC>(k, l, x, y);
 }
 
@@ -387,20 +400,21 @@ __device__ __forceinline__ void put_h0(const TrunkCtx& k, int col, int at, const
   }
 }
 
-// CTA b: branch b % 3, tiles b / 3, b / 3 + gridDim / 3, ...
-__global__ void __launch_bounds__(kTrunkThreads, 5) k_train_trunk_fwd(const __grid_constant__ TrainArgs a) {
+// CTA b: branch b % 3; its tiles g = 0 .. G - 1 at a time: b / 3 G + g, then
+// gridDim / 3 G further on.
+__global__ void __launch_bounds__(kTrunkTiles * kTrunkThreads, 2) k_train_trunk_fwd(const __grid_constant__ TrainArgs a) {
   extern __shared__ __align__(16) float sm[];
   TrunkCtx k;
   trunk_ctx(k, a);
   k.Ws = sm;
   k.Bs = k.Ws + kTrunkW;
-  k.X = k.Bs + kTrunkX;
+  k.X = k.Bs + kTrunkX + k.g * 64 * kRS;
   trunk_weights(k, true);
   __syncthreads();
   const int tiles = (a.n + kR - 1) / kR;
   const size_t N = a.wk.rows;
   int buf = 0;
-  for (int tile = blockIdx.x / 3; tile < tiles; tile += gridDim.x / 3) {
+  for (int tile = blockIdx.x / 3 * kTrunkTiles + k.g; tile < tiles; tile += gridDim.x / 3 * kTrunkTiles) {
     trunk_tile(k, tile);
     {
       float y1[1][4] = {}, y2[2][4], y4[4][4];
@@ -522,7 +536,7 @@ __device__ __forceinline__ void tile_bwd(const TrunkCtx& k, BwdState& b, int l, 
     st4(D + (k.c * NC + j) * kRS + 4 * k.rg, d[j]);
   }
   asm volatile("cp.async.wait_all;" ::: "memory");
-  __syncthreads();
+  tile_sync(k);
   fetch_step(k, b, i + 1);
   tile_dw<NC>(k, l, k.X + (i & 1) * 32 * kRS, D, d);
 #pragma unroll
@@ -593,7 +607,7 @@ __device__ __forceinline__ void narrow(const TrunkCtx& k, BwdState& b, const flo
   b.buf ^= 1;
 #pragma unroll
   for (int j = 0; j < 2 * NC; ++j) st4(D + (k.c * 2 * NC + j) * kRS + 4 * k.rg, w[j]);
-  __syncthreads();
+  tile_sync(k);
 #pragma unroll
   for (int j = 0; j < NC; ++j) {
     const float4 v = ld4(D + (k.c * NC + j) * kRS + 4 * k.rg);
@@ -632,20 +646,22 @@ __device__ __forceinline__ void take_dh0(const TrunkCtx& k, int col, int at, con
   row_sums(k, dsp, (size_t)6 * k.a->wk.rows, s);
 }
 
-__global__ void __launch_bounds__(kTrunkThreads, 3) k_train_trunk_bwd(const __grid_constant__ TrainArgs a) {
+__global__ void __launch_bounds__(kTrunkTiles * kTrunkThreads, 2) k_train_trunk_bwd(const __grid_constant__ TrainArgs a) {
   extern __shared__ __align__(16) float sm[];
   TrunkCtx k;
   trunk_ctx(k, a);
   k.Ws = sm;
   k.Bs = nullptr;
-  k.X = k.Ws + kTrunkW;
+  k.X = k.Ws + kTrunkW + k.g * 128 * kRS;
   k.D = k.X + 64 * kRS;
-  const int tiles = (a.n + kR - 1) / kR, stride = gridDim.x / 3;
+  const int tiles = (a.n + kR - 1) / kR, stride = gridDim.x / 3 * kTrunkTiles;
+  const int first = blockIdx.x / 3 * kTrunkTiles + k.g;
   const size_t N = a.wk.rows;
-  BwdState b{0, 0, (int)blockIdx.x / 3, 0};
+  BwdState b{0, 0, first, 0};
   if (b.next < tiles) fetch_step(k, b, kLayers);
-  trunk_weights(k, false);  // the first layer's barrier is behind them
-  for (int tile = blockIdx.x / 3; tile < tiles; tile += stride) {
+  trunk_weights(k, false);
+  __syncthreads();
+  for (int tile = first; tile < tiles; tile += stride) {
     trunk_tile(k, tile);
     b.step = 0;
     b.next = tile + stride < tiles ? tile + stride : -1;
@@ -1301,9 +1317,9 @@ static int tile_attrs() {
     return (int)MR_OK;
   });
 }
-static unsigned trunk_grid(int n, int per_sm) {
-  const int tiles = (n + kR - 1) / kR;
-  return 3u * (unsigned)std::min(tiles, std::max(1, per_sm * sm_count() / 3));
+static unsigned trunk_grid(int n) {  // two CTAs per SM
+  const int ctas = ((n + kR - 1) / kR + kTrunkTiles - 1) / kTrunkTiles;
+  return 3u * (unsigned)std::min(ctas, std::max(1, 2 * sm_count() / 3));
 }
 
 // Statistics, gates and the trunks' forward: wk.h0 of the rows.
@@ -1312,7 +1328,7 @@ int launch_train_trunk_fwd(const TrainArgs& a, cudaStream_t s) {
   if (rc) return rc;
   k_train_stats<<<(a.n + kR - 1) / kR, 256, (75 + 16) * kRS * 4, s>>>(a);
   MR_CUDA(cudaGetLastError());
-  k_train_trunk_fwd<<<trunk_grid(a.n, 5), kTrunkThreads, kFwdSmem, s>>>(a);
+  k_train_trunk_fwd<<<trunk_grid(a.n), kTrunkTiles * kTrunkThreads, kFwdSmem, s>>>(a);
   MR_CUDA(cudaGetLastError());
   return MR_OK;
 }
@@ -1330,7 +1346,7 @@ int launch_train_tail(const TrainArgs& a, cudaStream_t s) {
 }
 // The trunks and the gates backward from wk.dh0.
 int launch_train_trunk_bwd(const TrainArgs& a, cudaStream_t s) {
-  k_train_trunk_bwd<<<trunk_grid(a.n, 3), kTrunkThreads, kBwdSmem, s>>>(a);
+  k_train_trunk_bwd<<<trunk_grid(a.n), kTrunkTiles * kTrunkThreads, kBwdSmem, s>>>(a);
   MR_CUDA(cudaGetLastError());
   k_train_gates<<<(a.n + kR - 1) / kR, 256, kGatesSmem, s>>>(a);
   MR_CUDA(cudaGetLastError());
