@@ -178,16 +178,30 @@ __device__ __forceinline__ void add_col_sums16(float* g, const float (&v)[16]) {
   if (lane < 16 && s != 0.0f) atomicAdd(g + lane, s);
 }
 
-// The head's tensor-core halves for tiles of 128 rows, one thread per row
-// (TMEM lane). BWD false: LC0 -> LC1 -> LC2 forward as MMAs, A3 (after ReLU)
+constexpr int kHeadTcThreads = 256;
+// 16 consecutive weight gradients (16-byte aligned).
+__device__ __forceinline__ void add16(float* g, const float (&v)[16]) {
+#pragma unroll
+  for (int i = 0; i < 16; i += 4)
+    atomicAdd(reinterpret_cast<float4*>(g + i), make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]));
+}
+static_assert(make_train_tables().lc0w % 4 == 0 && make_train_tables().lc1w % 4 == 0 && make_train_tables().lc2w % 4 == 0,
+              "add16's alignment");
+// The head's tensor-core halves for tiles of 128 rows, two threads per row (TMEM
+// lane), each with half of a layer's columns. BWD false: LC0 -> LC1 -> LC2 forward as MMAs, A3 (after ReLU)
 // to wk.a3 for the tail kernel (k_train_tail). BWD true: the forward of LC0
 // and LC1 again, then from wk.da3 per layer one MMA round with the input
 // gradient (dY W, W read MN-major) and the weight gradient (dY^T X, both tiles
 // read MN-major) accumulated in tensor memory; the head-input gradient goes to
 // wk.dh0 for the trunks' backward. One kernel with the tail in between, its
 // rows' products on the same 128 threads, took 2.44 ms for 65,536 rows.
+//
+// Bound by the latency of a tile's chain of MMAs and epilogues (issue 7 %): the
+// next tile's input is loaded under it. 65,536 rows, forward 36 -> 29 us,
+// backward 103 -> 51; of the latter 42 us by the flush of the weight gradients,
+// whose lanes hold rows of 512 bytes: four values to an atomic.
 template <bool BWD>
-__global__ void __launch_bounds__(128, 1) k_train_head_tc(const __grid_constant__ TrainArgs a,
+__global__ void __launch_bounds__(kHeadTcThreads, 1) k_train_head_tc(const __grid_constant__ TrainArgs a,
                                                           const uint8_t* __restrict__ image, int* err) {
   extern __shared__ __align__(1024) uint8_t sm[];
   uint8_t* img = sm;
@@ -197,8 +211,8 @@ __global__ void __launch_bounds__(128, 1) k_train_head_tc(const __grid_constant_
   uint8_t* tWk = sm + kOffWk;
   uint64_t* mbar = reinterpret_cast<uint64_t*>(sm + kOffWk + kWkSlot);
   uint32_t* holder = reinterpret_cast<uint32_t*>(sm + kOffWk + kWkSlot + 8);
-  const int t = threadIdx.x, warp = t >> 5;
-  for (int i = t; i < kHeadImgBytes / 16; i += 128)
+  const int t = threadIdx.x, warp = t >> 5, r = t & 127, half = t >> 7;
+  for (int i = t; i < kHeadImgBytes / 16; i += kHeadTcThreads)
     reinterpret_cast<uint4*>(img)[i] = __ldg(reinterpret_cast<const uint4*>(image) + i);
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(holder)),
@@ -211,7 +225,7 @@ __global__ void __launch_bounds__(128, 1) k_train_head_tc(const __grid_constant_
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tm = *holder, lane = (uint32_t)(32 * warp) << 16;
+  const uint32_t tm = *holder, lane = (uint32_t)(32 * (warp & 3)) << 16;
   const uint32_t sW0 = smem_u32(img + kImgW0), sW1 = smem_u32(img + kImgW1), sW2 = smem_u32(img + kImgW2);
   const uint32_t sH0 = smem_u32(tH0), sA1 = smem_u32(tA1), sA2 = smem_u32(tA2), sWk = smem_u32(tWk);
   const TrainTables& T = c_tt;
@@ -234,59 +248,71 @@ __global__ void __launch_bounds__(128, 1) k_train_head_tc(const __grid_constant_
     tc_fence_after();
   };
   const int tiles = (a.n + 127) / 128;
+  // A tile's head input, loaded one tile ahead: 64 contiguous bytes of 8 rows
+  // per warp and load, 16 rows per warp.
+  const int hr = 16 * warp + ((t & 31) >> 2), hc = 4 * (t & 3);
+  float4 hv[16];
+  auto load_h0 = [&](int tile) {
+#pragma unroll
+    for (int i = 0; i < 16; ++i)
+      hv[i] = *reinterpret_cast<const float4*>(a.wk.h0 + (size_t)min(tile * 128 + hr + 8 * (i >> 3), a.n - 1) * 128 + hc +
+                                               16 * (i & 7));
+  };
+  load_h0(blockIdx.x);
   for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-    const int row = tile * 128 + t;
+    const int row = tile * 128 + r;
     const bool valid = row < a.n;
     const int k = valid ? row : a.n - 1;
     // H0 -> BF16 tile
-    {
-      const float4* src = reinterpret_cast<const float4*>(a.wk.h0 + (size_t)k * 128);
-#pragma unroll 2
-      for (int c = 0; c < 128; c += 16) {
-        float v[16];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const float4 x = src[c / 4 + q];
-          v[4 * q] = x.x; v[4 * q + 1] = x.y; v[4 * q + 2] = x.z; v[4 * q + 3] = x.w;
-        }
-        put16(tH0, t, c, 128, v);
-      }
+    for (int i = 0; i < 16; ++i)
+      *reinterpret_cast<uint2*>(tH0 + canon_off(hr + 8 * (i >> 3), hc + 16 * (i & 7), 128)) =
+          make_uint2(pack_bf16(hv[i].x, hv[i].y), pack_bf16(hv[i].z, hv[i].w));
+    if (tile + (int)gridDim.x < tiles) load_h0(tile + gridDim.x);
+    float4 d3[4];  // this thread's part of dA3
+    if constexpr (BWD) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        d3[q] = valid ? reinterpret_cast<const float4*>(a.wk.da3 + (size_t)k * 32 + 16 * half)[q]
+                      : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
     const uint32_t fw = idesc_bf16_mn(128, 128, 0, 0);
     round([&] {
       for (int s = 0; s < 8; ++s) umma_bf16(tm + kColWork, kdesc(sH0, 128, s), kdesc(sW0, 128, s), fw, s > 0);
     });
     // A1 = ReLU(LC0 H0 + b)
-    uint32_t m1[4] = {0u, 0u, 0u, 0u};
+    uint32_t m1[2] = {0u, 0u};  // signs of this thread's columns
 #pragma unroll
-    for (int h = 0; h < 8; ++h) {
+    for (int q = 0; q < 4; ++q) {
+      const int h = 4 * half + q;
       float v[16];
       tmem_ld16(tm + lane + kColWork + 16 * h, v);
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
         const float x = v[i] + __ldg(W + T.lc0b + 16 * h + i);
-        if (x > 0.0f) m1[h / 2] |= 1u << ((16 * h + i) & 31);
+        if (x > 0.0f) m1[q / 2] |= 1u << ((16 * q + i) & 31);
         v[i] = x > 0.0f ? x : 0.0f;
       }
-      put16(tA1, t, 16 * h, 128, v);
+      put16(tA1, r, 16 * h, 128, v);
     }
     round([&] {
       const uint32_t id = idesc_bf16_mn(128, 64, 0, 0);
       for (int s = 0; s < 8; ++s) umma_bf16(tm + kColWork, kdesc(sA1, 128, s), kdesc(sW1, 128, s), id, s > 0);
     });
     // A2 = ReLU(LC1 A1 + b)
-    uint32_t m2[2] = {0u, 0u};
+    uint32_t m2 = 0u;
 #pragma unroll
-    for (int h = 0; h < 4; ++h) {
+    for (int q = 0; q < 2; ++q) {
+      const int h = 2 * half + q;
       float v[16];
       tmem_ld16(tm + lane + kColWork + 16 * h, v);
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
         const float x = v[i] + __ldg(W + T.lc1b + 16 * h + i);
-        if (x > 0.0f) m2[h / 2] |= 1u << ((16 * h + i) & 31);
+        if (x > 0.0f) m2 |= 1u << (16 * q + i);
         v[i] = x > 0.0f ? x : 0.0f;
       }
-      put16(tA2, t, 16 * h, 64, v);
+      put16(tA2, r, 16 * h, 64, v);
     }
     if constexpr (!BWD) {
       round([&] {
@@ -294,8 +320,8 @@ __global__ void __launch_bounds__(128, 1) k_train_head_tc(const __grid_constant_
         for (int s = 0; s < 4; ++s) umma_bf16(tm + kColWork, kdesc(sA2, 64, s), kdesc(sW2, 64, s), id, s > 0);
       });
       // A3 = ReLU(LC2 A2 + b)
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
+      {
+        const int h = half;
         float v[16];
         tmem_ld16(tm + lane + kColWork + 16 * h, v);
 #pragma unroll
@@ -308,17 +334,16 @@ __global__ void __launch_bounds__(128, 1) k_train_head_tc(const __grid_constant_
       }
     } else {
       // dA3 -> working tile; LC2's input and weight gradients
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
+      {
+        const int h = half;
         float v[16];
-        const float4* src = reinterpret_cast<const float4*>(a.wk.da3 + (size_t)k * 32 + 16 * h);
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-          const float4 x = valid ? src[q] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+          const float4 x = d3[q];
           v[4 * q] = x.x; v[4 * q + 1] = x.y; v[4 * q + 2] = x.z; v[4 * q + 3] = x.w;
         }
         add_col_sums16(G + T.lc2b + 16 * h, v);
-        put16(tWk, t, 16 * h, 32, v);
+        put16(tWk, r, 16 * h, 32, v);
       }
       const uint32_t acc0 = first ? 0u : 1u;
       round([&] {
@@ -328,16 +353,14 @@ __global__ void __launch_bounds__(128, 1) k_train_head_tc(const __grid_constant_
       });
       // dA2 = (dA3 LC2) * [A2 > 0]
 #pragma unroll
-      for (int h = 0; h < 4; ++h) {
+      for (int q = 0; q < 2; ++q) {
+        const int h = 2 * half + q;
         float v[16];
         tmem_ld16(tm + lane + kColWork + 16 * h, v);
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          const int j = 16 * h + i;
-          v[i] = (m2[j >> 5] >> (j & 31)) & 1u ? v[i] : 0.0f;
-        }
+        for (int i = 0; i < 16; ++i) v[i] = (m2 >> (16 * q + i)) & 1u ? v[i] : 0.0f;
         add_col_sums16(G + T.lc1b + 16 * h, v);
-        put16(tWk, t, 16 * h, 64, v);
+        put16(tWk, r, 16 * h, 64, v);
       }
       round([&] {
         const uint32_t dx = idesc_bf16_mn(128, 128, 0, 1), dw = idesc_bf16_mn(128, 128, 1, 1);
@@ -346,16 +369,14 @@ __global__ void __launch_bounds__(128, 1) k_train_head_tc(const __grid_constant_
       });
       // dA1 = (dA2 LC1) * [A1 > 0]
 #pragma unroll
-      for (int h = 0; h < 8; ++h) {
+      for (int q = 0; q < 4; ++q) {
+        const int h = 4 * half + q;
         float v[16];
         tmem_ld16(tm + lane + kColWork + 16 * h, v);
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          const int j = 16 * h + i;
-          v[i] = (m1[j >> 5] >> (j & 31)) & 1u ? v[i] : 0.0f;
-        }
+        for (int i = 0; i < 16; ++i) v[i] = (m1[q / 2] >> ((16 * q + i) & 31)) & 1u ? v[i] : 0.0f;
         add_col_sums16(G + T.lc0b + 16 * h, v);
-        put16(tWk, t, 16 * h, 128, v);
+        put16(tWk, r, 16 * h, 128, v);
       }
       round([&] {
         const uint32_t dx = idesc_bf16_mn(128, 128, 0, 1), dw = idesc_bf16_mn(128, 128, 1, 1);
@@ -364,7 +385,7 @@ __global__ void __launch_bounds__(128, 1) k_train_head_tc(const __grid_constant_
       });
       // dH0 = dA1 LC0
 #pragma unroll 2
-      for (int h = 0; h < 8; ++h) {
+      for (int h = 4 * half; h < 4 * half + 4; ++h) {
         float v[16];
         tmem_ld16(tm + lane + kColWork + 16 * h, v);
         if (valid) {
@@ -379,28 +400,25 @@ __global__ void __launch_bounds__(128, 1) k_train_head_tc(const __grid_constant_
   // the CTA's weight gradients: TMEM lane = output unit
   if (BWD && !first && ok) {
 #pragma unroll 1
-    for (int h = 0; h < 8; ++h) {
+    for (int h = 4 * half; h < 4 * half + 4; ++h) {
       float v[16];
       tmem_ld16(tm + lane + kColG0 + 16 * h, v);
-#pragma unroll
-      for (int i = 0; i < 16; ++i) atomicAdd(G + T.lc0w + t * 128 + 16 * h + i, v[i]);
+      add16(G + T.lc0w + r * 128 + 16 * h, v);
     }
-    if (warp < 2) {
+    if ((warp & 3) < 2) {
 #pragma unroll 1
-      for (int h = 0; h < 8; ++h) {
+      for (int h = 4 * half; h < 4 * half + 4; ++h) {
         float v[16];
         tmem_ld16(tm + lane + kColG1 + 16 * h, v);
-#pragma unroll
-        for (int i = 0; i < 16; ++i) atomicAdd(G + T.lc1w + t * 128 + 16 * h + i, v[i]);
+        add16(G + T.lc1w + r * 128 + 16 * h, v);
       }
     }
-    if (warp == 0) {
+    if ((warp & 3) == 0) {
 #pragma unroll 1
-      for (int h = 0; h < 4; ++h) {
+      for (int h = 2 * half; h < 2 * half + 2; ++h) {
         float v[16];
         tmem_ld16(tm + lane + kColG2 + 16 * h, v);
-#pragma unroll
-        for (int i = 0; i < 16; ++i) atomicAdd(G + T.lc2w + t * 64 + 16 * h + i, v[i]);
+        add16(G + T.lc2w + r * 64 + 16 * h, v);
       }
     }
   }
@@ -430,11 +448,11 @@ int launch_head_tc(const TrainArgs& a, const uint8_t* img, int* err, cudaStream_
   });
   if (rc) return rc;
   const int grid = std::min((a.n + 127) / 128, sm_count());
-  k_train_head_tc<false><<<grid, 128, kHeadTrainSmem, s>>>(a, img, err);
+  k_train_head_tc<false><<<grid, kHeadTcThreads, kHeadTrainSmem, s>>>(a, img, err);
   MR_CUDA(cudaGetLastError());
   rc = launch_train_tail(a, s);
   if (rc) return rc;
-  k_train_head_tc<true><<<grid, 128, kHeadTrainSmem, s>>>(a, img, err);
+  k_train_head_tc<true><<<grid, kHeadTcThreads, kHeadTrainSmem, s>>>(a, img, err);
   MR_CUDA(cudaGetLastError());
   return MR_OK;
 }
