@@ -142,23 +142,39 @@ __global__ void __launch_bounds__(128) k_interactive_pt(InterArgs a) {
   mr_histogram& h = a.hist[pix];
   double* m = a.mom + pix;
   const size_t N = a.npx;
+  const F3 r = f3(L.x / (L.x + 1.0f), L.y / (L.y + 1.0f), L.z / (L.z + 1.0f));
+  float* const b0 = h.bin + (int)floorf(fminf(r.x, 0.999f) * kBins);
+  float* const b1 = h.bin + (int)floorf(fminf(r.y, 0.999f) * kBins) + kBins;
+  float* const b2 = h.bin + (int)floorf(fminf(r.z, 0.999f) * kBins) + 2 * kBins;
+  // every load before the first store, which the compiler could not move past
+  // them: 1080p 174 -> 124 us
+  float n = 0.0f, n0 = 0.0f, n1 = 0.0f, n2 = 0.0f;
+  double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0, s4 = 0.0;
   if (a.fnum == 0) {
     for (int i = 0; i < 3 * kBins; ++i) h.bin[i] = 0.0f;
-    h.total_samples = 0.0f;
-    h.x2 = 0.0f;
-    h.x = 0.0f;
-    for (int k = 0; k < 5; ++k) m[k * N] = 0.0;
+  } else {
+    n = h.total_samples;
+    n0 = *b0;
+    n1 = *b1;
+    n2 = *b2;
+    s0 = m[0];
+    s1 = m[N];
+    s2 = m[2 * N];
+    s3 = m[3 * N];
+    s4 = m[4 * N];
   }
-  const F3 r = f3(L.x / (L.x + 1.0f), L.y / (L.y + 1.0f), L.z / (L.z + 1.0f));
-  h.total_samples += 1.0f;
-  h.bin[(int)floorf(fminf(r.x, 0.999f) * kBins)] += 1.0f;
-  h.bin[(int)floorf(fminf(r.y, 0.999f) * kBins) + kBins] += 1.0f;
-  h.bin[(int)floorf(fminf(r.z, 0.999f) * kBins) + 2 * kBins] += 1.0f;
+  h.total_samples = n + 1.0f;
+  *b0 = n0 + 1.0f;
+  *b1 = n1 + 1.0f;
+  *b2 = n2 + 1.0f;
   const float l = r.x + r.y + r.z;
   // FP64 sums; the fp32 fields hold sum / n, n = fnum + 1 (the reference's
   // running means with rate 1 / (1 + fnum))
-  const double s0 = m[0] + (double)L.x, s1 = m[N] + (double)L.y, s2 = m[2 * N] + (double)L.z;
-  const double s3 = m[3 * N] + (double)l, s4 = m[4 * N] + (double)l * (double)l;
+  s0 += (double)L.x;
+  s1 += (double)L.y;
+  s2 += (double)L.z;
+  s3 += (double)l;
+  s4 += (double)l * (double)l;
   m[0] = s0;
   m[N] = s1;
   m[2 * N] = s2;
