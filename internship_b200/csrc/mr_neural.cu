@@ -21,6 +21,8 @@
 
 namespace mr {
 
+static int sampling_carveouts();
+
 struct Tables {
   const float* __restrict__ mips;
   const float* __restrict__ tr;
@@ -917,6 +919,8 @@ static int neural_passes(Volume* v, const Network* net, const mr_render_params* 
   Tables tabs;
   rc = fill_tables(v, samp, &tabs, s);
   if (rc) return rc;
+  rc = sampling_carveouts();
+  if (rc) return rc;
   // The per-point table (one block) runs on the volume's side stream beside
   // the trace, which does not read it; the gather waits for it. Where nothing
   // may be created it runs in line.
@@ -1425,8 +1429,32 @@ static size_t batch_scratch_bytes(long long wave, bool spill) {
   return neural_scratch_bytes((size_t)wave, spill) + ((size_t)wave * sizeof(int) + 255) / 256 * 256;
 }
 
+// Shared-memory share of the SM for the kernels that sample the tables and the
+// density, whose texel rate is that of their L1: nothing for the gathers, a
+// quarter for the traces (up to 40 KB of random words per SM). Without a
+// preference their blocks may start on SMs that a network kernel of another
+// stream has set to all shared memory, where little L1 is left: three batches of
+// 8 views on streams of their own took 3,510 us each against 2,510 one after the
+// other, now 2,420.
+static int sampling_carveouts() {
+  static DeviceCache set;
+  return set.once([] {
+    const auto prefer = [](const void* f, int percent) {
+      return cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, percent);
+    };
+    for (const void* f : {(const void*)k_gather_fm<kSampTex>, (const void*)k_gather_fm<kSampGather>,
+                          (const void*)k_gather_fm<kSampLoad>, (const void*)k_gather_batch<kSampTex>,
+                          (const void*)k_gather_batch<kSampGather>})
+      MR_CUDA(prefer(f, cudaSharedmemCarveoutMaxL1));
+    for (const void* f : {(const void*)k_nn_trace, (const void*)k_trace_batch}) MR_CUDA(prefer(f, 25));
+    return (int)MR_OK;
+  });
+}
+
 // Stream-ordered launches of one batch frame (eager or under capture).
 static int batch_launches(Batch& b, const Network* net, cudaStream_t s) {
+  const int crc = sampling_carveouts();
+  if (crc) return crc;
   const size_t cap = (size_t)b.wave;
   const size_t rbytes = records_round(cap);
   Records rec = carve_records(b.scratch, cap);
