@@ -428,7 +428,8 @@ int mr_train_frames(const float* dev_dir, int32_t n, mr_float3 light_dir, uint32
  * gradient buffer. The loss of a row is (X - log(1 + label / srp.x))^2, X the
  * head output of the first albedo channel (the network predicts
  * max(exp(X) - 1, 0) * srp); the step loss is its mean over the n rows.
- * dev_desc n x 576 and dev_aux n x 5 as mr_gather_descriptors writes them. */
+ * dev_desc n x 576 and dev_aux n x 5 as mr_gather_descriptors writes them, at
+ * any float address (16-byte aligned tables are read faster). */
 int mr_trainer_create(const float* host_weights, size_t count, mr_trainer** out);
 int mr_trainer_destroy(mr_trainer* t);
 /* Gradient of the mean loss (MR_WEIGHT_TOTAL floats) without updating. */

@@ -52,6 +52,22 @@ __device__ __forceinline__ float dot4(float4 a, float4 b, float acc) {
 __device__ __forceinline__ void add_grad(float* g, float v) {
   if (v != 0.0f) atomicAdd(g, v);
 }
+// NC (1, 2 or 4) consecutive descriptor features. Descriptor rows are 2304
+// bytes, so every piece is aligned to its size if the caller's table is to 16
+// bytes (WIDE); any other table is read one feature at a time.
+template <int NC, bool WIDE>
+__device__ __forceinline__ void load_desc(const float* __restrict__ p, float (&v)[NC]) {
+  if constexpr (NC == 4 && WIDE) {
+    const float4 q = __ldg(reinterpret_cast<const float4*>(p));
+    v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+  } else if constexpr (NC == 2 && WIDE) {
+    const float2 q = __ldg(reinterpret_cast<const float2*>(p));
+    v[0] = q.x; v[1] = q.y;
+  } else {
+#pragma unroll
+    for (int i = 0; i < NC; ++i) v[i] = __ldg(p + i);
+  }
+}
 
 // ---- statistics and gates ------------------------------------------------------
 // Per-row layers of the gates, four rows (4 rg ..) per thread: a weight load
@@ -96,6 +112,7 @@ __device__ __forceinline__ void fin1(const float* P, const float* __restrict__ W
   st4(SW + o * kRS + 4 * rg, relu4(s));
 }
 
+template <bool WIDE>
 __global__ void __launch_bounds__(256) k_train_stats(TrainArgs a) {
   extern __shared__ __align__(16) float sm[];
   float* P = sm;             // 75 features: mean, max, g, gamma, srp
@@ -106,13 +123,13 @@ __global__ void __launch_bounds__(256) k_train_stats(TrainArgs a) {
   // one (row, block, branch) segment of the descriptor at a time
   for (int i = threadIdx.x; i < kR * 36; i += 256) {
     const int row = i / 36, q = i - row * 36, b = q / 3, br = q - 3 * b, S = T.S[b];
-    const float4* d = reinterpret_cast<const float4*>(a.desc + (size_t)min(r0 + row, a.n - 1) * 576 + br * 192 +
-                                                      T.from[b]);
+    const float* d = a.desc + (size_t)min(r0 + row, a.n - 1) * 576 + br * 192 + T.from[b];
     float s = 0.0f, m = -10000.0f;
-    for (int k = 0; k < S / 4; ++k) {
-      const float4 v = __ldg(d + k);
-      s += v.x; s += v.y; s += v.z; s += v.w;
-      m = fmaxf(fmaxf(fmaxf(fmaxf(m, v.x), v.y), v.z), v.w);
+    for (int k = 0; k < S; k += 4) {
+      float v[4];
+      load_desc<4, WIDE>(d + k, v);
+      s += v[0]; s += v[1]; s += v[2]; s += v[3];
+      m = fmaxf(fmaxf(fmaxf(fmaxf(m, v[0]), v[1]), v[2]), v[3]);
     }
     P[q * kRS + row] = s / (float)S;
     P[(36 + q) * kRS + row] = m;
@@ -244,22 +261,12 @@ __device__ __forceinline__ void trunk_weights(const TrunkCtx& k, bool biases) {
 
 // The descriptor features of layer l (a block's) at the caller's rows and
 // columns: s[r][j].
-template <int NC>
+template <int NC, bool WIDE>
 __device__ __forceinline__ void load_features(const TrunkCtx& k, int block, float (&s)[4][NC]) {
   const int f = k.br * 192 + c_tt.from[block] + k.c * NC;
 #pragma unroll
-  for (int r = 0; r < 4; ++r) {
-    const float* p = k.a->desc + (size_t)min(k.r0 + 4 * k.rg + r, k.a->n - 1) * 576 + f;
-    if constexpr (NC == 4) {
-      const float4 v = __ldg(reinterpret_cast<const float4*>(p));
-      s[r][0] = v.x; s[r][1] = v.y; s[r][2] = v.z; s[r][3] = v.w;
-    } else if constexpr (NC == 2) {
-      const float2 v = __ldg(reinterpret_cast<const float2*>(p));
-      s[r][0] = v.x; s[r][1] = v.y;
-    } else {
-      s[r][0] = __ldg(p);
-    }
-  }
+  for (int r = 0; r < 4; ++r)
+    load_desc<NC, WIDE>(k.a->desc + (size_t)min(k.r0 + 4 * k.rg + r, k.a->n - 1) * 576 + f, s[r]);
 }
 
 // Rows 4 rg .. 4 rg + 3, outputs c NC .. c NC + NC - 1 of layer l from the
@@ -316,7 +323,7 @@ __device__ __forceinline__ void put_input(const TrunkCtx& k, int l, float* x, in
 // l - shift). y: the running output, in and out; with `rep` the last block
 // doubles the width (REP3) and leaves its output in the next input tile for
 // take_wide. buf: the input tile to use, alternating (one barrier a layer).
-template <int NC>
+template <int NC, bool WIDE>
 __device__ __forceinline__ void blocks_fwd(const TrunkCtx& k, int l, int count, int shift, bool rep, int& buf,
                                            float (&y)[NC][4]) {
   constexpr int S = 8 * NC;
@@ -324,7 +331,7 @@ __device__ __forceinline__ void blocks_fwd(const TrunkCtx& k, int l, int count, 
     return ld4(k.a->wk.gate + (size_t)(3 * (l - shift) + k.br) * k.a->wk.rows + k.r0 + 4 * k.rg);
   };
   float s[4][NC];
-  load_features<NC>(k, l - shift, s);
+  load_features<NC, WIDE>(k, l - shift, s);
   float4 g = gate(l);
 #pragma unroll 1
   for (int n = 0; n < count; ++n, ++l) {
@@ -337,7 +344,7 @@ __device__ __forceinline__ void blocks_fwd(const TrunkCtx& k, int l, int count, 
     tile_sync(k);
     float sn[4][NC];
     if (n + 1 < count) {  // lands during the products
-      load_features<NC>(k, l + 1 - shift, sn);
+      load_features<NC, WIDE>(k, l + 1 - shift, sn);
       g = gate(l + 1);
     }
     tile_fwd<NC>(k, l, x, y);
@@ -402,6 +409,7 @@ __device__ __forceinline__ void put_h0(const TrunkCtx& k, int col, int at, const
 
 // CTA b: branch b % 3; its tiles g = 0 .. G - 1 at a time: b / 3 G + g, then
 // gridDim / 3 G further on.
+template <bool WIDE>
 __global__ void __launch_bounds__(kTrunkTiles * kTrunkThreads, 2) k_train_trunk_fwd(const __grid_constant__ TrainArgs a) {
   extern __shared__ __align__(16) float sm[];
   TrunkCtx k;
@@ -418,16 +426,16 @@ __global__ void __launch_bounds__(kTrunkTiles * kTrunkThreads, 2) k_train_trunk_
     trunk_tile(k, tile);
     {
       float y1[1][4] = {}, y2[2][4], y4[4][4];
-      blocks_fwd<1>(k, 0, 2, 0, true, buf, y1);
+      blocks_fwd<1, WIDE>(k, 0, 2, 0, true, buf, y1);
       take_wide<2>(k, buf, y2);
-      blocks_fwd<2>(k, 2, 3, 0, true, buf, y2);
+      blocks_fwd<2, WIDE>(k, 2, 3, 0, true, buf, y2);
       take_wide<4>(k, buf, y4);
-      blocks_fwd<4>(k, 5, 3, 0, false, buf, y4);
+      blocks_fwd<4, WIDE>(k, 5, 3, 0, false, buf, y4);
       last_fwd<4>(k, 8, buf, y4);
       put_h0<4>(k, 32 * k.br, 0, ld4(a.wk.sp + (size_t)k.br * N + k.r0 + 4 * k.rg), y4);
     }
     float yl[1][4] = {};
-    blocks_fwd<1>(k, 9, 4, 1, false, buf, yl);
+    blocks_fwd<1, WIDE>(k, 9, 4, 1, false, buf, yl);
     last_fwd<1>(k, 13, buf, yl);
     put_h0<1>(k, 96 + 8 * k.br, 32, ld4(a.wk.sp + (size_t)(3 + k.br) * N + k.r0 + 4 * k.rg), yl);
   }
@@ -583,12 +591,12 @@ __device__ __forceinline__ void row_sums(const TrunkCtx& k, float* half0, size_t
 }
 
 // Blocks l, l - 1, ..., l - count + 1 backward; d as in tile_bwd.
-template <int NC>
+template <int NC, bool WIDE>
 __device__ __forceinline__ void blocks_bwd(const TrunkCtx& k, BwdState& b, int l, int count, int shift, float (&d)[NC][4]) {
 #pragma unroll 1
   for (int n = 0; n < count; ++n, --l) {
     float s[4][NC];
-    load_features<NC>(k, l - shift, s);  // for the gate's gradient; lands during the products
+    load_features<NC, WIDE>(k, l - shift, s);  // for the gate's gradient; lands during the products
     tile_bwd<NC>(k, b, l, d);
     float dg[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
@@ -646,6 +654,7 @@ __device__ __forceinline__ void take_dh0(const TrunkCtx& k, int col, int at, con
   row_sums(k, dsp, (size_t)6 * k.a->wk.rows, s);
 }
 
+template <bool WIDE>
 __global__ void __launch_bounds__(kTrunkTiles * kTrunkThreads, 2) k_train_trunk_bwd(const __grid_constant__ TrainArgs a) {
   extern __shared__ __align__(16) float sm[];
   TrunkCtx k;
@@ -669,17 +678,17 @@ __global__ void __launch_bounds__(kTrunkTiles * kTrunkThreads, 2) k_train_trunk_
       float d4[4][4], d2[2][4], d1[1][4];
       take_dh0<4>(k, 32 * k.br, 0, ld4(a.wk.sp + (size_t)k.br * N + k.r0 + 4 * k.rg), a.wk.dsp + (size_t)k.br * N, d4);
       tile_bwd<4>(k, b, 8, d4);
-      blocks_bwd<4>(k, b, 7, 3, 0, d4);
+      blocks_bwd<4, WIDE>(k, b, 7, 3, 0, d4);
       narrow<2>(k, b, d4, d2);
-      blocks_bwd<2>(k, b, 4, 3, 0, d2);
+      blocks_bwd<2, WIDE>(k, b, 4, 3, 0, d2);
       narrow<1>(k, b, d2, d1);
-      blocks_bwd<1>(k, b, 1, 2, 0, d1);
+      blocks_bwd<1, WIDE>(k, b, 1, 2, 0, d1);
     }
     float dl[1][4];
     take_dh0<1>(k, 96 + 8 * k.br, 32, ld4(a.wk.sp + (size_t)(3 + k.br) * N + k.r0 + 4 * k.rg),
                 a.wk.dsp + (size_t)(3 + k.br) * N, dl);
     tile_bwd<1>(k, b, 13, dl);
-    blocks_bwd<1>(k, b, 12, 4, 1, dl);
+    blocks_bwd<1, WIDE>(k, b, 12, 4, 1, dl);
   }
 }
 
@@ -1309,8 +1318,10 @@ __global__ void __launch_bounds__(256, 2) k_train_gates(const __grid_constant__ 
 static int tile_attrs() {
   static DeviceCache attr;
   return attr.once([] {
-    MR_CUDA(cudaFuncSetAttribute(k_train_trunk_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, kFwdSmem));
-    MR_CUDA(cudaFuncSetAttribute(k_train_trunk_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, kBwdSmem));
+    MR_CUDA(cudaFuncSetAttribute(k_train_trunk_fwd<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFwdSmem));
+    MR_CUDA(cudaFuncSetAttribute(k_train_trunk_fwd<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFwdSmem));
+    MR_CUDA(cudaFuncSetAttribute(k_train_trunk_bwd<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBwdSmem));
+    MR_CUDA(cudaFuncSetAttribute(k_train_trunk_bwd<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBwdSmem));
     MR_CUDA(cudaFuncSetAttribute(k_train_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailSmem));
     MR_CUDA(cudaFuncSetAttribute(k_train_head, cudaFuncAttributeMaxDynamicSharedMemorySize, kHeadSmem2));
     MR_CUDA(cudaFuncSetAttribute(k_train_gates, cudaFuncAttributeMaxDynamicSharedMemorySize, kGatesSmem));
@@ -1321,14 +1332,18 @@ static unsigned trunk_grid(int n) {  // two CTAs per SM
   const int ctas = ((n + kR - 1) / kR + kTrunkTiles - 1) / kTrunkTiles;
   return 3u * (unsigned)std::min(ctas, std::max(1, 2 * sm_count() / 3));
 }
+// The descriptors' 16-byte loads (load_desc).
+static bool wide_rows(const TrainArgs& a) { return (reinterpret_cast<uintptr_t>(a.desc) & 15) == 0; }
 
 // Statistics, gates and the trunks' forward: wk.h0 of the rows.
 int launch_train_trunk_fwd(const TrainArgs& a, cudaStream_t s) {
   int rc = tile_attrs();
   if (rc) return rc;
-  k_train_stats<<<(a.n + kR - 1) / kR, 256, (75 + 16) * kRS * 4, s>>>(a);
+  const auto stats = wide_rows(a) ? k_train_stats<true> : k_train_stats<false>;
+  stats<<<(a.n + kR - 1) / kR, 256, (75 + 16) * kRS * 4, s>>>(a);
   MR_CUDA(cudaGetLastError());
-  k_train_trunk_fwd<<<trunk_grid(a.n), kTrunkTiles * kTrunkThreads, kFwdSmem, s>>>(a);
+  const auto trunk = wide_rows(a) ? k_train_trunk_fwd<true> : k_train_trunk_fwd<false>;
+  trunk<<<trunk_grid(a.n), kTrunkTiles * kTrunkThreads, kFwdSmem, s>>>(a);
   MR_CUDA(cudaGetLastError());
   return MR_OK;
 }
@@ -1346,7 +1361,8 @@ int launch_train_tail(const TrainArgs& a, cudaStream_t s) {
 }
 // The trunks and the gates backward from wk.dh0.
 int launch_train_trunk_bwd(const TrainArgs& a, cudaStream_t s) {
-  k_train_trunk_bwd<<<trunk_grid(a.n), kTrunkTiles * kTrunkThreads, kBwdSmem, s>>>(a);
+  const auto trunk = wide_rows(a) ? k_train_trunk_bwd<true> : k_train_trunk_bwd<false>;
+  trunk<<<trunk_grid(a.n), kTrunkTiles * kTrunkThreads, kBwdSmem, s>>>(a);
   MR_CUDA(cudaGetLastError());
   k_train_gates<<<(a.n + kR - 1) / kR, 256, kGatesSmem, s>>>(a);
   MR_CUDA(cudaGetLastError());
