@@ -394,11 +394,12 @@ static int head_error(Trainer& t) {
 static int fwd_bwd(Trainer& t, const float* desc, const float* aux, const float* label, int n, cudaStream_t s) {
   MR_CUDA(cudaMemsetAsync(t.loss, 0, sizeof(float), s));
   const size_t need = (size_t)(std::min(n, kStepRows) + kTrainRows - 1) / kTrainRows * kTrainRows;
-  // Under a capture that comes before any call of this size, the buffers are
-  // nodes of the graph instead.
+  // Under a capture the buffers are nodes of the graph, also where t.work is
+  // large enough: a later call with more rows frees t.work, and a replay must
+  // not write there.
   float* temp = nullptr;
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  if (need > t.cap && s && cudaStreamIsCapturing(s, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusActive) {
+  if (s && cudaStreamIsCapturing(s, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusActive) {
     MR_CUDA(cudaMallocAsync(&temp, need * kTrainWorkFloats * sizeof(float), s));
   } else if (need > t.cap) {
     cudaFree(t.work);

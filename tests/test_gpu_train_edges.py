@@ -1,5 +1,7 @@
 """Training calls at the edges of what they accept: descriptor tables at any
-float address."""
+float address, and steps captured into a graph before the trainer grows."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -37,3 +39,51 @@ def test_descriptors_at_any_float_address(precision, shift, n):
     assert np.linalg.norm(ref) > 0
     assert np.linalg.norm(got - ref) <= 2e-5 * np.linalg.norm(ref)
     assert loss == pytest.approx(ref_loss, rel=1e-5)
+
+
+def _alloc_nodes(graph):
+    """Memory allocation nodes of a captured graph (a cudaGraph_t)."""
+    cuda = C.CDLL("libcuda.so.1")
+    n = C.c_size_t()
+    assert cuda.cuGraphGetNodes(C.c_void_p(graph), None, C.byref(n)) == 0
+    nodes = (C.c_void_p * n.value)()
+    assert cuda.cuGraphGetNodes(C.c_void_p(graph), nodes, C.byref(n)) == 0
+    kind, count = C.c_int(), 0
+    for h in nodes:
+        assert cuda.cuGraphNodeGetType(C.c_void_p(h), C.byref(kind)) == 0
+        count += kind.value == 10  # CU_GRAPH_NODE_TYPE_MEM_ALLOC
+    return count
+
+
+@pytest.mark.parametrize("precision", ["fp32", "bf16"])
+def test_captured_step_outlives_the_trainers_buffers(precision):
+    """A step captured while the trainer's buffers are large enough for it must
+    not depend on them: a later call with more rows frees them. The graph's own
+    allocation is checked before anything is replayed. One replay then updates
+    the weights as one direct step does (up to the atomics' order, which Adam's
+    first step can turn into a sign at a gradient near zero)."""
+    import torch
+    from internship_b200 import _lib
+    from internship_b200.train import Trainer
+    from internship_b200.weights import active_random_weights
+    w = active_random_weights(2)
+    d, more = _rows(200, 9), _rows(1000, 10)
+    ptr = [C.c_void_p(x.data_ptr()) for x in d]
+    a, b = Trainer(w, precision), Trainer(w, precision)
+    b.step(*d, 1e-3)
+    a.gradient(*d)  # the trainer has buffers for 200 rows
+    g = torch.cuda.CUDAGraph(keep_graph=True)
+    torch.cuda.synchronize()
+    with torch.cuda.graph(g):
+        s = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+        _lib.check(_lib.load().mr_trainer_step(a.handle, *ptr, 200, 1e-3, None, s))
+    assert _alloc_nodes(g.raw_cuda_graph()) == 1
+    a.gradient(*more)
+    g.instantiate()
+    g.replay()
+    torch.cuda.synchronize()
+    wa, wb = a.weights(), b.weights()
+    a.close()
+    b.close()
+    assert np.abs(wa - w).max() > 5e-4
+    assert (np.abs(wa - wb) > 1e-6).mean() < 0.01
