@@ -220,15 +220,17 @@ struct Trainer {
   float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
   int precision = MR_PREC_FP32;
   // The step's buffers (TrainWork) for up to `cap` rows, grown on demand to
-  // at most kStepRows: larger batches run in pieces.
+  // at most kStepRows: larger batches run in pieces, and so do batches whose
+  // buffers do not fit into the device's free memory.
   float* work = nullptr;
   size_t cap = 0;
   uint8_t* img = nullptr;  // BF16 head weights, rebuilt from w every step
   int* err = nullptr;      // set when a bounded wait of the head kernel gives up
 };
 
-// Rows of one pass of a step: 65,536 rows take 136 MB of buffers.
+// Rows of one pass of a step: 65,536 rows take 361 MB of buffers.
 constexpr int kStepRows = 65536;
+static_assert(kStepRows * kTrainWorkFloats * sizeof(float) == 360710144, "the figure above");
 
 int launch_head_pack(const float* w, uint8_t* img, cudaStream_t s);
 int launch_head_tc(const TrainArgs& a, const uint8_t* img, int* err, cudaStream_t s);
@@ -393,7 +395,8 @@ static int head_error(Trainer& t) {
 
 static int fwd_bwd(Trainer& t, const float* desc, const float* aux, const float* label, int n, cudaStream_t s) {
   MR_CUDA(cudaMemsetAsync(t.loss, 0, sizeof(float), s));
-  const size_t need = (size_t)(std::min(n, kStepRows) + kTrainRows - 1) / kTrainRows * kTrainRows;
+  const auto whole_tiles = [](size_t rows) { return (rows + kTrainRows - 1) / kTrainRows * kTrainRows; };
+  const size_t need = whole_tiles(std::min(n, kStepRows));
   // Under a capture the buffers are nodes of the graph, also where t.work is
   // large enough: a later call with more rows frees t.work, and a replay must
   // not write there.
@@ -405,9 +408,16 @@ static int fwd_bwd(Trainer& t, const float* desc, const float* aux, const float*
     cudaFree(t.work);
     t.work = nullptr;
     t.cap = 0;
-    cudaError_t e = cudaMalloc(&t.work, need * kTrainWorkFloats * sizeof(float));
-    if (e != cudaSuccess) return set_error(MR_ERR_NOMEM, "training buffers for %zu rows: %s", need, cudaGetErrorString(e));
-    t.cap = need;
+    // where the device is nearly full, buffers for fewer rows and smaller pieces
+    size_t rows = need;
+    cudaError_t e = cudaMalloc(&t.work, rows * kTrainWorkFloats * sizeof(float));
+    while (e == cudaErrorMemoryAllocation && rows > kTrainRows) {
+      rows = whole_tiles(rows / 2);
+      e = cudaMalloc(&t.work, rows * kTrainWorkFloats * sizeof(float));
+    }
+    cudaGetLastError();  // the failed attempts'
+    if (e != cudaSuccess) return set_error(MR_ERR_NOMEM, "training buffers for %zu rows: %s", rows, cudaGetErrorString(e));
+    t.cap = rows;
   }
   TrainArgs a;
   a.w = t.w;
@@ -434,8 +444,9 @@ static int fwd_bwd(Trainer& t, const float* desc, const float* aux, const float*
   a.wk.mask = reinterpret_cast<uint16_t*>(take(kTrunkMaskFloats));
   const bool tc = t.precision == MR_PREC_BF16;
   int rc = tc ? launch_head_pack(t.w, t.img, s) : (int)MR_OK;
-  for (int r0 = 0; r0 < n && !rc; r0 += kStepRows) {
-    a.n = std::min(kStepRows, n - r0);
+  const int piece = (int)std::min<size_t>(kStepRows, a.wk.rows);
+  for (int r0 = 0; r0 < n && !rc; r0 += piece) {
+    a.n = std::min(piece, n - r0);
     a.desc = desc + (size_t)r0 * 576;
     a.aux = aux + (size_t)r0 * 5;
     a.label = label + r0;
