@@ -1145,11 +1145,16 @@ extern "C" int mr_radiance_predict(const mr_network* nh, int32_t precision, cons
   // channels. Pieces are whole waves of the network's first kernel that the
   // pool keeps (up to 210 MB; the fp32 trunk's four tiles of 128 rows per SM;
   // one and a half waves take the same time). 1000 BF16 rows: 198 us reading
-  // rows, 66 with their tiles on an SM each.
+  // rows, 66 with their tiles on an SM each. Where the device is nearly full,
+  // smaller pieces.
   const size_t per_row = tc ? 576 + 120 : 576;
-  const int piece = std::min(n, sm_count() * 512);
+  int piece = std::min(n, sm_count() * 512);
   float* tmp = nullptr;
   cudaError_t e = pool_alloc((void**)&tmp, (size_t)piece * per_row * sizeof(float), s);
+  while (e == cudaErrorMemoryAllocation && piece > 128) {
+    piece = (piece / 2 + 127) / 128 * 128;
+    e = pool_alloc((void**)&tmp, (size_t)piece * per_row * sizeof(float), s);
+  }
   if (e != cudaSuccess) return set_error(MR_ERR_NOMEM, "network temporary: %s", cudaGetErrorString(e));
   int rc = MR_OK;
   for (int r0 = 0; r0 < n && rc == MR_OK; r0 += piece) {

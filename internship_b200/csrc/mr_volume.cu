@@ -575,7 +575,9 @@ static cudaMemPool_t device_pool(bool create) {
 }
 cudaError_t pool_alloc(void** p, size_t bytes, cudaStream_t s) {
   cudaMemPool_t pool = device_pool(true);
-  return pool ? cudaMallocFromPoolAsync(p, bytes, pool, s) : cudaMallocAsync(p, bytes, s);
+  const cudaError_t e = pool ? cudaMallocFromPoolAsync(p, bytes, pool, s) : cudaMallocAsync(p, bytes, s);
+  if (e == cudaErrorMemoryAllocation) cudaGetLastError();  // reported here, not by the next launch's check
+  return e;
 }
 void network_pool_trim() {
   if (cudaMemPool_t pool = device_pool(false)) cudaMemPoolTrimTo(pool, 0);

@@ -6,6 +6,8 @@ import ctypes as C
 import numpy as np
 import pytest
 
+from tests.nearly_full import nearly_full
+
 pytestmark = pytest.mark.gpu
 
 
@@ -94,7 +96,6 @@ def test_step_on_a_nearly_full_device():
     """20,011 rows, whose buffers would take 110 MB, with some 64 MB free: the
     step runs in pieces. The gradient of the whole batch, in whichever pieces,
     is a sum by atomics (tolerance as above)."""
-    import torch
     from internship_b200.train import Trainer
     from internship_b200.weights import active_random_weights
     w = active_random_weights(2)
@@ -104,19 +105,8 @@ def test_step_on_a_nearly_full_device():
     tr.close()
     tr = Trainer(w)
     tr.gradient(*[x[:64] for x in d])
-    torch.cuda.synchronize()
-    hog = []
-    try:
-        while True:  # large blocks first; the device hands out memory in pieces of 2 MB
-            free = torch.cuda.mem_get_info()[0] - (64 << 20)
-            if free < (4 << 20):
-                break
-            hog.append(torch.cuda.caching_allocator_alloc(free // (2 << 20) * (2 << 20)))
+    with nearly_full(64 << 20):
         got, loss = tr.gradient(*d)
-    finally:
-        for p in hog:
-            torch.cuda.caching_allocator_delete(p)
-        torch.cuda.empty_cache()
     tr.close()
     assert np.linalg.norm(got - ref) <= 2e-5 * np.linalg.norm(ref)
     assert loss == pytest.approx(ref_loss, rel=1e-5)
