@@ -180,7 +180,7 @@ int mr_network_destroy(mr_network* h) {
   cudaFree(h->n.w);
   cudaFree(h->n.stencil);
   free_packed(&h->n);
-  network_pool_trim();
+  pool_trim();
   delete h;
   return MR_OK;
 }

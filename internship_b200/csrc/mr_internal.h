@@ -192,11 +192,12 @@ inline F3 to_f3(const mr_float3& a) { return F3{a.x, a.y, a.z}; }
 // Stream-ordered temporary memory from a pool of the library's own on the
 // current device. Up to kPoolKeep bytes stay with the pool between calls (the
 // runtime's default pool returns everything to the device at each
-// synchronisation and maps it again on the next call); network_pool_trim gives
-// unused memory back.
+// synchronisation and maps it again on the next call); pool_trim gives the
+// unused memory of all devices back (when a volume or a network, whose calls
+// used it, is destroyed).
 constexpr size_t kPoolKeep = (size_t)256 << 20;
 cudaError_t pool_alloc(void** p, size_t bytes, cudaStream_t s);
-void network_pool_trim();
+void pool_trim();
 
 // Grows v->scratch to at least `bytes` (stream-ordered free of the old block).
 int ensure_scratch(Volume* v, size_t bytes, cudaStream_t s);

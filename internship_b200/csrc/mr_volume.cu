@@ -553,11 +553,11 @@ void destroy_textures(Volume* v) {
 // One pool per device, created on first use.
 static std::mutex g_pool_mu;
 static cudaMemPool_t g_pool[kMaxDevices];
-static cudaMemPool_t device_pool(bool create) {
+static cudaMemPool_t device_pool() {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return nullptr;
   std::lock_guard<std::mutex> lock(g_pool_mu);
-  if (!g_pool[dev] && create) {
+  if (!g_pool[dev]) {
     cudaMemPoolProps props = {};
     props.allocType = cudaMemAllocationTypePinned;
     props.location.type = cudaMemLocationTypeDevice;
@@ -574,13 +574,16 @@ static cudaMemPool_t device_pool(bool create) {
   return g_pool[dev];
 }
 cudaError_t pool_alloc(void** p, size_t bytes, cudaStream_t s) {
-  cudaMemPool_t pool = device_pool(true);
+  cudaMemPool_t pool = device_pool();
   const cudaError_t e = pool ? cudaMallocFromPoolAsync(p, bytes, pool, s) : cudaMallocAsync(p, bytes, s);
   if (e == cudaErrorMemoryAllocation) cudaGetLastError();  // reported here, not by the next launch's check
   return e;
 }
-void network_pool_trim() {
-  if (cudaMemPool_t pool = device_pool(false)) cudaMemPoolTrimTo(pool, 0);
+void pool_trim() {
+  cudaDeviceSynchronize();  // a pool gives back what the host has seen freed
+  std::lock_guard<std::mutex> lock(g_pool_mu);
+  for (cudaMemPool_t pool : g_pool)
+    if (pool) cudaMemPoolTrimTo(pool, 0);
 }
 
 int ensure_scratch(Volume* v, size_t bytes, cudaStream_t s) {
@@ -669,6 +672,7 @@ int mr_volume_destroy(mr_volume* h) {
     cudaStreamDestroy(v->side_stream);
   }
   destroy_textures(v);
+  pool_trim();
   delete h;
   return MR_OK;
 }
