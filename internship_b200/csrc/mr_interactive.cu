@@ -195,10 +195,13 @@ constexpr int kHistFloats = 3 * kBins + 3;                       // 33
 // One staged halo pixel: its histogram (bins, total, x2, x) then its colour,
 // 36 floats (144 bytes), so every record starts on a 16-byte boundary.
 constexpr int kRec = kHistFloats + 3;
-// Flag of a record's nonzero-bin mask: its channels' bins differ.
-constexpr uint32_t kColour = 1u << 31, kBinMask = (1u << (3 * kBins)) - 1u;
-// records, nonzero-bin masks, (sqrt n, 1 / sqrt n) of each record's count
-constexpr int kDenoiseSmem = kSpan * kSpan * (kRec + 3) * (int)sizeof(float);
+// Flag beside the nonzero-bin masks of a group of records: some record's
+// channels differ in their bins.
+constexpr uint32_t kColour = 1u << 31;
+// records, nonzero-bin masks, (sqrt n, 1 / sqrt n) of each record's count; the
+// masks of 32 records or-ed together
+constexpr int kGroups = (kSpan * kSpan + 31) / 32;
+constexpr int kDenoiseSmem = (kSpan * kSpan * (kRec + 3) + kGroups) * (int)sizeof(float);
 
 __device__ __forceinline__ void cp_async4(float* dst, const float* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
@@ -283,7 +286,9 @@ __device__ __forceinline__ float compare(const float (&cb)[3 * kBins], float2 cs
 // under white light and one albedo; a warp takes this form when everything
 // around its pixels is. 1080p, filter on every pixel: 2.20 ms in compare()
 // (bound by its 30 reciprocals a neighbour), 1.16 ms here with all ten bins in
-// use; 0.80 -> 0.58 ms on eight frames of a cloud.
+// use; 0.80 -> 0.58 ms on eight frames of a cloud. The choice costs coloured
+// histograms 0.6 % (2,209 -> 2,224 us; 2,237 with the general form first in
+// the code and a flag in each record's mask to clear at every use).
 template <int G>
 __device__ __forceinline__ float compare_gray(const float (&cb)[3 * kBins], float2 cs, uint32_t cm, const float* nr,
                                               float2 ns, uint32_t nm) {
@@ -330,6 +335,7 @@ __global__ void __launch_bounds__(256, 2) k_denoise(DenoiseArgs a) {
   float* rec = sm;                                                           // kSpan^2 records
   uint32_t* msk = reinterpret_cast<uint32_t*>(sm + kSpan * kSpan * kRec);  // nonzero bins of each record
   float2* rsq = reinterpret_cast<float2*>(sm + kSpan * kSpan * (kRec + 1));  // (sqrt n, 1 / sqrt n) per record
+  uint32_t* grp = reinterpret_cast<uint32_t*>(sm + kSpan * kSpan * (kRec + 3));  // masks of 32 records, kColour
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
   const int c0 = blockIdx.x * kTile - kHalo, r0 = blockIdx.y * kTile - kHalo;
   const bool filter = a.denoise && a.frame != 0;
@@ -350,31 +356,37 @@ __global__ void __launch_bounds__(256, 2) k_denoise(DenoiseArgs a) {
   asm volatile("cp.async.wait_all;\n" ::: "memory");
   __syncthreads();
   if (filter) {
-    for (int q = threadIdx.x; q < kSpan * kSpan; q += blockDim.x) {
-      const float4* r = reinterpret_cast<const float4*>(rec + q * kRec);
-      float e[32];
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        const float4 v = r[k];
-        e[4 * k] = v.x; e[4 * k + 1] = v.y; e[4 * k + 2] = v.z; e[4 * k + 3] = v.w;
-      }
+    for (int g = threadIdx.x >> 5; g < kGroups; g += 8) {
+      const int q = 32 * g + (threadIdx.x & 31);
       uint32_t m = 0;
       bool same = true;  // the three channels' bins
+      if (q < kSpan * kSpan) {
+        const float4* r = reinterpret_cast<const float4*>(rec + q * kRec);
+        float e[32];
 #pragma unroll
-      for (int k = 0; k < 3 * kBins; ++k) m |= (e[k] != 0.0f ? 1u : 0u) << k;
+        for (int k = 0; k < 8; ++k) {
+          const float4 v = r[k];
+          e[4 * k] = v.x; e[4 * k + 1] = v.y; e[4 * k + 2] = v.z; e[4 * k + 3] = v.w;
+        }
 #pragma unroll
-      for (int k = 0; k < kBins; ++k) same = same && e[k] == e[k + kBins] && e[k] == e[k + 2 * kBins];
-      msk[q] = m | (same ? 0u : kColour);
-      const float rn = sqrtf(rec[q * kRec + 3 * kBins]);
-      rsq[q] = make_float2(rn, 1.0f / rn);
+        for (int k = 0; k < 3 * kBins; ++k) m |= (e[k] != 0.0f ? 1u : 0u) << k;
+#pragma unroll
+        for (int k = 0; k < kBins; ++k) same = same && e[k] == e[k + kBins] && e[k] == e[k + 2 * kBins];
+        msk[q] = m;
+        const float rn = sqrtf(rec[q * kRec + 3 * kBins]);
+        rsq[q] = make_float2(rn, 1.0f / rn);
+      }
+      m = __reduce_or_sync(0xffffffffu, m | (same ? 0u : kColour));
+      if ((threadIdx.x & 31) == 0) grp[g] = m;
     }
     __syncthreads();
   }
-  // bins in use around the warp's two rows of pixels
+  // bins in use around the warp's two rows of pixels (and a few records more:
+  // whole groups)
   uint32_t around = 0;
   if (filter) {
-    const uint32_t* mw = msk + (threadIdx.x >> 5) * 2 * kSpan;
-    for (int i = threadIdx.x & 31; i < (2 + 2 * kHalo) * kSpan; i += 32) around |= mw[i];
+    const int q0 = (threadIdx.x >> 5) * 2 * kSpan, g = q0 / 32 + (threadIdx.x & 31);
+    if (g <= (q0 + (2 + 2 * kHalo) * kSpan - 1) / 32) around = grp[g];
     around = __reduce_or_sync(0xffffffffu, around);
   }
   const int row = blockIdx.y * kTile + ty, col = blockIdx.x * kTile + tx;
@@ -415,7 +427,7 @@ __global__ void __launch_bounds__(256, 2) k_denoise(DenoiseArgs a) {
         for (int j = 0; j < 4; ++j)
           if (4 * k + j < 3 * kBins) cb[4 * k + j] = e[j];
       }
-      const uint32_t cm = msk[li] & kBinMask;
+      const uint32_t cm = msk[li];
       const float2 cs = rsq[li];
       res = f3(0, 0, 0);
       float ws = 0.0f;
@@ -426,20 +438,20 @@ __global__ void __launch_bounds__(256, 2) k_denoise(DenoiseArgs a) {
             // the staged halo is already clamped, as UnRoll clamps
             const int q = li + dr * kSpan + dc;
             const float* nr = rec + q * kRec;
-            const float w = fmaxf(0.0f, 1.0f - 1.2f * cmp(nr, rsq[q], msk[q] & kBinMask));
+            const float w = fmaxf(0.0f, 1.0f - 1.2f * cmp(nr, rsq[q], msk[q]));
             const float4 cv = *reinterpret_cast<const float4*>(nr + 32);  // x, then the colour
             res = res + f3(cv.y, cv.z, cv.w) * w;
             ws += w;
           }
       };
-      if (around & kColour)
-        sweep([&](const float* nr, float2 ns, uint32_t nm) { return compare(cb, cs, cm, nr, ns, nm); });
-      else if (around & 0x300u)
-        sweep([&](const float* nr, float2 ns, uint32_t nm) { return compare_gray<3>(cb, cs, cm, nr, ns, nm); });
-      else if (around & 0xf0u)
-        sweep([&](const float* nr, float2 ns, uint32_t nm) { return compare_gray<2>(cb, cs, cm, nr, ns, nm); });
-      else
+      if (!(around & (kColour | 0x3f0u)))
         sweep([&](const float* nr, float2 ns, uint32_t nm) { return compare_gray<1>(cb, cs, cm, nr, ns, nm); });
+      else if (!(around & (kColour | 0x300u)))
+        sweep([&](const float* nr, float2 ns, uint32_t nm) { return compare_gray<2>(cb, cs, cm, nr, ns, nm); });
+      else if (!(around & kColour))
+        sweep([&](const float* nr, float2 ns, uint32_t nm) { return compare_gray<3>(cb, cs, cm, nr, ns, nm); });
+      else
+        sweep([&](const float* nr, float2 ns, uint32_t nm) { return compare(cb, cs, cm, nr, ns, nm); });
       res = res / ws;
     }
   }
