@@ -134,34 +134,6 @@ __device__ __forceinline__ F3 sky(const PathScene& sc, F3 d) {
   return sc.env_map ? env_lookup(sc.env_map, sc.env_w, sc.env_h, sc.env, d) : sc.env;
 }
 
-// CalculateRadiance (core/render.cuh:200-258), one sample.
-__device__ __forceinline__ F3 path_radiance(const Medium& m, const PathScene& sc, Rng& rng, F3 ori, F3 dir,
-                                            float* first_t, TrackStats& st) {
-  dir = normalize(dir);
-  float t = -1;
-  float dis = ray_box_offset(ori, dir);
-  if (dis < 0) { *first_t = t; return sky(sc, dir); }
-  F3 res = f3(0, 0, 0);
-  F3 pos = ori + dir * dis;
-  F3 rd = dir;
-  F3 rate = f3(1, 1, 1);
-  for (int s = 0; s < sc.max_bounces; ++s) {
-    F3 np, nd;
-    float maxd = ray_box_distance(pos, rd);
-    bool hit = next_vertex(m, rng, sc.alpha, sc.g, pos, rd, maxd, np, nd, st);
-    if (!hit) { res = res + sky(sc, rd) * rate; break; }
-    if (s == 0) t = length(ori - np);
-    pos = np;
-    rate = rate * sc.scatter;
-    maxd = ray_box_distance(pos, sc.L);
-    float ph = hg_phase(dot(rd, sc.L), sc.g);
-    res = res + (sc.light_color * rate) * (transmittance(m, rng, pos, sc.L, maxd, sc.alpha, st) * ph);
-    rd = nd;
-  }
-  *first_t = t;
-  return res;
-}
-
 struct CameraModel {
   F3 ori, fwd, up, right;
   int width, height;

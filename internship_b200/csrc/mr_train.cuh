@@ -9,7 +9,7 @@
 namespace mr {
 
 struct TrainTables {
-  int S[12], mode[12], from[12], pid[12], se0[12], se1[12], w[12][3], b[12][3];
+  int S[12], from[12], se0[12], se1[12], w[12][3], b[12][3];
   int l81w[3], l81b[3], ld41w[3], ld41b[3];
   int f1, f2, ggw, ggb, lc0w, lc0b, lc1w, lc1b, lc2w, lc2b, lxw, lxb, lxrw[12], lxrb[12], lx12w, lx12b;
 };
@@ -17,7 +17,6 @@ constexpr TrainTables make_train_tables() {
   TrainTables t{};
   const WeightTable wt = make_weight_table();
   const int S[12] = {8, 8, 16, 16, 16, 32, 32, 32, 8, 8, 8, 8};
-  const int mode[12] = {0, 2, 1, 1, 2, 1, 1, 1, 0, 1, 1, 1};
   const int from[12] = {0, 8, 16, 32, 48, 64, 96, 128, 160, 168, 176, 184};
   const int se0[12] = {MR_W_LSE01W, MR_W_LSE11W, MR_W_LSE21W, MR_W_LSE31W, MR_W_LSE41W, MR_W_LSE51W,
                        MR_W_LSE61W, MR_W_LSE71W, MR_W_LDSE01W, MR_W_LDSE11W, MR_W_LDSE21W, MR_W_LDSE31W};
@@ -36,7 +35,7 @@ constexpr TrainTables make_train_tables() {
                          {MR_W_LD01B, MR_W_LD_Tr01B, MR_W_LD_Hg01B}, {MR_W_LD11B, MR_W_LD_Tr11B, MR_W_LD_Hg11B},
                          {MR_W_LD21B, MR_W_LD_Tr21B, MR_W_LD_Hg21B}, {MR_W_LD31B, MR_W_LD_Tr31B, MR_W_LD_Hg31B}};
   for (int i = 0; i < 12; ++i) {
-    t.S[i] = S[i]; t.mode[i] = mode[i]; t.from[i] = from[i]; t.pid[i] = 3 * i;
+    t.S[i] = S[i]; t.from[i] = from[i];
     t.se0[i] = wt.off[se0[i]]; t.se1[i] = wt.off[se1[i]];
     for (int br = 0; br < 3; ++br) { t.w[i][br] = wt.off[lw[i][br]]; t.b[i][br] = wt.off[lb[i][br]]; }
   }
