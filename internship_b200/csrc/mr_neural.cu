@@ -1305,8 +1305,9 @@ __global__ void k_sphere_h0_batch(const BatchJob* __restrict__ jobs, const float
 
 // Groups of points per record in the batched gather (gather_groups' largest
 // gains need no more; a launch covers the wave's pixels, of which the records
-// are a part, so more groups would mostly add empty blocks). Batch of 8 views,
-// texture filter: 1097 us at one group, 1033 at three.
+// are a part, so more groups add empty blocks). Gather at 1, 3 and 6 groups,
+// us: 2 small views, exact sampler 398 / 166 / 103, texture filter 218 / 93 /
+// 64; 8 views of up to 1024 x 1024, 2076 / 1701 / 1506 and 1186 / 1062 / 1089.
 constexpr int kBatchGroups = 3;
 template <int SAMP>
 __global__ void __launch_bounds__(256, 3) k_gather_batch(const BatchJob* __restrict__ jobs,
