@@ -1,6 +1,6 @@
 """Training calls at the edges of what they accept: descriptor tables at any
-float address, steps captured into a graph before the trainer grows, and steps
-on a device that is nearly full."""
+float address, one row, steps captured into a graph before the trainer grows,
+and steps on a device that is nearly full."""
 import ctypes as C
 
 import numpy as np
@@ -41,6 +41,24 @@ def test_descriptors_at_any_float_address(precision, shift, n):
     tr.close()
     assert np.linalg.norm(ref) > 0
     assert np.linalg.norm(got - ref) <= 2e-5 * np.linalg.norm(ref)
+    assert loss == pytest.approx(ref_loss, rel=1e-5)
+
+
+# A batch of one row, and the same row 65 times, at every place of a tile and as
+# the only row of a second one: the same mean gradient. The copies' terms are
+# equal, so the sums round at the size of the gradient's entries; in BF16 the
+# 1 / 65 shifts the roundings of the rows' gradients, 2^-9 each at most.
+@pytest.mark.parametrize("precision,tol", [("fp32", 2e-5), ("bf16", 1e-2)])
+def test_one_row_equals_its_copies(precision, tol):
+    from internship_b200.train import Trainer
+    from internship_b200.weights import active_random_weights
+    one = _rows(1, 3)
+    tr = Trainer(active_random_weights(2), precision)
+    g, loss = tr.gradient(*one)
+    ref, ref_loss = tr.gradient(*[x.expand(65, *x.shape[1:]).contiguous() for x in one])
+    tr.close()
+    assert np.linalg.norm(ref) > 0
+    assert np.linalg.norm(g - ref) <= tol * np.linalg.norm(ref)
     assert loss == pytest.approx(ref_loss, rel=1e-5)
 
 
