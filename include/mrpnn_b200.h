@@ -7,6 +7,21 @@
  * the current device; `stream` is a cudaStream_t passed as void* (NULL = the
  * legacy default stream).
  *
+ * Device memory that stays allocated between calls:
+ *  - a volume's density and its tables (184 MB whatever its resolution), and
+ *    texture copies of the density and of 86 MB of the tables once a render
+ *    needs them; the scratch of its largest neural render; the frames of its
+ *    host renders (one for mr_render_host, two for mr_render_host_async);
+ *  - a trainer's buffers: 5.5 KB per row of its largest batch, at most 361 MB
+ *    (less where the device is nearly full: batches then run in pieces);
+ *  - a pool per device, shared by all objects, from which offline delta
+ *    tracking takes 24 bytes per pixel and mr_radiance_predict 2.3 (FP32) or
+ *    2.8 KB per row for at most 75,776 rows (148 SMs x 512) at a time: at most
+ *    256 MiB stay in it, and what is unused goes back when a volume or a
+ *    network is destroyed.
+ * Under a stream capture the pool's and the trainer's buffers are allocation
+ * nodes of the graph instead.
+ *
  * Each entry point names the reference interface it replaces
  * (paths relative to the reference project).
  */
@@ -44,7 +59,9 @@ typedef enum {
 typedef enum { MR_RT_PT = 0, MR_RT_RPNN = 1, MR_RT_MRPNN = 2, MR_RT_MARCHING_MRPNN = 3 } mr_render_type;
 
 /* Arithmetic of the radiance-predictor MLP.
- * FP32: CUDA cores, the reference's arithmetic order.
+ * FP32: fp32 accuracy. The per-row parts run on the CUDA cores; the main trunk's
+ *       16- and 32-wide layers and LC0..LC2 run on the tensor cores, their operands
+ *       split into three BF16 or two TF32 parts, FP32 accumulation.
  * BF16: tcgen05 tensor cores, BF16 operands, FP32 accumulation.
  * FP8:  tcgen05 tensor cores, E4M3 operands with a power-of-two scale per
  *       layer (weights) and per row (activations), FP32 accumulation. */
@@ -440,8 +457,8 @@ int mr_trainer_gradient(mr_trainer* t, const float* dev_desc, const float* dev_a
 int mr_trainer_step(mr_trainer* t, const float* dev_desc, const float* dev_aux, const float* dev_label, int32_t n,
                     float lr, float* host_loss, void* stream);
 int mr_trainer_weights(const mr_trainer* t, float* host_out, size_t count);
-/* Arithmetic of the training step: MR_PREC_FP32 (default; every layer on the
- * CUDA cores, one row per thread) or MR_PREC_BF16: the head's LC0 / LC1 / LC2
+/* Arithmetic of the training step: MR_PREC_FP32 (default; every layer in FP32 on
+ * the CUDA cores, over tiles of 64 rows) or MR_PREC_BF16: the head's LC0 / LC1 / LC2
  * forward, input-gradient and weight-gradient products as tcgen05 MMAs with
  * BF16 operands and FP32 accumulation, the rest in FP32; Adam keeps the FP32
  * master weights either way. */
