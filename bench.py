@@ -176,24 +176,25 @@ def run_reference(args, rank):
 
 TRAINED = os.path.join(ROOT, "internship_b200", "data", "mrpnn_trained.npy")
 
-# DRAM bytes (read + write) per unit from one ncu capture of each kernel on the
-# 960x540 case of this frame (ncu --set full, one launch each): per active pixel
-# for the gathers and networks (the fp32 network: k_tc32_trunk + k_light_trunk +
-# k_tc32_head + k_tc32_tail),
-# per density fetch for the trace. A launch's traffic = this figure x the
-# launch's units.
-TRAFFIC_PER_UNIT = {"k_simt": 3377.8, "k_tc32_trunk": 2103.4, "k_mlp_tc": 2456.3, "k_gather_fm_exact": 2463.2,
-                    "k_gather_fm_texture": 2447.0, "k_nn_trace": 52.56}
-# k_nn_trace: dram__bytes_read + write of one launch of the 1080p bench frame
-# (759.9 MB for 14.46 M density fetches); the others at 960x540 per active pixel.
+# DRAM bytes (read + write) per unit, from ncu captures of single launches: per
+# density fetch for the trace, per active pixel for the others (the fp32
+# network: k_tc32_trunk + k_light_trunk + k_tc32_head + k_tc32_tail, 3201.0 +
+# 560.1 + 710.2 + 148.5). The fp32 / exact frame's kernels at 1920x1080 (14.47 M
+# fetches, 322,070 active pixels), the texture gather and the tensor-core network
+# at 960x540. A launch's traffic = this figure x the launch's units.
+TRAFFIC_PER_UNIT = {"k_simt": 4619.7, "k_tc32_trunk": 3201.0, "k_mlp_tc": 2412.3, "k_gather_fm_exact": 2451.8,
+                    "k_gather_fm_texture": 2456.8, "k_nn_trace": 48.06}
 SIMT_KERNELS = ("k_tc32_trunk + k_light_trunk + k_tc32_head + k_tc32_tail (fp32 network: tcgen05 trunk in "
                 "BF16 parts and head in three-term TF32 products, fp32-accurate; CUDA-core light trunk and tail)")
 # The library's kernels of one fp32 / exact-sampler frame, in launch order
 # (as an ncu launch list of this command shows them).
 FP32_FRAME_KERNELS = ("k_sphere_h0", "k_nn_trace", "k_gather_fm", "k_tc32_trunk", "k_light_trunk", "k_tc32_head",
                       "k_tc32_tail")
-# algorithmic FLOPs per active pixel of the fp32 main-trunk kernel (blocks 0..7 and L81)
-TRUNK_FLOP_PER_PIXEL = 32.9e3
+# FLOPs per active pixel of the fp32 main-trunk kernel (blocks 0..7 and L81): its
+# 16- and 32-wide layers (14,592 multiply-adds) run as six BF16 products each on
+# the tensor cores, the gates and the width-8 blocks on the CUDA cores
+TRUNK_MMA_FLOP_PER_PIXEL = 6 * 2 * 14592
+TRUNK_ROW_FLOP_PER_PIXEL = 32.9e3 - 2 * 14592
 # fp32 FMA rate of the CUDA cores (148 SMs x 128 lanes x 2 FLOP x 1.965 GHz), nominal
 FP32_PEAK_TFLOPS = 148 * 128 * 2 * 1.965e9 / 1e12
 
@@ -728,25 +729,28 @@ def main():
     stages["nn_trace"]["traffic"] = TRAFFIC_PER_UNIT["k_nn_trace"] * fetches
     stages["nn_gather"]["traffic"] = TRAFFIC_PER_UNIT["k_gather_fm_exact"] * active
     stages["nn_network"]["traffic"] = TRAFFIC_PER_UNIT["k_simt"] * active
-    stages["nn_network"]["fp32_fma_peak"] = FP32_PEAK_TFLOPS
-    stages["nn_network"]["frac_of_fp32_fma_peak"] = stages["nn_network"]["achieved"] / FP32_PEAK_TFLOPS
     for s_ in stages.values():
-        s_["traffic_source"] = "ncu dram__bytes_read+write per unit at 960x540, scaled by this launch's units"
-    stages["nn_trace"]["traffic_source"] = ("ncu dram__bytes_read+write of one 1080p launch (52.56 B per fetch), "
-                                            "scaled by this launch's fetches")
+        s_["traffic_source"] = "ncu dram__bytes_read+write of one 1080p launch, scaled by this launch's units"
     # the dominant single kernel of the frame: the trace, the gather, or the
     # largest of the network's four kernels (the main trunk, timed on its own
     # as library stage 7)
     trunk_ms = head["stage"][7]
     kernels = {"k_nn_trace": dict(stages["nn_trace"], stage="nn_trace"),
                "k_gather_fm": dict(stages["nn_gather"], stage="nn_gather"),
-               "k_tc32_trunk": {"bound": "fp32", "kernel": "k_tc32_trunk (fp32 main trunk: layers on the tensor cores in BF16 parts, per-row code on the CUDA cores)",
+               "k_tc32_trunk": {"bound": "tensor",
+                                "kernel": "k_tc32_trunk (fp32 main trunk: layers on the tensor cores in BF16 parts, "
+                                          "per-row code on the CUDA cores)",
                                 "ms": trunk_ms,
-                                "achieved": TRUNK_FLOP_PER_PIXEL * active / (trunk_ms / 1e3) / 1e12,
-                                "peak": FP32_PEAK_TFLOPS, "unit": "TFLOP/s",
-                                "peak_source": "nominal fp32 FMA rate (148 SMs x 128 lanes x 2 x 1.965 GHz)",
+                                "achieved": TRUNK_MMA_FLOP_PER_PIXEL * active / (trunk_ms / 1e3) / 1e12,
+                                "peak": bf16, "unit": "TFLOP/s", "peak_source": src,
+                                "cuda_cores": {"achieved": TRUNK_ROW_FLOP_PER_PIXEL * active / (trunk_ms / 1e3) / 1e12,
+                                               "peak": FP32_PEAK_TFLOPS, "unit": "TFLOP/s",
+                                               "peak_source": "nominal fp32 FMA rate "
+                                                              "(148 SMs x 128 lanes x 2 x 1.965 GHz)"},
+                                "limiter": "instruction issue and latency of the per-row code (52 % of the issue "
+                                           "slots); neither peak is near",
                                 "stage": "nn_network"}}
-    kernels["k_tc32_trunk"]["frac"] = kernels["k_tc32_trunk"]["achieved"] / FP32_PEAK_TFLOPS
+    kernels["k_tc32_trunk"]["frac"] = kernels["k_tc32_trunk"]["achieved"] / bf16
     kernels["k_tc32_trunk"]["traffic"] = TRAFFIC_PER_UNIT["k_tc32_trunk"] * active
     dom = max(kernels, key=lambda k: kernels[k]["ms"])
     roofline = kernels[dom]
