@@ -17,13 +17,14 @@ struct DTArgs {
   CameraModel cam;
   uint32_t seed, sample_offset;
   int spp;
-  unsigned long long total;         // W*H*spp
+  int row0, rows;                   // the rendered rows
+  unsigned long long total;         // their pixels*spp (half the pixels with checker)
   unsigned long long* queue;        // work counter (zeroed before launch)
   unsigned long long* counters;     // [0] fetches, [1] paths, [2] loop caps
   float* store;                     // W*H*3 (nullable): one path per pixel, its radiance written, no sums
   int checker, flip;                // store only: half the pixels, those with (row + flip) & 1 == col & 1
-  double* sum64;                    // W*H*3 (unless store)
-  double* sumsq64;                  // W*H*3 (nullable)
+  double* sum64;                    // (unless store) indexed by the frame's pixels, the rendered rows used
+  double* sumsq64;                  // likewise (nullable)
 };
 
 // Per-pixel sums of one finished path's radiance (clamped at 0).
@@ -68,8 +69,12 @@ struct PixelPaths {
       const unsigned s = (unsigned)(w / P);
       pix = (unsigned)(w - (unsigned long long)s * P);
       const int per_row = a.checker ? (a.cam.width + 1) / 2 : a.cam.width;
-      const int row = pix / per_row;
+      int row = pix / per_row;
       int col = pix - row * per_row;
+      if (a.row0) {
+        row += a.row0;
+        pix += a.row0 * a.cam.width;
+      }
       if (a.checker) {
         col = 2 * col + ((row + a.flip) & 1);
         if (col >= a.cam.width) continue;
@@ -99,7 +104,7 @@ __global__ void __launch_bounds__(128) k_delta_track(const __grid_constant__ DTA
   __shared__ uint32_t ring[kRingWords * 128];
   TrackStats st{0, 0};
   const int per_row = a.checker ? (a.cam.width + 1) / 2 : a.cam.width;
-  PixelPaths pp{a, (unsigned long long)per_row * a.cam.height, {}, {}, {}, 0, 0};
+  PixelPaths pp{a, (unsigned long long)per_row * a.rows, {}, {}, {}, 0, 0};
   pp.rng.attach(ring);
   run_paths(pp, a.m, a.sc.alpha, a.sc.g, a.sc.L, a.sc.max_bounces, st);
   const unsigned paths = pp.paths;
@@ -245,9 +250,11 @@ int check_params(const mr_render_params* p) {
   return MR_OK;
 }
 
-// Launch the tracer: adds the samples' radiance to sum64 and, unless null,
-// its square to sumsq64.
-int launch_delta_track(Volume* v, const mr_render_params* p, double* sum64, double* sumsq64, cudaStream_t s) {
+// Launch the tracer over `rows` rows from row0 on: adds the samples' radiance
+// to sum64 (of these rows) and, unless null, its square to sumsq64. The volume's
+// counters start anew with row 0.
+static int launch_delta_track(Volume* v, const mr_render_params* p, int row0, int rows, double* sum64, double* sumsq64,
+                              cudaStream_t s) {
   if (!v->data_set) return set_error(MR_ERR_STATE, "render before mr_volume_set_data");
   if (!v->mips_valid) return set_error(MR_ERR_STATE, "render before mr_volume_update");
   DTArgs a;
@@ -262,14 +269,16 @@ int launch_delta_track(Volume* v, const mr_render_params* p, double* sum64, doub
   a.seed = p->seed;
   a.sample_offset = p->sample_offset;
   a.spp = p->spp;
-  a.total = (unsigned long long)p->width * p->height * p->spp;
+  a.row0 = row0;
+  a.rows = rows;
+  a.total = (unsigned long long)p->width * rows * p->spp;
   a.queue = v->d_counters + 4;
   a.counters = v->d_counters;
   a.store = nullptr;
   a.checker = a.flip = 0;
-  a.sum64 = sum64;
-  a.sumsq64 = sumsq64;
-  MR_CUDA(cudaMemsetAsync(v->d_counters, 0, kCounters * sizeof(unsigned long long), s));
+  a.sum64 = sum64 - (size_t)row0 * p->width * 3;
+  a.sumsq64 = sumsq64 ? sumsq64 - (size_t)row0 * p->width * 3 : nullptr;
+  MR_CUDA(cudaMemsetAsync(row0 ? a.queue : v->d_counters, 0, (row0 ? 1 : kCounters) * sizeof(unsigned long long), s));
   v->timer.mark(ST_PT, s);
   k_delta_track<<<dt_grid(), 128, 0, s>>>(a);
   v->timer.mark(ST_PT, s);
@@ -292,6 +301,8 @@ int launch_path_frame(Volume* v, const mr_render_params* p, uint32_t sample, int
   a.seed = p->seed;
   a.sample_offset = sample;
   a.spp = 1;
+  a.row0 = 0;
+  a.rows = p->height;
   a.total = (unsigned long long)(checker ? (p->width + 1) / 2 : p->width) * p->height;
   a.queue = v->d_counters + kCounters;
   a.counters = nullptr;
@@ -307,20 +318,31 @@ int launch_path_frame(Volume* v, const mr_render_params* p, uint32_t sample, int
 
 // A pixel's samples finish in any order. Their FP64 sum is exact for all but
 // extreme ranges of radiance, so two renders of one request agree, which fp32
-// sums in the order of the atomics did only by timing.
+// sums in the order of the atomics did only by timing. Where the device is
+// nearly full, fewer rows at a time: the same image.
 int render_pt(Volume* v, const mr_render_params* p, float* dev_rgb, cudaStream_t s) {
-  const size_t n = (size_t)p->width * p->height * 3;
+  const size_t row = (size_t)p->width * 3;
+  int rows = p->height;
   double* sum = nullptr;
-  cudaError_t e = pool_alloc((void**)&sum, n * sizeof(double), s);
-  if (e != cudaSuccess) return set_error(MR_ERR_NOMEM, "sample sums of %zu bytes: %s", n * sizeof(double), cudaGetErrorString(e));
+  cudaError_t e = pool_alloc((void**)&sum, rows * row * sizeof(double), s);
+  while (e == cudaErrorMemoryAllocation && rows > 1) {
+    rows = (rows + 1) / 2;
+    e = pool_alloc((void**)&sum, rows * row * sizeof(double), s);
+  }
+  if (e != cudaSuccess)
+    return set_error(MR_ERR_NOMEM, "sample sums of %zu bytes: %s", rows * row * sizeof(double), cudaGetErrorString(e));
   int rc = MR_OK;
-  e = cudaMemsetAsync(sum, 0, n * sizeof(double), s);
-  if (e != cudaSuccess) rc = cuda_error(e, "cudaMemsetAsync(sample sums)");
-  if (rc == MR_OK) rc = launch_delta_track(v, p, sum, nullptr, s);
-  if (rc == MR_OK) {
-    k_mean<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(sum, dev_rgb, n, (double)p->spp);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) rc = cuda_error(e, "k_mean");
+  for (int r0 = 0; r0 < p->height && rc == MR_OK; r0 += rows) {
+    const int m = std::min(rows, p->height - r0);
+    const size_t n = m * row;
+    e = cudaMemsetAsync(sum, 0, n * sizeof(double), s);
+    if (e != cudaSuccess) rc = cuda_error(e, "cudaMemsetAsync(sample sums)");
+    if (rc == MR_OK) rc = launch_delta_track(v, p, r0, m, sum, nullptr, s);
+    if (rc == MR_OK) {
+      k_mean<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(sum, dev_rgb + r0 * row, n, (double)p->spp);
+      e = cudaGetLastError();
+      if (e != cudaSuccess) rc = cuda_error(e, "k_mean");
+    }
   }
   MR_CUDA(cudaFreeAsync(sum, s));
   return rc;
@@ -336,5 +358,5 @@ extern "C" int mr_render_accumulate_f64(mr_volume* h, const mr_render_params* p,
   if (!h || !dev_sum) return set_error(MR_ERR_ARG, "mr_render_accumulate_f64: NULL argument");
   int rc = check_params(p);
   if (rc) return rc;
-  return launch_delta_track(&h->v, p, dev_sum, dev_sumsq, (cudaStream_t)stream);
+  return launch_delta_track(&h->v, p, 0, p->height, dev_sum, dev_sumsq, (cudaStream_t)stream);
 }
