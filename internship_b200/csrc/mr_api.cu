@@ -180,7 +180,7 @@ int mr_network_destroy(mr_network* h) {
   cudaFree(h->n.w);
   cudaFree(h->n.stencil);
   free_packed(&h->n);
-  pool_trim();
+  pool_trim(0);
   delete h;
   return MR_OK;
 }

@@ -579,11 +579,11 @@ cudaError_t pool_alloc(void** p, size_t bytes, cudaStream_t s) {
   if (e == cudaErrorMemoryAllocation) cudaGetLastError();  // reported here, not by the next launch's check
   return e;
 }
-void pool_trim() {
+void pool_trim(size_t keep) {
   cudaDeviceSynchronize();  // a pool gives back what the host has seen freed
   std::lock_guard<std::mutex> lock(g_pool_mu);
   for (cudaMemPool_t pool : g_pool)
-    if (pool) cudaMemPoolTrimTo(pool, 0);
+    if (pool) cudaMemPoolTrimTo(pool, keep);
 }
 
 int ensure_scratch(Volume* v, size_t bytes, cudaStream_t s) {
@@ -672,7 +672,7 @@ int mr_volume_destroy(mr_volume* h) {
     cudaStreamDestroy(v->side_stream);
   }
   destroy_textures(v);
-  pool_trim();
+  pool_trim(kPoolKeepVolume);
   delete h;
   return MR_OK;
 }

@@ -21,8 +21,9 @@ def _offline_render(side, out):
     v.close()
 
 
-def test_offline_tracking_leaves_no_memory_behind():
-    """A 2048 x 2048 render sums its samples in 96 MiB of FP64."""
+def test_offline_tracking_gives_its_memory_back():
+    """A 2048 x 2048 render sums its samples in 96 MiB of FP64; the library keeps
+    at most 32 MiB of that after the volume."""
     import torch
     import internship_b200 as mr
     out = torch.zeros(2048 * 2048 * 3, device="cuda")
@@ -32,6 +33,8 @@ def test_offline_tracking_leaves_no_memory_behind():
     free = torch.cuda.mem_get_info()[0]
     _offline_render(2048, out)
     torch.cuda.synchronize()
+    assert torch.cuda.mem_get_info()[0] >= free - (32 << 20)
+    mr.Network(mr.xavier_weights(1)).close()
     assert torch.cuda.mem_get_info()[0] >= free
 
 
