@@ -17,8 +17,9 @@
  *  - a pool per device, shared by all objects, from which offline delta
  *    tracking takes 24 bytes per pixel and mr_radiance_predict 2.3 (FP32) or
  *    2.8 KB per row for at most 75,776 rows (148 SMs x 512) at a time: at most
- *    256 MiB stay in it; what is unused goes back when a network is destroyed,
- *    and all but 32 MiB of it when a volume is.
+ *    256 MiB stay in it; what is unused, as far as the caller has waited for the
+ *    calls that used it, goes back when a network is destroyed, and all but
+ *    32 MiB of it when a volume is.
  * Under a stream capture the pool's and the trainer's buffers are allocation
  * nodes of the graph instead.
  *

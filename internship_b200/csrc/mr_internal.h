@@ -192,12 +192,14 @@ inline F3 to_f3(const mr_float3& a) { return F3{a.x, a.y, a.z}; }
 // Stream-ordered temporary memory from a pool of the library's own on the
 // current device. Up to kPoolKeep bytes stay with the pool between calls (the
 // runtime's default pool returns everything to the device at each
-// synchronisation and maps it again on the next call); pool_trim gives the
+// synchronisation and maps it again on the next call). pool_trim gives the
 // unused memory above `keep` bytes of all devices back, when a volume or a
-// network, whose calls used it, is destroyed. A volume leaves one mapping unit
-// of the pool, for the next volume's frames (a megapixel of offline tracking):
-// mapping it again makes that volume's first render 0.3 ms longer (256 x 256 x 64
-// spp: 3.9 and 4.2 ms).
+// network, whose calls used it, is destroyed: what the host has waited for (a
+// stream, an event or the device). It does not wait itself, which would break a
+// capture under way in another thread. A volume leaves one mapping unit of the
+// pool for the next volume's frames (a megapixel of offline tracking): mapping
+// it again makes that volume's first render 0.3 ms longer (256 x 256 x 64 spp:
+// 3.9 and 4.2 ms).
 constexpr size_t kPoolKeep = (size_t)256 << 20, kPoolKeepVolume = (size_t)32 << 20;
 cudaError_t pool_alloc(void** p, size_t bytes, cudaStream_t s);
 void pool_trim(size_t keep);

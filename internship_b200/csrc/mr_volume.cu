@@ -580,7 +580,6 @@ cudaError_t pool_alloc(void** p, size_t bytes, cudaStream_t s) {
   return e;
 }
 void pool_trim(size_t keep) {
-  cudaDeviceSynchronize();  // a pool gives back what the host has seen freed
   std::lock_guard<std::mutex> lock(g_pool_mu);
   for (cudaMemPool_t pool : g_pool)
     if (pool) cudaMemPoolTrimTo(pool, keep);

@@ -11,6 +11,7 @@ pytestmark = pytest.mark.gpu
 
 def _offline_render(side, out):
     """A volume, one delta-tracking render into `out`, and the volume's end."""
+    import torch
     import internship_b200 as mr
     from internship_b200 import _lib, scenes
     v = mr.VolumeRender(16)
@@ -18,6 +19,7 @@ def _offline_render(side, out):
     v.Update()
     p = scenes.make_params(side, side, 1, bounces=4)
     _lib.check(_lib.load().mr_render(v.handle, None, C.byref(p), C.c_void_p(out.data_ptr()), None))
+    torch.cuda.synchronize()
     v.close()
 
 
